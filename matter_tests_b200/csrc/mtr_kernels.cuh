@@ -712,12 +712,6 @@ constexpr int kMaxTileThreads = 256;
 #ifndef MTR_DEFGRAD_MIN_BLOCKS_F32
 #define MTR_DEFGRAD_MIN_BLOCKS_F32 6
 #endif
-// The return mapping takes its SVD from the symmetric eigenproblem of F F^T
-// (svd_sym); 0 selects the two-sided Jacobi iteration with the reference's
-// ordering and sign conventions instead.
-#ifndef MTR_SYM_SVD
-#define MTR_SYM_SVD 1
-#endif
 #ifndef MTR_G2P_MIN_BLOCKS
 #define MTR_G2P_MIN_BLOCKS 3
 #endif
@@ -1383,7 +1377,7 @@ __device__ __forceinline__ void defgrad_and_store(const StepArgsT<R>& A, uint32_
 #pragma unroll
     for (int c = 0; c < D; ++c) p.F[r][c] = p.F[r][c] + T2[r][c];
   double tau[Sym<D>::n];
-  plastic = return_map<D, PM, MTR_SYM_SVD != 0>(*A.P, dt, p.F, p.s, tau, flags);
+  plastic = return_map<D, PM>(*A.P, dt, p.F, p.s, tau, flags);
   store_defgrad<D, R>(A.out, A.Np, s, p.F, p.s, tau);
 }
 
@@ -1392,22 +1386,6 @@ __device__ __forceinline__ void defgrad_and_store(const StepArgsT<R>& A, uint32_
 // particles' stencils can reach (the PN^D patch of the tile) from the node
 // arrays into shared memory, then every particle gathers from there.
 // ---------------------------------------------------------------------------
-
-// copies NF fields of D components each, src[f] = [D][cap] node arrays
-template <int D, int NF, typename R>
-__device__ __forceinline__ void load_node_patch(const StepCommon& A, const StepHeader* H, const int (&n0)[3],
-                                                const R* const (&src)[NF], R* dst /*[NF*D][NODES]*/) {
-  constexpr int NODES = Tiling<D>::NODES;
-  const uint32_t cap = A.cap_nodes;
-  for (int n = threadIdx.x; n < NODES; n += blockDim.x) {
-    uint32_t l = 0;
-    const bool in = patch_node<D>(H, n0, n, l);
-#pragma unroll
-    for (int f = 0; f < NF; ++f)
-#pragma unroll
-      for (int a = 0; a < D; ++a) dst[(f * D + a) * NODES + n] = in ? src[f][(size_t)a * cap + l] : R(0.0);
-  }
-}
 
 // Reference velocity of a tile: the FP64 node velocity at the patch node
 // nearest the tile centre (zero outside the grid, and always zero on the FP64
@@ -1427,112 +1405,225 @@ __device__ __forceinline__ void tile_vref(const StepCommon& A, const StepHeader*
   }
 }
 
-// node velocity patch as deviations from vref, rounded to R
-template <int D, typename R>
-__device__ __forceinline__ void load_velocity_patch(const StepCommon& A, const StepHeader* H, const int (&n0)[3],
-                                                    const double* src, const double (&vref)[3],
-                                                    R* dst /*[D][NODES]*/) {
-  constexpr int NODES = Tiling<D>::NODES;
+// Node patch of the gathers, interleaved: values per node are the D velocity
+// components (deviations from vref, rounded to R) and, with FLIP, the D flip
+// components, padded so that a node is read with vector loads.
+template <int D, bool FLIP, typename R>
+struct NodePatch {
+  static constexpr int STRIDE = D == 2 ? (FLIP ? 4 : 2) : (FLIP ? (sizeof(R) == 8 ? 6 : 8) : 4);
+  static constexpr int SIZE = STRIDE * Tiling<D>::NODES;
+};
+
+template <typename R>
+struct Vec2;
+template <>
+struct Vec2<double> {
+  using T = double2;
+};
+template <>
+struct Vec2<float> {
+  using T = float2;
+};
+
+// v (and with WF flip) of one patch node
+template <int D, bool WF, typename R>
+__device__ __forceinline__ void load_node(const R* __restrict__ p, R (&v)[3], R (&f)[3]) {
+  if constexpr (D == 2) {
+    if constexpr (sizeof(R) == 4 && WF) {
+      const float4 q = *reinterpret_cast<const float4*>(p);
+      v[0] = q.x;
+      v[1] = q.y;
+      f[0] = q.z;
+      f[1] = q.w;
+    } else {
+      const auto q = *reinterpret_cast<const typename Vec2<R>::T*>(p);
+      v[0] = q.x;
+      v[1] = q.y;
+      if constexpr (WF) {
+        const auto g = *reinterpret_cast<const typename Vec2<R>::T*>(p + 2);
+        f[0] = g.x;
+        f[1] = g.y;
+      }
+    }
+  } else if constexpr (sizeof(R) == 8) {
+    const double2 q = *reinterpret_cast<const double2*>(p);
+    v[0] = q.x;
+    v[1] = q.y;
+    if constexpr (WF) {
+      const double2 g = *reinterpret_cast<const double2*>(p + 2), h = *reinterpret_cast<const double2*>(p + 4);
+      v[2] = g.x;
+      f[0] = g.y;
+      f[1] = h.x;
+      f[2] = h.y;
+    } else {
+      v[2] = p[2];
+    }
+  } else {
+    const float4 q = *reinterpret_cast<const float4*>(p);
+    v[0] = q.x;
+    v[1] = q.y;
+    v[2] = q.z;
+    if constexpr (WF) {
+      const float2 g = *reinterpret_cast<const float2*>(p + 4);
+      f[0] = q.w;
+      f[1] = g.x;
+      f[2] = g.y;
+    }
+  }
+}
+
+// fills a node patch from the node velocities src (minus vref) and, with
+// FLIP and want_flip, the node flips
+template <int D, bool FLIP, typename R>
+__device__ __forceinline__ void load_patch(const StepCommon& A, const StepHeader* H, const int (&n0)[3],
+                                           const double* src, const double (&vref)[3], const R* flip, bool want_flip,
+                                           R* dst) {
   const uint32_t cap = A.cap_nodes;
-  for (int n = threadIdx.x; n < NODES; n += blockDim.x) {
+  for (int n = threadIdx.x; n < Tiling<D>::NODES; n += blockDim.x) {
     uint32_t l = 0;
     const bool in = patch_node<D>(H, n0, n, l);
+    R* q = dst + n * NodePatch<D, FLIP, R>::STRIDE;
 #pragma unroll
     for (int a = 0; a < D; ++a) {
       if constexpr (kFP64<R>)
-        dst[a * NODES + n] = in ? src[(size_t)a * cap + l] : 0.0;
+        q[a] = in ? src[(size_t)a * cap + l] : 0.0;
       else
-        dst[a * NODES + n] = in ? (R)(src[(size_t)a * cap + l] - vref[a]) : R(0.0);
+        q[a] = in ? (R)(src[(size_t)a * cap + l] - vref[a]) : R(0.0);
+    }
+    if constexpr (FLIP) {
+#pragma unroll
+      for (int a = 0; a < D; ++a) q[D + a] = in && want_flip ? flip[(size_t)a * cap + l] : R(0.0);
     }
   }
 }
 
 // G2P gather (g2p.cpp:24-77) and velocity gradient (deformation_update.cpp:17-40)
 // from a shared node patch; lb = stencil base relative to the patch origin.
-// Sums are factorised over the tensor-product stencil.  The offsets and the
-// spline argument are formed in FP64 from the FP64 position, then rounded to
-// R.  pv holds node velocities minus vref: B-spline weights sum to one and
-// reproduce linears, so pic = vref + sum w dv, while B and grad v need the
-// deviations only.
-// The sums over the stencil's x layers ii0 .. ii1-1: ps = sum w v (deviations
-// from vref on the mixed path), B, flip and grad v (unscaled).
-template <int D, int DEG, bool GRADV, typename R>
-__device__ __forceinline__ void gather_sums(const R* pv, const R* pf, const double (*crd)[Tiling<D>::PN],
-                                            const int (&lb)[3], const double (&xp)[3], double ioh, R (&ps)[3],
-                                            R (&Bp)[D][D], R (&flp)[3], R (&gv)[D][D], bool want_b, bool want_flip,
-                                            int ii0, int ii1) {
-  constexpr int PN = Tiling<D>::PN, NODES = Tiling<D>::NODES;
-  R w[3][4], dw[3][4], pd[3][4];
+// The offsets and the spline argument are formed in FP64 from the FP64
+// position, then rounded to R.  The patch holds node velocities minus vref:
+// B-spline weights sum to one and reproduce linears, so pic = vref + sum w dv,
+// while B and grad v need the deviations only.
+//
+// The sums are factorised over the tensor-product stencil, innermost axis
+// first: per node only sum w_z v, sum w_z dz v, sum w_z' v and sum w_z flip
+// are formed, rows of 4 nodes are then combined with the y factors and planes
+// of 16 with the x factors.  USL in 3D takes 12 multiply-adds per node and
+// 18 per row instead of 32 per node, MUSL 9 instead of 20, and the deformation
+// update 6 instead of 12.  The x planes stay a loop: unrolling all 64 nodes
+// made the return-mapping kernels too large for the instruction cache.
+// The innermost rows are read as vectors from the interleaved patch (3D USL:
+// three 16-byte loads per node instead of six of 8 bytes in FP64).  What bounds
+// it then is FP64 issue and the registers of the sums (measured together with
+// the series return mapping, see hencky_series).
+template <int D, int DEG, bool FLIP, bool WP, bool WB, bool WF, bool GV, typename R>
+__device__ __forceinline__ void gather_sums(const R* pv, const double (*crd)[Tiling<D>::PN], const int (&lb)[3],
+                                            const double (&xp)[3], double ioh, R (&ps)[3], R (&Bp)[D][D], R (&flp)[3],
+                                            R (&gv)[D][D]) {
+  constexpr int PN = Tiling<D>::PN, STR = NodePatch<D, FLIP, R>::STRIDE;
+  constexpr int Z = D - 1;  // innermost axis
+  R wz[4], dz[4], pz[4], wy[4], dy[4], py[4];
+  auto axis = [&](int a, int o, R& w, R& dw, R& wp) {
+    const double c = crd[a][lb[a] + o];
+    const R u = (R)((xp[a] - c) * ioh);
+    w = bspline_N<DEG>(u);
+    dw = GV ? bspline_dN<DEG>(u) : R(0.0);
+    wp = WB ? w * (R)(c - xp[a]) : R(0.0);
+  };
 #pragma unroll
-  for (int a = 0; a < D; ++a)
-#pragma unroll
-    for (int o = 0; o < 4; ++o) {
-      const double c = crd[a][lb[a] + o];
-      const R u = (R)((xp[a] - c) * ioh);
-      w[a][o] = bspline_N<DEG>(u);
-      dw[a][o] = GRADV ? bspline_dN<DEG>(u) : R(0.0);
-      pd[a][o] = (R)(c - xp[a]);
-    }
+  for (int o = 0; o < 4; ++o) {
+    axis(Z, o, wz[o], dz[o], pz[o]);
+    if constexpr (D == 3) axis(1, o, wy[o], dy[o], py[o]);
+  }
 #pragma unroll
   for (int a = 0; a < 3; ++a) ps[a] = flp[a] = R(0.0);
 #pragma unroll
   for (int r = 0; r < D; ++r)
 #pragma unroll
     for (int c = 0; c < D; ++c) Bp[r][c] = gv[r][c] = R(0.0);
-  constexpr int KN = D == 3 ? 4 : 1;
-  // the x layers of the stencil stay a loop: unrolling all 64 nodes made
-  // the return-mapping kernels that call this too large for the instruction
-  // cache
-#pragma unroll 1
-  for (int ii = ii0; ii < ii1; ++ii)
+  const R* plane = pv + (D == 3 ? (lb[0] * PN + lb[1]) * PN + lb[2] : lb[0] * PN + lb[1]) * STR;
+  // sums of one row of 4 nodes along the innermost axis
+  auto row = [&](const R* q, R (&s0)[3], R (&s1)[3], R (&s2)[3], R (&f0)[3]) {
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
-      const R wxy = w[0][ii] * w[1][jj];
-      const R gx_ = dw[0][ii] * w[1][jj], gy_ = w[0][ii] * dw[1][jj];
+    for (int a = 0; a < D; ++a) s0[a] = s1[a] = s2[a] = f0[a] = R(0.0);
 #pragma unroll
-      for (int kk = 0; kk < KN; ++kk) {
-        const int node = D == 3 ? ((lb[0] + ii) * PN + (lb[1] + jj)) * PN + (lb[2] + kk) : (lb[0] + ii) * PN + (lb[1] + jj);
-        const R weight = D == 3 ? wxy * w[2][kk] : wxy;
-        R vi[D];
+    for (int k = 0; k < 4; ++k) {
+      R v[3], f[3];
+      load_node<D, WF, R>(q + k * STR, v, f);
 #pragma unroll
-        for (int a = 0; a < D; ++a) vi[a] = pv[a * NODES + node];
-#pragma unroll
-        for (int a = 0; a < D; ++a) ps[a] += vi[a] * weight;
-        if (want_b) {
-          R wpd[3] = {weight * pd[0][ii], weight * pd[1][jj], D == 3 ? weight * pd[2][kk] : R(0.0)};
-#pragma unroll
-          for (int r = 0; r < D; ++r)
-#pragma unroll
-            for (int c = 0; c < D; ++c) Bp[r][c] += vi[r] * wpd[c];
-        }
-        if (want_flip) {
-#pragma unroll
-          for (int a = 0; a < D; ++a) flp[a] += pf[a * NODES + node] * weight;
-        }
-        if (GRADV) {
-          R g[3];
-          if constexpr (D == 3) {
-            g[0] = gx_ * w[2][kk];
-            g[1] = gy_ * w[2][kk];
-            g[2] = wxy * dw[2][kk];
-          } else {
-            g[0] = gx_;
-            g[1] = gy_;
-          }
-#pragma unroll
-          for (int r = 0; r < D; ++r)
-#pragma unroll
-            for (int c = 0; c < D; ++c) gv[r][c] += vi[r] * g[c];
-        }
+      for (int a = 0; a < D; ++a) {
+        s0[a] += wz[k] * v[a];
+        if constexpr (WB) s1[a] += pz[k] * v[a];
+        if constexpr (GV) s2[a] += dz[k] * v[a];
+        if constexpr (WF) f0[a] += wz[k] * f[a];
       }
     }
+  };
+#pragma unroll 1
+  for (int ii = 0; ii < 4; ++ii, plane += (D == 3 ? PN * PN : PN) * STR) {
+    R wx, dx, px;
+    axis(0, ii, wx, dx, px);
+    R r0[3], rz[3], gz[3], rf[3];  // plane sums: w, w times offset (innermost), gradient (innermost), flip
+    if constexpr (D == 3) {
+      R ry[3], gy[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) r0[a] = rz[a] = gz[a] = rf[a] = ry[a] = gy[a] = R(0.0);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        R s0[3], s1[3], s2[3], f0[3];
+        row(plane + j * PN * STR, s0, s1, s2, f0);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          r0[a] += wy[j] * s0[a];
+          if constexpr (WB) {
+            ry[a] += py[j] * s0[a];
+            rz[a] += wy[j] * s1[a];
+          }
+          if constexpr (GV) {
+            gy[a] += dy[j] * s0[a];
+            gz[a] += wy[j] * s2[a];
+          }
+          if constexpr (WF) rf[a] += wy[j] * f0[a];
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        if constexpr (WB) Bp[a][1] += wx * ry[a];
+        if constexpr (GV) gv[a][1] += wx * gy[a];
+      }
+    } else {
+      row(plane, r0, rz, gz, rf);
+    }
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+      if constexpr (WP) ps[a] += wx * r0[a];
+      if constexpr (WB) {
+        Bp[a][0] += px * r0[a];
+        Bp[a][Z] += wx * rz[a];
+      }
+      if constexpr (GV) {
+        gv[a][0] += dx * r0[a];
+        gv[a][Z] += wx * gz[a];
+      }
+      if constexpr (WF) flp[a] += wx * rf[a];
+    }
+  }
 }
 
-// pic = vref + ps (the FP64 path gathers the velocities themselves), grad v
-// scaled by 1/dx
-template <int D, bool GRADV, typename R>
-__device__ __forceinline__ void gather_finish(const R (&ps)[3], const double (&vref)[3], double ioh, double (&pic)[3],
-                                              R (&gv)[D][D]) {
+// The sums a transfer scheme needs (B for APIC and AFLIP, flip for all but
+// APIC), pic = vref + ps (the FP64 path gathers the velocities themselves) and
+// grad v scaled by 1/dx.
+template <int D, int DEG, bool GV, typename R>
+__device__ __forceinline__ void gather_patch(const R* pv, const double (*crd)[Tiling<D>::PN], const int (&lb)[3],
+                                             const double (&xp)[3], double ioh, const double (&vref)[3],
+                                             double (&pic)[3], R (&Bp)[D][D], R (&flp)[3], R (&gv)[D][D], bool want_b,
+                                             bool want_flip) {
+  R ps[3];
+  if (!want_flip)
+    gather_sums<D, DEG, true, true, true, false, GV, R>(pv, crd, lb, xp, ioh, ps, Bp, flp, gv);
+  else if (want_b)
+    gather_sums<D, DEG, true, true, true, true, GV, R>(pv, crd, lb, xp, ioh, ps, Bp, flp, gv);
+  else
+    gather_sums<D, DEG, true, true, false, true, GV, R>(pv, crd, lb, xp, ioh, ps, Bp, flp, gv);
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     if constexpr (kFP64<R>)
@@ -1540,7 +1631,7 @@ __device__ __forceinline__ void gather_finish(const R (&ps)[3], const double (&v
     else
       pic[a] = vref[a] + (double)ps[a];
   }
-  if (GRADV) {
+  if (GV) {
     const R iohR = (R)ioh;
 #pragma unroll
     for (int r = 0; r < D; ++r)
@@ -1549,14 +1640,17 @@ __device__ __forceinline__ void gather_finish(const R (&ps)[3], const double (&v
   }
 }
 
-template <int D, int DEG, bool GRADV, typename R>
-__device__ __forceinline__ void gather_patch(const R* pv, const R* pf, const double (*crd)[Tiling<D>::PN],
-                                             const int (&lb)[3], const double (&xp)[3], double ioh,
-                                             const double (&vref)[3], double (&pic)[3], R (&Bp)[D][D], R (&flp)[3],
-                                             R (&gv)[D][D], bool want_b, bool want_flip) {
-  R ps[3];
-  gather_sums<D, DEG, GRADV, R>(pv, pf, crd, lb, xp, ioh, ps, Bp, flp, gv, want_b, want_flip, 0, 4);
-  gather_finish<D, GRADV, R>(ps, vref, ioh, pic, gv);
+// grad v alone (MUSL deformation update), from a patch without flips
+template <int D, int DEG, typename R>
+__device__ __forceinline__ void gather_gradv(const R* pv, const double (*crd)[Tiling<D>::PN], const int (&lb)[3],
+                                             const double (&xp)[3], double ioh, R (&gv)[D][D]) {
+  R ps[3], Bp[D][D], flp[3];
+  gather_sums<D, DEG, false, false, false, false, true, R>(pv, crd, lb, xp, ioh, ps, Bp, flp, gv);
+  const R iohR = (R)ioh;
+#pragma unroll
+  for (int r = 0; r < D; ++r)
+#pragma unroll
+    for (int c = 0; c < D; ++c) gv[r][c] *= iohR;
 }
 
 // ---------------------------------------------------------------------------
@@ -1566,7 +1660,7 @@ __device__ __forceinline__ void gather_patch(const R* pv, const R* pf, const dou
 template <int D, int DEG, typename R, int PM>
 __device__ __forceinline__ void g2p_t_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid, const uint32_t nblk) {
   using TL = Tiling<D>;
-  constexpr int PN = TL::PN, NODES = TL::NODES;
+  constexpr int PN = TL::PN;
   StepHeader* H = A.H;
   if (step_inactive(H)) return;
   const uint32_t t = bid;
@@ -1574,18 +1668,17 @@ __device__ __forceinline__ void g2p_t_body(const StepArgsT<R>& A, const uint32_t
   const uint32_t pb = A.tile_begin[t], pe = A.tile_end[t];
   if (pb >= pe) return;
   const DevParams& P = *A.P;
-  __shared__ R pv[2 * D * NODES];
+  __shared__ __align__(16) R pv[NodePatch<D, true, R>::SIZE];
   __shared__ double crd[3][PN];
   int n0[3];
   load_tile_setup<D>(A, H, t, n0, crd);
   double vref[3];
   tile_vref<D, R>(A, H, n0, A.nv, vref);
-  load_velocity_patch<D, R>(A, H, n0, A.nv, vref, pv);
-  const R* const src[1] = {A.nflip};
-  load_node_patch<D, 1, R>(A, H, n0, src, pv + D * NODES);
+  const double fr = P.flip_ratio;
+  load_patch<D, true, R>(A, H, n0, A.nv, vref, A.nflip, fr >= -1, pv);
   __syncthreads();
   const uint32_t Np = A.Np;
-  const double dt = H->dt, fr = P.flip_ratio, ioh = P.one_over_dx;
+  const double dt = H->dt, ioh = P.one_over_dx;
   unsigned nplastic = 0;
   for (uint32_t s = pb + threadIdx.x; s < pe; s += blockDim.x) {
     const uint32_t j = perm[s];
@@ -1595,7 +1688,7 @@ __device__ __forceinline__ void g2p_t_body(const StepArgsT<R>& A, const uint32_t
     R flp[3], Bp[D][D], gv[D][D];
     int lb[3];
     if (local_base<D>(H, p.x, ioh, n0, false, lb)) {
-      gather_patch<D, DEG, true, R>(pv, pv + D * NODES, crd, lb, p.x, ioh, vref, pic, Bp, flp, gv, fr < 0, fr >= -1);
+      gather_patch<D, DEG, true, R>(pv, crd, lb, p.x, ioh, vref, pic, Bp, flp, gv, fr < 0, fr >= -1);
     } else {
       raise_status(H, MTR_STATUS_STENCIL_OOB, p.id);
 #pragma unroll
@@ -1682,7 +1775,7 @@ constexpr size_t musl_crd_bytes() {
 }
 template <int D, typename R>
 constexpr size_t musl_patch_bytes() {
-  return align16(sizeof(R) * 3 * D * Tiling<D>::NODES);
+  return align16(sizeof(R) * NodePatch<D, true, R>::SIZE) + align16(sizeof(R) * D * Tiling<D>::NODES);
 }
 template <int D, typename R>
 constexpr size_t musl_smem_bytes(int threads) {
@@ -1702,20 +1795,20 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
   const DevParams& P = *A.P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double(*crd)[PN] = reinterpret_cast<double(*)[PN]>(smem_raw);
-  R* pv = reinterpret_cast<R*>(smem_raw + musl_crd_bytes<D, R>());  // [2D][NODES] node v, flip
-  R(*vsum)[NODES] = reinterpret_cast<R(*)[NODES]>(pv + 2 * D * NODES);  // [D][NODES]
+  R* pv = reinterpret_cast<R*>(smem_raw + musl_crd_bytes<D, R>());  // node v, flip
+  R(*vsum)[NODES] = reinterpret_cast<R(*)[NODES]>(
+      smem_raw + musl_crd_bytes<D, R>() + align16(sizeof(R) * NodePatch<D, true, R>::SIZE));  // [D][NODES]
   MStage<D, R>* st = reinterpret_cast<MStage<D, R>*>(smem_raw + musl_crd_bytes<D, R>() + musl_patch_bytes<D, R>());
   int n0[3];
   load_tile_setup<D>(A, H, t, n0, crd);
   double vref[3];
   tile_vref<D, R>(A, H, n0, A.nv, vref);
-  load_velocity_patch<D, R>(A, H, n0, A.nv, vref, pv);
-  const R* const src[1] = {A.nflip};
-  load_node_patch<D, 1, R>(A, H, n0, src, pv + D * NODES);
+  const double fr = P.flip_ratio;
+  load_patch<D, true, R>(A, H, n0, A.nv, vref, A.nflip, fr >= -1, pv);
   for (int i = threadIdx.x; i < D * NODES; i += blockDim.x) (&vsum[0][0])[i] = R(0.0);
   __syncthreads();
   const uint32_t Np = A.Np;
-  const double dt = H->dt, fr = P.flip_ratio, ioh = P.one_over_dx;
+  const double dt = H->dt, ioh = P.one_over_dx;
   const R apicD = (R)P.apicDinverse;
   const bool apic = fr < 0;
   const int lane = threadIdx.x & 31;
@@ -1799,8 +1892,7 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
         int lb[3];
         const bool ok = local_base<D>(H, xp, ioh, n0, false, lb);
         if (ok) {
-          gather_patch<D, DEG, false, R>(pv, pv + D * NODES, crd, lb, xp, ioh, vref, pic, Bp, flp, gv, apic,
-                                         fr >= -1);
+          gather_patch<D, DEG, false, R>(pv, crd, lb, xp, ioh, vref, pic, Bp, flp, gv, apic, fr >= -1);
         } else {
           raise_status(H, MTR_STATUS_STENCIL_OOB, pid);
 #pragma unroll
@@ -1929,20 +2021,20 @@ __global__ void __launch_bounds__(256) k_musl_norm(StepArgsT<R> A) {
 template <int D, int DEG, typename R, int PM>
 __device__ __forceinline__ void defgrad_t_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid, const uint32_t nblk) {
   using TL = Tiling<D>;
-  constexpr int PN = TL::PN, NODES = TL::NODES;
+  constexpr int PN = TL::PN;
   StepHeader* H = A.H;
   if (step_inactive(H)) return;
   const uint32_t t = bid;
   if (t >= H->ntiles) return;
   const uint32_t pb = A.tile_begin[t], pe = A.tile_end[t];
   if (pb >= pe) return;
-  __shared__ R pv[D * NODES];
+  __shared__ __align__(16) R pv[NodePatch<D, false, R>::SIZE];
   __shared__ double crd[3][PN];
   int n0[3];
   load_tile_setup<D>(A, H, t, n0, crd);
   double vref[3];
   tile_vref<D, R>(A, H, n0, A.v2, vref);
-  load_velocity_patch<D, R>(A, H, n0, A.v2, vref, pv);
+  load_patch<D, false, R>(A, H, n0, A.v2, vref, (const R*)nullptr, false, pv);
   __syncthreads();
   const uint32_t Np = A.Np;
   const double dt = H->dt, ioh = A.P->one_over_dx;
@@ -1951,11 +2043,10 @@ __device__ __forceinline__ void defgrad_t_body(const StepArgsT<R>& A, const uint
     const uint32_t j = perm[s];
     PLoad<D> p;
     load_particle<D, R>(A.in, Np, j, p);
-    double pic[3];
-    R flp[3], Bp[D][D], gv[D][D];
+    R gv[D][D];
     int lb[3];
     if (local_base<D>(H, p.x, ioh, n0, false, lb)) {
-      gather_patch<D, DEG, true, R>(pv, nullptr, crd, lb, p.x, ioh, vref, pic, Bp, flp, gv, false, false);
+      gather_gradv<D, DEG, R>(pv, crd, lb, p.x, ioh, gv);
     } else {
       raise_status(H, MTR_STATUS_STENCIL_OOB, p.id);
 #pragma unroll
