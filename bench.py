@@ -251,10 +251,12 @@ def kernel_bytes(name, p, Np, Ga, G, wr=8.0):
         return G * (2 * wr * (2 + 2 * d) + w8 * d + wr * (d + 1))
     if name == "k_musl_norm":
         return G * (wr + 2 * w8 * d)
-    if name.startswith("k_sort_hist"):
-        return Np * (w8 * d + 4) if "keys" in name else Np * 4
-    if name == "k_sort_scatter":
-        return Np * 16
+    if name == "k_sort_keys":
+        return Np * (w8 * d + 8)
+    if name == "k_sort_place":
+        return Np * 12
+    if name == "k_sort_rank":
+        return Np * 12
     if name == "k_bbox":
         return Np * (w8 * d + wr * d)
     return None

@@ -280,8 +280,8 @@ int mtr_batch_create(mtr_ctx* const* ctxs, int n, mtr_batch** out);
 /* Replaces the members of a batch (no counterpart in the reference): the
  * batch keeps its stream, the block shapes of every group whose key stays in
  * use and its instantiated step graph, which the next mtr_batch_step updates
- * in place when the launch sequence is unchanged (same groups and radix
- * passes) instead of instantiating it again.  A serving loop calls it when
+ * in place when the launch sequence is unchanged (same groups) instead of
+ * instantiating it again.  A serving loop calls it when
  * scenes join or leave.  Members that leave stay alive. */
 int mtr_batch_set_members(mtr_batch* batch, mtr_ctx* const* ctxs, int n);
 /* How many batch rebuilds updated the instantiated graph in place. */
@@ -384,7 +384,7 @@ int mtr_batch_set_tile_threads(mtr_batch* batch, int group, const int* threads /
  * graph, solvers living inside a framework that owns all device memory
  * through its own pool, real-time loops that must not risk an allocation.
  * Nothing is allocated: the sort, tile and accumulator scratch lives in one
- * fixed device array (~10 MB, held by every GPU that loads the library until
+ * fixed device array (~12 MB, held by every GPU that loads the library until
  * exit).  Inputs and outputs are device pointers the caller owns:
  *   x, v  [dim][Np] component-major; B [dim*dim][Np], entry (r,c) at r*dim+c
  *         (read only when params->flip_ratio < 0); gx, gy, gz the node

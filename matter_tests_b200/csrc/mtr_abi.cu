@@ -153,11 +153,9 @@ struct mtr_ctx {
   double *gx = nullptr, *gy = nullptr, *gz = nullptr;
   void *acc = nullptr, *nflip = nullptr, *nmass = nullptr, *nfric = nullptr;
   double *nv = nullptr, *v2 = nullptr;  // node velocities: FP64 on both paths
-  uint32_t *tile_begin = nullptr, *tile_end = nullptr;
   // sort
-  uint32_t *keys0 = nullptr, *keysA = nullptr, *valsA = nullptr, *keysB = nullptr, *valsB = nullptr;
-  uint32_t *hist = nullptr, *dtot = nullptr;
-  int sort_blocks = 0, passes = 0;
+  uint32_t *cell_count = nullptr, *cell_start = nullptr, *super = nullptr;  // with the grid
+  uint32_t *keys0 = nullptr, *perm_rank = nullptr, *perm_tmp = nullptr, *big_cells = nullptr;
   BBoxPartial* partials = nullptr;
   int npartials = 0;
   double* staging = nullptr;  // Np * dim * dim doubles
@@ -340,12 +338,12 @@ T* galloc(mtr_ctx* c, size_t n) {
 
 void free_grid(mtr_ctx* c) {
   for (void* p : {(void*)c->gx, (void*)c->gy, (void*)c->gz, (void*)c->acc, (void*)c->nv,
-                  (void*)c->nflip, (void*)c->nmass, (void*)c->nfric, (void*)c->v2, (void*)c->tile_begin,
-                  (void*)c->tile_end})
+                  (void*)c->nflip, (void*)c->nmass, (void*)c->nfric, (void*)c->v2, (void*)c->cell_count,
+                  (void*)c->cell_start, (void*)c->super})
     if (p) cudaFreeAsync(p, c->stream);
   c->gx = c->gy = c->gz = c->nv = c->v2 = nullptr;
   c->acc = c->nflip = c->nmass = c->nfric = nullptr;
-  c->tile_begin = c->tile_end = nullptr;
+  c->cell_count = c->cell_start = c->super = nullptr;
 }
 
 void free_graphs(mtr_ctx* c) {
@@ -358,6 +356,11 @@ void free_graphs(mtr_ctx* c) {
 
 int tile_edge(int d) { return d == 3 ? 4 : 8; }
 
+// the sort's cells for `tiles` tiles, and one past the grid: blocks of
+// kSuperCells cells, and the entries of the cell arrays (whole blocks)
+uint32_t sort_supers(uint64_t tiles) { return (uint32_t)((tiles * 64 + 1 + kSuperCells - 1) / kSuperCells); }
+size_t sort_cells(uint64_t tiles) { return (size_t)sort_supers(tiles) * kSuperCells; }
+
 // Zeroes the grid channels a fresh grid starts from.
 void clear_grid(mtr_ctx* c) {
   const int d = c->dim;
@@ -368,6 +371,8 @@ void clear_grid(mtr_ctx* c) {
   CK(cudaMemsetAsync(c->nflip, 0, rs * d * nodes, c->stream));
   CK(cudaMemsetAsync(c->nmass, 0, rs * nodes, c->stream));
   CK(cudaMemsetAsync(c->v2, 0, sizeof(double) * d * nodes, c->stream));
+  CK(cudaMemsetAsync(c->cell_count, 0, sizeof(uint32_t) * sort_cells(c->cap_tiles), c->stream));
+  CK(cudaMemsetAsync(c->super, 0, sizeof(uint32_t) * sort_supers(c->cap_tiles), c->stream));
 }
 
 // (Re)allocates the grid for per-axis node capacities.
@@ -380,7 +385,7 @@ void alloc_grid(mtr_ctx* c, const uint32_t want[3]) {
     nodes *= c->cap_axis[a];
     tiles *= (a < d) ? (c->cap_axis[a] + tb - 1) / tb : 1;
   }
-  if (nodes > 0xffffffffull / 8 || tiles * 64ull > 0xffffffffull)
+  if (nodes > 0xffffffffull / 8 || tiles * 64ull > 0xffffffffull - 2 * kSuperCells)
     throw MtrError{MTR_ERR_OOM, "grid capacity exceeds the 32-bit node/key range"};
   c->cap_nodes = (uint32_t)nodes;
   c->cap_tiles = (uint32_t)tiles;
@@ -395,12 +400,10 @@ void alloc_grid(mtr_ctx* c, const uint32_t want[3]) {
   c->nmass = galloc<unsigned char>(c, rs * nodes);
   c->nfric = galloc<unsigned char>(c, rs * nodes);
   c->v2 = galloc<double>(c, (size_t)d * nodes);
-  c->tile_begin = galloc<uint32_t>(c, tiles);
-  c->tile_end = galloc<uint32_t>(c, tiles);
+  c->cell_count = galloc<uint32_t>(c, sort_cells(tiles));
+  c->cell_start = galloc<uint32_t>(c, sort_cells(tiles) + 4);
+  c->super = galloc<uint32_t>(c, sort_supers(tiles));
   clear_grid(c);
-  uint64_t keybits = 1;
-  while ((1ull << keybits) < tiles * 64ull) ++keybits;
-  c->passes = (int)((keybits + 7) / 8);
 }
 
 void mark(mtr_ctx* c, const char* name) { c->marks.record(name, c->stream); }
@@ -459,17 +462,13 @@ StepArgsT<R> make_args(mtr_ctx* c, int parity) {
   A.v2 = c->v2;
   A.xin = c->buf[parity].x;
   A.keys0 = c->keys0;
-  A.keysA = c->keysA;
-  A.valsA = c->valsA;
-  A.keysB = c->keysB;
-  A.valsB = c->valsB;
-  A.hist = c->hist;
-  A.dtot = c->dtot;
-  A.sort_blocks = c->sort_blocks;
-  A.tile_begin = c->tile_begin;
-  A.tile_end = c->tile_end;
-  A.skeys = (c->passes & 1) ? c->keysB : c->keysA;  // where the last radix pass writes
-  A.perm = (c->passes & 1) ? c->valsB : c->valsA;
+  A.perm_rank = c->perm_rank;
+  A.perm_tmp = c->perm_tmp;
+  A.cell_count = c->cell_count;
+  A.cell_start = c->cell_start;
+  A.super = c->super;
+  A.big_cells = c->big_cells;
+  A.perm = c->perm_rank;
   A.out_parity = 1 - parity;
   A.in = typed<R>(c->buf[parity]);
   A.out = typed<R>(c->buf[1 - parity]);
@@ -531,33 +530,17 @@ int enqueue_step_t(mtr_ctx* c, int parity) {
   ++n;
   mark(c, "k_header");
   // sort
-  const uint32_t* skeys = nullptr;
-  const uint32_t* perm = nullptr;
-  for (int pass = 0; pass < c->passes; ++pass) {
-    const int shift = 8 * pass;
-    const uint32_t* ksrc = pass == 0 ? c->keys0 : ((pass & 1) ? c->keysB : c->keysA);
-    const uint32_t* vsrc = pass == 0 ? nullptr : ((pass & 1) ? c->valsB : c->valsA);
-    uint32_t* kdst = (pass & 1) ? c->keysA : c->keysB;
-    uint32_t* vdst = (pass & 1) ? c->valsA : c->valsB;
-    if (pass == 0)
-      k_sort_hist<D, true><<<c->sort_blocks, kSortThreads, 0, st>>>(A, nullptr, shift);
-    else
-      k_sort_hist<D, false><<<c->sort_blocks, kSortThreads, 0, st>>>(A, ksrc, shift);
-    mark(c, pass == 0 ? "k_sort_hist(keys)" : "k_sort_hist");
-    k_sort_scan<<<256, 256, 0, st>>>(A);
-    mark(c, "k_sort_scan");
-    k_sort_scatter<<<c->sort_blocks, kSortThreads, 0, st>>>(A, ksrc, vsrc, kdst, vdst, shift);
-    mark(c, "k_sort_scatter");
-    n += 3;
-    skeys = kdst;
-    perm = vdst;
-  }
-  CK(cudaMemsetAsync(c->tile_begin, 0, sizeof(uint32_t) * c->cap_tiles, st));
-  CK(cudaMemsetAsync(c->tile_end, 0, sizeof(uint32_t) * c->cap_tiles, st));
-  mark(c, "memset(tiles)");
-  k_tile_ranges<<<std::min<uint32_t>((c->Np + 255) / 256, 148 * 8), 256, 0, st>>>(A, skeys);
-  ++n;
-  mark(c, "k_tile_ranges");
+  const uint32_t pblocks = (c->Np + kSortThreads - 1) / kSortThreads;
+  k_sort_keys<D><<<pblocks, kSortThreads, 0, st>>>(A);
+  mark(c, "k_sort_keys");
+  k_sort_scan<<<sort_supers(c->cap_tiles), kSortThreads, 0, st>>>(A);
+  mark(c, "k_sort_scan");
+  k_sort_place<<<pblocks, kSortThreads, 0, st>>>(A);
+  mark(c, "k_sort_place");
+  k_sort_rank<<<pblocks, kSortThreads, 0, st>>>(A);
+  mark(c, "k_sort_rank");
+  n += 4;
+  const uint32_t* perm = c->perm_rank;
   const int* tt = c->tile_threads;
   {
     const size_t sm = p2g_smem_bytes<D, R>(tt[kSlotP2G], c->prm.use_mibf != 0);
@@ -578,8 +561,6 @@ int enqueue_step_t(mtr_ctx* c, int parity) {
   ++n;
   mark(c, "k_grid");
   if (c->prm.use_musl) {
-    CK(cudaMemsetAsync(c->v2, 0, sizeof(double) * D * c->cap_nodes, st));
-    mark(c, "memset(v2)");
     const size_t sm = musl_smem_bytes<D, R>(tt[kSlotMUSL]);
     if (c->tile_split[kSlotMUSL] == 2)
       k_g2p_musl_w<D, DEG, R, 2><<<c->cap_tiles, tt[kSlotMUSL], sm, st>>>(A, perm);
@@ -843,7 +824,6 @@ struct mtr_batch_group {
   int dim = 3, deg = 2, musl = 0;
   int spm = -1;  // plastic model the return-mapping kernel is compiled for (-1: any)
   bool fp32 = false;
-  int passes = 1;
   std::vector<mtr_ctx*> members;
   void* dargs = nullptr;      // StepArgsT<R>[2][n]
   uint32_t* doff = nullptr;   // [kBK_KINDS][n + 1]
@@ -903,21 +883,15 @@ void free_batch_tables(mtr_batch* b) {
 template <typename R>
 void build_group_tables(mtr_batch* b, mtr_batch_group& g) {
   const int n = (int)g.members.size();
-  g.passes = 1;
-  for (mtr_ctx* c : g.members) g.passes = std::max(g.passes, c->passes);
   std::vector<StepArgsT<R>> args((size_t)2 * n);
   std::vector<uint32_t> off((size_t)kBK_KINDS * (n + 1), 0u);
   for (int s = 0; s < n; ++s) {
     mtr_ctx* c = g.members[s];
-    if (c->passes != g.passes) free_graphs(c);  // its own graphs were captured with fewer passes
-    c->passes = g.passes;                      // extra radix passes over zero digits keep the order
     for (int par = 0; par < 2; ++par) args[(size_t)par * n + s] = make_args<R>(c, par);
     const uint32_t cnt[kBK_KINDS] = {
         (uint32_t)c->npartials,
-        (uint32_t)c->sort_blocks,
-        (uint32_t)(256 / kScanDigitsPerBlock),
-        cap_blocks(c->Np, 256, 148 * 8),
-        cap_blocks(std::max<uint64_t>(c->cap_tiles, g.musl ? (uint64_t)g.dim * c->cap_nodes : 0), 256, 148 * 8),
+        (c->Np + kSortThreads - 1) / kSortThreads,
+        sort_supers(c->cap_tiles),
         c->cap_tiles,
         cap_blocks(c->cap_nodes, 256, 148 * 16),
         1u};
@@ -946,23 +920,19 @@ int enqueue_group_step_t(mtr_batch* b, mtr_batch_group& g, int gi) {
   int n = 0;
   kb_bbox<D, R><<<g.total[kBK_BBOX], 256, 0, st>>>(B);
   kb_header<D, R><<<g.total[kBK_ONE], 256, 0, st>>>(B);
-  kb_clear<D, R><<<g.total[kBK_CLEAR], 256, 0, st>>>(B);
-  n += 3;
-  for (int pass = 0; pass < g.passes; ++pass) {
-    kb_sort_hist<D, R><<<g.total[kBK_SORT], kSortThreads, 0, st>>>(B, pass);
-    kb_sort_scan<R><<<g.total[kBK_SCAN], 256, 0, st>>>(B);
-    kb_sort_scatter<R><<<g.total[kBK_SORT], kSortThreads, 0, st>>>(B, pass);
-    n += 3;
-  }
-  kb_tile_ranges<R><<<g.total[kBK_TILES], 256, 0, st>>>(B);
-  b->marks.record("kb_tile_ranges", st, gi);
+  kb_sort_keys<D, R><<<g.total[kBK_SORT], kSortThreads, 0, st>>>(B);
+  kb_sort_scan<R><<<g.total[kBK_SCAN], kSortThreads, 0, st>>>(B);
+  kb_sort_place<R><<<g.total[kBK_SORT], kSortThreads, 0, st>>>(B);
+  kb_sort_rank<R><<<g.total[kBK_SORT], kSortThreads, 0, st>>>(B);
+  n += 6;
+  b->marks.record("kb_sort", st, gi);
   const uint32_t tiles = g.total[kBK_TILEK];
   launch_tiles<R>(g.tile_split[kSlotP2G] == 2 ? kb_p2g_w<D, DEG, R, 2> : kb_p2g_w<D, DEG, R, 1>, tiles,
                   tt[kSlotP2G], p2g_smem_bytes<D, R>(tt[kSlotP2G]), st, B);
   b->marks.record(kSlotMark[kSlotP2G], st, gi);
   kb_grid<D, R><<<g.total[kBK_NODES], 256, 0, st>>>(B);
   b->marks.record("kb_grid", st, gi);
-  n += 3;
+  n += 2;
   if (g.musl) {
     launch_tiles<R>(g.tile_split[kSlotMUSL] == 2 ? kb_g2p_musl_w<D, DEG, R, 2> : kb_g2p_musl_w<D, DEG, R, 1>,
                     tiles, tt[kSlotMUSL], musl_smem_bytes<D, R>(tt[kSlotMUSL]), st, B);
@@ -1237,8 +1207,8 @@ int mtr_upload(mtr_ctx* c, const double* x, const double* v, const double* F, co
       free_graphs(c);
       for (void* p : c->pallocs) dfree(p);
       c->pallocs.clear();
-      for (void* p : {(void*)c->keys0, (void*)c->keysA, (void*)c->valsA, (void*)c->keysB, (void*)c->valsB,
-                      (void*)c->hist, (void*)c->dtot, (void*)c->partials, (void*)c->staging})
+      for (void* p : {(void*)c->keys0, (void*)c->perm_rank, (void*)c->perm_tmp, (void*)c->big_cells,
+                      (void*)c->partials, (void*)c->staging})
         dfree(p);
       c->Np = Np;
       c->hp.Np = Np;
@@ -1261,14 +1231,10 @@ int mtr_upload(mtr_ctx* c, const double* x, const double* v, const double* F, co
       c->flip = dalloc<unsigned char>(rs * Np * d);
       c->pallocs.push_back(c->pic);
       c->pallocs.push_back(c->flip);
-      c->sort_blocks = (int)((Np + kSortTile - 1) / kSortTile);
       c->keys0 = dalloc<uint32_t>(Np);
-      c->keysA = dalloc<uint32_t>(Np);
-      c->valsA = dalloc<uint32_t>(Np);
-      c->keysB = dalloc<uint32_t>(Np);
-      c->valsB = dalloc<uint32_t>(Np);
-      c->hist = dalloc<uint32_t>((size_t)256 * c->sort_blocks);
-      c->dtot = dalloc<uint32_t>(256);
+      c->perm_rank = dalloc<uint32_t>(Np);
+      c->perm_tmp = dalloc<uint32_t>(Np);
+      c->big_cells = dalloc<uint32_t>(Np / kBigCell + 1);
       c->npartials = (int)std::min<uint32_t>((Np + 255) / 256, 148 * 8);
       c->partials = dalloc<BBoxPartial>(c->npartials);
       c->staging = dalloc<double>((size_t)Np * std::max<int>(dd, (int)MTR_NUM_SCALARS));
@@ -1581,9 +1547,8 @@ int mtr_get_sort(mtr_ctx* c, uint32_t* keys_in_input_order, uint32_t* sorted_inp
     CK(cudaSetDevice(c->device));
     read_header(c);
     const uint32_t Np = c->Np;
-    const uint32_t* perm = (c->passes & 1) ? c->valsB : c->valsA;
     if (keys_in_input_order) CK(cudaMemcpy(keys_in_input_order, c->keys0, sizeof(uint32_t) * Np, cudaMemcpyDeviceToHost));
-    if (sorted_input_index) CK(cudaMemcpy(sorted_input_index, perm, sizeof(uint32_t) * Np, cudaMemcpyDeviceToHost));
+    if (sorted_input_index) CK(cudaMemcpy(sorted_input_index, c->perm_rank, sizeof(uint32_t) * Np, cudaMemcpyDeviceToHost));
     if (input_particle_id)
       CK(cudaMemcpy(input_particle_id, c->buf[1 - c->hH->cur].id, sizeof(uint32_t) * Np, cudaMemcpyDeviceToHost));
     return MTR_OK;
@@ -2002,10 +1967,9 @@ int mtr_footprint(const mtr_params* params, uint32_t Np, const double* x, uint64
     if ((p.dim != 2 && p.dim != 3) || !(p.dx > 0)) throw MtrError{MTR_ERR_INVALID, "dim must be 2 or 3, dx > 0"};
     const uint64_t d = p.dim, dd = d * d, ns = p.dim == 3 ? 6 : 3, n = Np;
     const uint64_t rs = p.precision == MTR_PREC_MIXED ? 4 : 8;
-    const uint64_t sort_blocks = (n + kSortTile - 1) / kSortTile;
     uint64_t total = 2 * (8 * d * n + rs * n * (d + 2 * dd + MTR_NUM_SCALARS + ns) + 4 * n)  // particle buffers
                      + 2 * rs * d * n                                                      // pic, flip
-                     + 5 * 4 * n + 4 * 256 * sort_blocks + 4 * 256                           // sort
+                     + 3 * 4 * n + 4 * (n / kBigCell + 1)                                    // sort
                      + 8 * n * std::max<uint64_t>(dd, MTR_NUM_SCALARS);                       // staging
     uint32_t want[3];
     grid_extent(p, Np, x, want);
@@ -2018,7 +1982,7 @@ int mtr_footprint(const mtr_params* params, uint32_t Np, const double* x, uint64
       axes += cap;
     }
     total += 8 * axes + rs * (2 + 2 * d) * nodes + 8 * d * nodes + rs * d * nodes + 2 * rs * nodes + 8 * d * nodes +
-             8 * tiles;
+             4 * (2 * sort_cells(tiles) + sort_supers(tiles));
     *bytes = total;
     return MTR_OK;
   });
@@ -2390,8 +2354,8 @@ void mtr_ctx_destroy(mtr_ctx* c) {
   free_graphs(c);
   free_grid(c);
   for (void* p : c->pallocs) dfree(p);
-  for (void* p : {(void*)c->keys0, (void*)c->keysA, (void*)c->valsA, (void*)c->keysB, (void*)c->valsB,
-                  (void*)c->hist, (void*)c->dtot, (void*)c->partials, (void*)c->staging, (void*)c->dP, (void*)c->dH})
+  for (void* p : {(void*)c->keys0, (void*)c->perm_rank, (void*)c->perm_tmp, (void*)c->big_cells, (void*)c->partials,
+                  (void*)c->staging, (void*)c->dP, (void*)c->dH})
     dfree(p);
   if (c->hH) cudaFreeHost(c->hH);
   if (c->stream) cudaStreamDestroy(c->stream);

@@ -80,6 +80,7 @@ struct StepHeader {
   uint32_t G;           // grid_nodes
   uint32_t T[3];        // tiles per axis
   uint32_t ntiles;
+  uint32_t nbig;        // cells of this step's sort with more than kBigCell particles
   double min_init[3], max_init[3], low_init[3], high_init[3];
   unsigned long long plastic_count;
   // FP64 balances of the last step (simulation.cpp:292-333): grid mass and

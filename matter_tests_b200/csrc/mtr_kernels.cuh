@@ -4,8 +4,8 @@
 // Step pipeline (all on one stream, no host round trip, CUDA-graph capturable):
 //   k_bbox        per-block min/max x, max |v|^2 and sum v    update_dt.cpp, remesh.cpp
 //   k_header      dt, gravity ramp, remesh + arange axes      update_dt.cpp:5-66, remesh.cpp:38-311
-//   k_sort_*      stable LSD radix sort by blocked cell key   (new: locality for P2G)
-//   k_tile_ranges particle range of every 4^3 (2D: 8^2) tile
+//   k_sort_*      stable counting sort by blocked cell key    (new: locality for P2G); the cell
+//                 starts it leaves are the particle ranges of every cell and 4^3 (2D: 8^2) tile
 //   k_p2g_w       tile block -> shared grid patch -> one global atomic per node and channel
 //                 (mass, momentum with APIC, force tau.grad w, MIBF friction)
 //                                                              p2g.cpp:6-100, explicit_euler_update.cpp:15-77
@@ -68,15 +68,14 @@ struct StepCommon {
   uint32_t cap_nodes;
   uint32_t cap_tiles;
   const double* xin;  // positions of the step's input buffer (sort keys)
-  uint32_t* keys0;    // cell key of each particle in input order
-  uint32_t *keysA, *valsA, *keysB, *valsB;
-  uint32_t* hist;  // [256][sort_blocks]
-  uint32_t* dtot;  // [256]
-  int sort_blocks;
-  uint32_t* tile_begin;
-  uint32_t* tile_end;
-  const uint32_t* skeys;  // sorted keys and permutation after the last radix pass
-  const uint32_t* perm;
+  uint32_t* keys0;      // cell key of each particle in input order
+  uint32_t* perm_rank;  // rank of each particle among its cell's arrivals, then the sorted permutation
+  uint32_t* perm_tmp;   // permutation with the cells in order and each cell's particles in arrival order
+  uint32_t* cell_count; // [cap_tiles * 64 + 1], zero between steps
+  uint32_t* cell_start; // [cap_tiles * 64 + 2]: first sorted particle of each cell of the last sort
+  uint32_t* super;      // particles of each kSuperCells cells, zero between steps
+  uint32_t* big_cells;  // cells with more than kBigCell particles (H->nbig of them)
+  const uint32_t* perm; // = perm_rank, the sorted permutation
   int out_parity;         // particle buffer this step writes
 };
 
@@ -99,8 +98,8 @@ constexpr bool kFP64 = std::is_same<R, double>::value;
 
 constexpr uint32_t kMaxAxisNodes = 1u << 22;
 constexpr int kSortThreads = 256;
-constexpr int kSortItems = 8;
-constexpr int kSortTile = kSortThreads * kSortItems;
+constexpr int kSuperCells = 4096;  // cells scanned by one block of k_sort_scan
+constexpr uint32_t kBigCell = 1024;  // cells with more particles are ordered by a whole block
 
 template <int D>
 struct Tiling {
@@ -270,6 +269,7 @@ __device__ __forceinline__ void header_body(const StepCommon& A) {
   __shared__ double s_low[3], s_high[3], s_stop[3];
   __shared__ int s_ok;
   if (lane == 0) {
+    H->nbig = 0;
     // balances of this step (read back by mtr_balance)
     H->grid_mass = 0.0;
 #pragma unroll
@@ -397,7 +397,30 @@ __global__ void __launch_bounds__(256) k_header(StepCommon A) {
 }
 
 // ---------------------------------------------------------------------------
-// 3. stable LSD radix sort of (blocked cell key, input position)
+// 3. stable counting sort of (blocked cell key, input position), four launches:
+//   k_sort_keys   key of every particle; its arrival rank in the cell from one
+//                 atomic per warp and cell; counts per cell and per kSuperCells cells
+//   k_sort_scan   exclusive scan of the cell counts (one block per kSuperCells
+//                 cells, whose base is the sum of the super counts before it);
+//                 leaves cell_start and clears the counts for the next step
+//   k_sort_place  particle index to cell_start + arrival rank
+//   k_sort_rank   stable order inside each cell: a particle's place is the
+//                 number of smaller indices in its cell
+// The last state is nearly in cell order, so all accesses are nearly
+// coalesced.  Bound: launches and memory latency.  An LSD radix sort of the
+// same keys needs three launches per 8-bit digit (9 for the 18-bit keys of the
+// 1M-particle collapse) and a pass over the sorted keys for the tile ranges,
+// which here are cell_start itself.
+// Measured on a B200, per step: the radix sort with its memsets and tile ranges
+// 11-16 launches and about 80 us at 1,024,000 particles; this one 4 launches,
+// 49 us (CUDA events around every launch, 4 us each of which is the event).
+// Whole steps: 5k particles in 2D 122 -> 100 us, 51,200 in 2D 138 -> 111 us,
+// 150k in 3D 250 -> 210 us, 1,024,000 in 3D FP64 1123 -> 1089 us.
+// A cell's ranking is quadratic in its particles (about 8 in 3D), which up to
+// kBigCell of them costs less than another launch; larger cells are ordered by
+// a whole block that walks the keys once.
+// Keys past the grid's cells (particles outside every tile) share one cell
+// after the last, which no tile reads.
 // ---------------------------------------------------------------------------
 template <int D>
 __device__ __forceinline__ uint32_t cell_key(const StepHeader* H, double ioh, const double (&x)[3]) {
@@ -416,192 +439,196 @@ __device__ __forceinline__ uint32_t cell_key(const StepHeader* H, double ioh, co
   return t * 64u + in;
 }
 
-// Per-block digit histogram.  The first pass computes the keys from x.
-template <int D, bool FIRST>
-__device__ __forceinline__ void sort_hist_body(const StepCommon& A, const uint32_t* __restrict__ keys,
-                                                            int shift, const uint32_t bid, const uint32_t nblk) {
-  if (step_inactive(A.H)) return;
-  __shared__ uint32_t h[256];
-  h[threadIdx.x] = 0;
-  __syncthreads();
-  const uint32_t base = bid * kSortTile;
-  const double ioh = A.P->one_over_dx;
-#pragma unroll
-  for (int r = 0; r < kSortItems; ++r) {
-    uint32_t i = base + r * kSortThreads + threadIdx.x;
-    if (i < A.Np) {
-      uint32_t k;
-      if (FIRST) {
-        double x[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int a = 0; a < D; ++a) x[a] = A.xin[(size_t)a * A.Np + i];
-        k = cell_key<D>(A.H, ioh, x);
-        A.keys0[i] = k;
-      } else {
-        k = keys[i];
-      }
-      atomicAdd(&h[(k >> shift) & 255u], 1u);
-    }
+__device__ __forceinline__ uint32_t sort_cell(const StepHeader* H, uint32_t key) {
+  const uint32_t last = H->ntiles * 64u;
+  return key < last ? key : last;
+}
+
+// counts the key of particle i (all threads of the block call) and keeps its
+// arrival rank.  The super counts are few, so their atomics are merged over the
+// block: one per run of warps that lie within the same kSuperCells cells.
+__device__ __forceinline__ void sort_count(const StepCommon& A, uint32_t i, bool valid, uint32_t key) {
+  __shared__ uint32_t wsup[kSortThreads / 32], wnum[kSortThreads / 32];
+  const uint32_t cell = valid ? sort_cell(A.H, key) : 0xffffffffu;
+  const unsigned peers = __match_any_sync(0xffffffffu, cell);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, leader = __ffs(peers) - 1;
+  uint32_t first = 0;
+  if (valid && lane == leader) first = atomicAdd(&A.cell_count[cell], (uint32_t)__popc(peers));
+  const uint32_t sup = valid ? cell / kSuperCells : 0xffffffffu;
+  const unsigned speers = __match_any_sync(0xffffffffu, sup);
+  if (lane == 0) {
+    wsup[warp] = sup;
+    wnum[warp] = valid ? (uint32_t)__popc(speers) : 0u;
+  } else if (valid && lane == __ffs(speers) - 1) {
+    atomicAdd(&A.super[sup], (uint32_t)__popc(speers));
   }
   __syncthreads();
-  A.hist[threadIdx.x * A.sort_blocks + bid] = h[threadIdx.x];
+  if (threadIdx.x == 0) {
+    uint32_t s = wsup[0], n = wnum[0];
+#pragma unroll
+    for (int w = 1; w < kSortThreads / 32; ++w) {
+      if (wsup[w] != s) {
+        if (n) atomicAdd(&A.super[s], n);
+        s = wsup[w];
+        n = 0;
+      }
+      n += wnum[w];
+    }
+    if (n) atomicAdd(&A.super[s], n);
+  }
+  first = __shfl_sync(0xffffffffu, first, leader);
+  if (valid) A.perm_rank[i] = first + __popc(peers & ((1u << lane) - 1u));
 }
 
-template <int D, bool FIRST>
-__global__ void __launch_bounds__(kSortThreads) k_sort_hist(StepCommon A, const uint32_t* __restrict__ keys,
-                                                            int shift) {
-  sort_hist_body<D, FIRST>(A, keys, shift, blockIdx.x, gridDim.x);
-}
-
-// Exclusive scan of each digit's row over the blocks; row totals to dtot.
-static __device__ __forceinline__ void sort_scan_body(const StepCommon& A, const uint32_t bid, const uint32_t nblk) {
+template <int D>
+__device__ __forceinline__ void sort_keys_body(const StepCommon& A, const uint32_t bid) {
   if (step_inactive(A.H)) return;
-  const int dgt = bid;
-  uint32_t* row = A.hist + (size_t)dgt * A.sort_blocks;
+  const uint32_t i = bid * kSortThreads + threadIdx.x;
+  const bool valid = i < A.Np;
+  uint32_t k = 0;
+  if (valid) {
+    double x[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int a = 0; a < D; ++a) x[a] = A.xin[(size_t)a * A.Np + i];
+    k = cell_key<D>(A.H, A.P->one_over_dx, x);
+    A.keys0[i] = k;
+  }
+  sort_count(A, i, valid, k);
+}
+
+template <int D>
+__global__ void __launch_bounds__(kSortThreads) k_sort_keys(StepCommon A) {
+  sort_keys_body<D>(A, blockIdx.x);
+}
+
+// sum over the block's 256 threads, to every thread; `ws` holds 8 values
+__device__ __forceinline__ uint32_t block_sum256(uint32_t v, uint32_t* ws) {
+  v = __reduce_add_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+  __syncthreads();
+  uint32_t s = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) s += ws[w];
+  __syncthreads();
+  return s;
+}
+
+// exclusive prefix over the block's 256 threads; total to every thread
+__device__ __forceinline__ uint32_t block_prefix256(uint32_t v, uint32_t* ws, uint32_t& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t incl = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += u;
+  }
+  if (lane == 31) ws[warp] = incl;
+  __syncthreads();
+  uint32_t pre = 0, sum = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    pre += w < warp ? ws[w] : 0u;
+    sum += ws[w];
+  }
+  __syncthreads();
+  total = sum;
+  return pre + incl - v;
+}
+
+static __device__ __forceinline__ void sort_scan_body(const StepCommon& A, const uint32_t bid) {
+  StepHeader* H = A.H;
+  if (step_inactive(H)) return;
+  const uint32_t ncell = H->ntiles * 64u + 1u, first = bid * kSuperCells;  // the last one: past the grid
+  if (first >= ncell) return;
   __shared__ uint32_t ws[8];
-  __shared__ uint32_t carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int b0 = 0; b0 < A.sort_blocks; b0 += 256) {
-    int b = b0 + threadIdx.x;
-    uint32_t v = b < A.sort_blocks ? row[b] : 0u;
-    uint32_t incl = v;
+  uint32_t before = 0;
+  for (uint32_t s = threadIdx.x; s < bid; s += kSortThreads) before += A.super[s];
+  const uint32_t base = block_sum256(before, ws);
+  constexpr int PER = kSuperCells / kSortThreads;
+  uint4* cnt = reinterpret_cast<uint4*>(A.cell_count + first) + threadIdx.x * (PER / 4);
+  uint4* out = reinterpret_cast<uint4*>(A.cell_start + first) + threadIdx.x * (PER / 4);
+  uint32_t c[PER], sum = 0;
 #pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
-      if ((threadIdx.x & 31) >= off) incl += t;
-    }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 31) ws[warp] = incl;
-    __syncthreads();
-    uint32_t wpre = 0;
-    for (int w = 0; w < warp; ++w) wpre += ws[w];
-    uint32_t total = 0;
-    for (int w = 0; w < 8; ++w) total += ws[w];
-    if (b < A.sort_blocks) row[b] = carry + wpre + incl - v;
-    __syncthreads();
-    if (threadIdx.x == 0) carry += total;
-    __syncthreads();
+  for (int q = 0; q < PER / 4; ++q) {
+    const uint4 u = cnt[q];
+    c[4 * q] = u.x;
+    c[4 * q + 1] = u.y;
+    c[4 * q + 2] = u.z;
+    c[4 * q + 3] = u.w;
   }
-  if (threadIdx.x == 0) A.dtot[dgt] = carry;
+#pragma unroll
+  for (int q = 0; q < PER; ++q) sum += c[q];
+  uint32_t total;
+  uint32_t at = base + block_prefix256(sum, ws, total);
+  if (sum) {
+#pragma unroll
+    for (int q = 0; q < PER / 4; ++q) cnt[q] = make_uint4(0u, 0u, 0u, 0u);
+  }
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const uint32_t n = c[q], cell = first + threadIdx.x * PER + q;
+    if (n > kBigCell && cell + 1 < ncell) A.big_cells[atomicAdd(&H->nbig, 1u)] = cell;
+    c[q] = at;
+    at += n;
+  }
+#pragma unroll
+  for (int q = 0; q < PER / 4; ++q) out[q] = make_uint4(c[4 * q], c[4 * q + 1], c[4 * q + 2], c[4 * q + 3]);
 }
 
-static __global__ void __launch_bounds__(256) k_sort_scan(StepCommon A) {
-  sort_scan_body(A, blockIdx.x, gridDim.x);
-}
+static __global__ void __launch_bounds__(kSortThreads) k_sort_scan(StepCommon A) { sort_scan_body(A, blockIdx.x); }
 
-// The same scan with one warp per digit, kScanDigitsPerBlock digits per
-// 256-thread block: the batched form, where most scenes have few sort blocks
-// and a block per digit and scene would leave the blocks nearly idle.
-constexpr int kScanDigitsPerBlock = 8;
-static __device__ __forceinline__ void sort_scan_warp_body(const StepCommon& A, const uint32_t bid) {
+static __device__ __forceinline__ void sort_place_body(const StepCommon& A, const uint32_t bid) {
   if (step_inactive(A.H)) return;
-  const int lane = threadIdx.x & 31;
-  const int dgt = (int)bid * kScanDigitsPerBlock + (int)(threadIdx.x >> 5);
-  if (dgt >= 256) return;  // no block-wide barrier below
-  uint32_t* row = A.hist + (size_t)dgt * A.sort_blocks;
-  uint32_t carry = 0;
-  for (int b0 = 0; b0 < A.sort_blocks; b0 += 32) {
-    const int b = b0 + lane;
-    const uint32_t v = b < A.sort_blocks ? row[b] : 0u;
-    uint32_t incl = v;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += t;
-    }
-    if (b < A.sort_blocks) row[b] = carry + incl - v;
-    carry += __shfl_sync(0xffffffffu, incl, 31);
-  }
-  if (lane == 0) A.dtot[dgt] = carry;
+  if (bid == 0)  // the scan has read the super counts
+    for (uint32_t s = threadIdx.x; s * kSuperCells <= A.H->ntiles * 64u; s += kSortThreads) A.super[s] = 0u;
+  const uint32_t i = bid * kSortThreads + threadIdx.x;
+  if (i < A.Np) A.perm_tmp[A.cell_start[sort_cell(A.H, A.keys0[i])] + A.perm_rank[i]] = i;
 }
 
-// Stable scatter.  Elements are ranked round by round (256 at a time, in
-// index order) with warp match + per-warp digit counts, which keeps equal
-// digits in input order.
-static __device__ __forceinline__ void sort_scatter_body(const StepCommon& A, const uint32_t* __restrict__ ksrc,
-                                                               const uint32_t* __restrict__ vsrc, uint32_t* kdst,
-                                                               uint32_t* vdst, int shift, const uint32_t bid, const uint32_t nblk) {
-  if (step_inactive(A.H)) return;
-  __shared__ uint32_t goff[256];
-  __shared__ uint32_t run[256];
-  __shared__ uint32_t wcnt[kSortThreads / 32][256];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  {  // digit base = exclusive prefix of digit totals, plus this block's row offset
-    uint32_t v = A.dtot[tid];
-    uint32_t incl = v;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += t;
-    }
-    __shared__ uint32_t ws[8];
-    if (lane == 31) ws[warp] = incl;
-    __syncthreads();
-    uint32_t wpre = 0;
-    for (int w = 0; w < warp; ++w) wpre += ws[w];
-    goff[tid] = wpre + incl - v + A.hist[(size_t)tid * A.sort_blocks + bid];
-    run[tid] = 0;
-  }
-  const uint32_t base = bid * kSortTile;
-  const unsigned lt_mask = (1u << lane) - 1u;
-  for (int r = 0; r < kSortItems; ++r) {
-#pragma unroll
-    for (int w = 0; w < kSortThreads / 32; ++w) wcnt[w][tid] = 0;
-    __syncthreads();
-    const uint32_t i = base + r * kSortThreads + tid;
-    const bool valid = i < A.Np;
-    uint32_t k = 0, val = 0, dgt = 256;
-    if (valid) {
-      k = ksrc[i];
-      val = vsrc ? vsrc[i] : i;
-      dgt = (k >> shift) & 255u;
-    }
-    const unsigned peers = __match_any_sync(0xffffffffu, dgt);
-    const uint32_t rank = __popc(peers & lt_mask);
-    if (valid && rank == 0) wcnt[warp][dgt] = __popc(peers);
-    __syncthreads();
-    {  // exclusive prefix over warps per digit, on top of earlier rounds
-      uint32_t acc = run[tid];
-#pragma unroll
-      for (int w = 0; w < kSortThreads / 32; ++w) {
-        uint32_t c = wcnt[w][tid];
-        wcnt[w][tid] = acc;
-        acc += c;
+static __global__ void __launch_bounds__(kSortThreads) k_sort_place(StepCommon A) { sort_place_body(A, blockIdx.x); }
+
+static __device__ __forceinline__ void sort_rank_body(const StepCommon& A, const uint32_t bid, const uint32_t nblk) {
+  const StepHeader* H = A.H;
+  if (step_inactive(H)) return;
+  const uint32_t p = bid * kSortThreads + threadIdx.x;
+  if (p < A.Np) {
+    const uint32_t i = A.perm_tmp[p], cell = A.keys0[i];
+    if (cell >= H->ntiles * 64u) {
+      A.perm_rank[p] = i;
+    } else {
+      const uint32_t b = A.cell_start[cell], e = A.cell_start[cell + 1];
+      if (e - b <= kBigCell) {
+        uint32_t r = b;
+        for (uint32_t q = b; q < e; ++q) r += A.perm_tmp[q] < i ? 1u : 0u;
+        A.perm_rank[r] = i;
       }
-      run[tid] = acc;
     }
-    __syncthreads();
-    if (valid) {
-      const uint32_t pos = goff[dgt] + wcnt[warp][dgt] + rank;
-      kdst[pos] = k;
-      vdst[pos] = val;
+  }
+  const uint32_t nbig = H->nbig;
+  if (bid >= nbig) return;  // the whole block together below
+  __shared__ uint32_t ws[8];
+  for (uint32_t g = bid; g < nbig; g += nblk) {
+    const uint32_t cell = A.big_cells[g];
+    uint32_t at = A.cell_start[cell];
+    for (uint32_t i0 = 0; i0 < A.Np; i0 += kSortThreads) {
+      const uint32_t i = i0 + threadIdx.x;
+      const bool mine = i < A.Np && A.keys0[i] == cell;
+      uint32_t total;
+      const uint32_t pre = block_prefix256(mine ? 1u : 0u, ws, total);
+      if (mine) A.perm_rank[at + pre] = i;
+      at += total;
     }
-    __syncthreads();
   }
 }
 
-static __global__ void __launch_bounds__(kSortThreads) k_sort_scatter(StepCommon A, const uint32_t* __restrict__ ksrc,
-                                                               const uint32_t* __restrict__ vsrc, uint32_t* kdst,
-                                                               uint32_t* vdst, int shift) {
-  sort_scatter_body(A, ksrc, vsrc, kdst, vdst, shift, blockIdx.x, gridDim.x);
+static __global__ void __launch_bounds__(kSortThreads) k_sort_rank(StepCommon A) {
+  sort_rank_body(A, blockIdx.x, gridDim.x);
 }
 
-// ---------------------------------------------------------------------------
-// 4. tile ranges over the sorted keys
-// ---------------------------------------------------------------------------
-static __device__ __forceinline__ void tile_ranges_body(const StepCommon& A, const uint32_t* __restrict__ skeys, const uint32_t bid, const uint32_t nblk) {
-  if (step_inactive(A.H)) return;
-  for (uint32_t s = bid * blockDim.x + threadIdx.x; s < A.Np; s += nblk * blockDim.x) {
-    const uint32_t t = skeys[s] >> 6;
-    if (t >= A.cap_tiles) continue;
-    if (s == 0 || (skeys[s - 1] >> 6) != t) A.tile_begin[t] = s;
-    if (s == A.Np - 1 || (skeys[s + 1] >> 6) != t) A.tile_end[t] = s + 1;
-  }
-}
-
-static __global__ void __launch_bounds__(256) k_tile_ranges(StepCommon A, const uint32_t* __restrict__ skeys) {
-  tile_ranges_body(A, skeys, blockIdx.x, gridDim.x);
+// particles [pb, pe) of tile t
+__device__ __forceinline__ void tile_range(const StepCommon& A, uint32_t t, uint32_t& pb, uint32_t& pe) {
+  pb = A.cell_start[t * 64u];
+  pe = A.cell_start[t * 64u + 64u];
 }
 
 template <int D>
@@ -823,7 +850,8 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
   if (step_inactive(H)) return;
   const uint32_t t = bid;
   if (t >= H->ntiles) return;
-  const uint32_t pb = A.tile_begin[t], pe = A.tile_end[t];
+  uint32_t pb, pe;
+  tile_range(A, t, pb, pe);
   if (pb >= pe) return;
   const DevParams& P = *A.P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1267,6 +1295,10 @@ __device__ __forceinline__ void grid_body(const StepArgsT<R>& A, const uint32_t 
     }
     A.nmass[l] = (R)mi;
     if (P.use_mibf) A.nfric[l] = (R)fric;
+    if (P.use_musl) {
+#pragma unroll
+      for (int a = 0; a < D; ++a) A.v2[(size_t)a * cap + l] = 0.0;  // re-projection accumulator of this step
+    }
 #pragma unroll
     for (int ch = 0; ch < Tiling<D>::NCH; ++ch) A.acc[(size_t)ch * cap + l] = R(0.0);  // ready for the next step
   }
@@ -1665,7 +1697,8 @@ __device__ __forceinline__ void g2p_t_body(const StepArgsT<R>& A, const uint32_t
   if (step_inactive(H)) return;
   const uint32_t t = bid;
   if (t >= H->ntiles) return;
-  const uint32_t pb = A.tile_begin[t], pe = A.tile_end[t];
+  uint32_t pb, pe;
+  tile_range(A, t, pb, pe);
   if (pb >= pe) return;
   const DevParams& P = *A.P;
   __shared__ __align__(16) R pv[NodePatch<D, true, R>::SIZE];
@@ -1790,7 +1823,8 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
   if (step_inactive(H)) return;
   const uint32_t t = bid;
   if (t >= H->ntiles) return;
-  const uint32_t pb = A.tile_begin[t], pe = A.tile_end[t];
+  uint32_t pb, pe;
+  tile_range(A, t, pb, pe);
   if (pb >= pe) return;
   const DevParams& P = *A.P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -2026,7 +2060,8 @@ __device__ __forceinline__ void defgrad_t_body(const StepArgsT<R>& A, const uint
   if (step_inactive(H)) return;
   const uint32_t t = bid;
   if (t >= H->ntiles) return;
-  const uint32_t pb = A.tile_begin[t], pe = A.tile_end[t];
+  uint32_t pb, pe;
+  tile_range(A, t, pb, pe);
   if (pb >= pe) return;
   __shared__ __align__(16) R pv[NodePatch<D, false, R>::SIZE];
   __shared__ double crd[3][PN];
@@ -2121,7 +2156,7 @@ __global__ void k_tail(StepCommon A, int out_parity) {
 // names, so one captured graph stays valid while scenes advance, stop or
 // regrow independently.
 // ---------------------------------------------------------------------------
-enum BatchKind { kBK_BBOX = 0, kBK_SORT, kBK_SCAN, kBK_TILES, kBK_CLEAR, kBK_TILEK, kBK_NODES, kBK_ONE, kBK_KINDS };
+enum BatchKind { kBK_BBOX = 0, kBK_SORT, kBK_SCAN, kBK_TILEK, kBK_NODES, kBK_ONE, kBK_KINDS };
 
 template <typename R>
 struct BatchView {
@@ -2180,59 +2215,32 @@ __global__ void __launch_bounds__(256) kb_header(BatchView<R> B) {
   if (A) header_body<D>(*A);
 }
 
-// zeroes the tile ranges and (MUSL) the re-projection accumulator of an
-// active scene (the single-scene step does this with memsets)
 template <int D, typename R>
-__global__ void __launch_bounds__(256) kb_clear(BatchView<R> B) {
-  uint32_t b, nb;
-  const StepArgsT<R>* A = batch_locate(B, kBK_CLEAR, b, nb);
-  if (!A || step_inactive(A->H)) return;
-  const uint32_t stride = nb * blockDim.x;
-  for (uint32_t i = b * blockDim.x + threadIdx.x; i < A->cap_tiles; i += stride) {
-    A->tile_begin[i] = 0u;
-    A->tile_end[i] = 0u;
-  }
-  if (A->P->use_musl) {
-    const size_t n = (size_t)D * A->cap_nodes;
-    for (size_t i = b * blockDim.x + threadIdx.x; i < n; i += stride) A->v2[i] = 0.0;
-  }
-}
-
-template <int D, typename R>
-__global__ void __launch_bounds__(kSortThreads) kb_sort_hist(BatchView<R> B, int pass) {
+__global__ void __launch_bounds__(kSortThreads) kb_sort_keys(BatchView<R> B) {
   uint32_t b, nb;
   const StepArgsT<R>* A = batch_locate(B, kBK_SORT, b, nb);
-  if (!A) return;
-  if (pass == 0)
-    sort_hist_body<D, true>(*A, nullptr, 0, b, nb);
-  else
-    sort_hist_body<D, false>(*A, (pass & 1) ? A->keysB : A->keysA, 8 * pass, b, nb);
+  if (A) sort_keys_body<D>(*A, b);
 }
 
 template <typename R>
-__global__ void __launch_bounds__(256) kb_sort_scan(BatchView<R> B) {
+__global__ void __launch_bounds__(kSortThreads) kb_sort_scan(BatchView<R> B) {
   uint32_t b, nb;
   const StepArgsT<R>* A = batch_locate(B, kBK_SCAN, b, nb);
-  if (A) sort_scan_warp_body(*A, b);
+  if (A) sort_scan_body(*A, b);
 }
 
 template <typename R>
-__global__ void __launch_bounds__(kSortThreads) kb_sort_scatter(BatchView<R> B, int pass) {
+__global__ void __launch_bounds__(kSortThreads) kb_sort_place(BatchView<R> B) {
   uint32_t b, nb;
   const StepArgsT<R>* A = batch_locate(B, kBK_SORT, b, nb);
-  if (!A) return;
-  const uint32_t* ksrc = pass == 0 ? A->keys0 : ((pass & 1) ? A->keysB : A->keysA);
-  const uint32_t* vsrc = pass == 0 ? nullptr : ((pass & 1) ? A->valsB : A->valsA);
-  uint32_t* kdst = (pass & 1) ? A->keysA : A->keysB;
-  uint32_t* vdst = (pass & 1) ? A->valsA : A->valsB;
-  sort_scatter_body(*A, ksrc, vsrc, kdst, vdst, 8 * pass, b, nb);
+  if (A) sort_place_body(*A, b);
 }
 
 template <typename R>
-__global__ void __launch_bounds__(256) kb_tile_ranges(BatchView<R> B) {
+__global__ void __launch_bounds__(kSortThreads) kb_sort_rank(BatchView<R> B) {
   uint32_t b, nb;
-  const StepArgsT<R>* A = batch_locate(B, kBK_TILES, b, nb);
-  if (A) tile_ranges_body(*A, A->skeys, b, nb);
+  const StepArgsT<R>* A = batch_locate(B, kBK_SORT, b, nb);
+  if (A) sort_rank_body(*A, b, nb);
 }
 
 template <int D, int DEG, typename R, int XS = 1>

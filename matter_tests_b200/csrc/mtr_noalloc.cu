@@ -14,7 +14,7 @@
 //
 // Limits: at most MTR_NOALLOC_MAX_PARTICLES particles and
 // MTR_NOALLOC_MAX_NODES grid nodes per call; larger requests are rejected
-// with MTR_ERR_TOO_LARGE before anything is launched.  The array costs ~10 MB of device memory on every GPU
+// with MTR_ERR_TOO_LARGE before anything is launched.  The array costs ~12 MB of device memory on every GPU
 // that loads the library, until the process exits.
 //
 // Sharing: every call on a device uses the same array.  Each call clears
@@ -43,8 +43,12 @@ namespace {
 constexpr int kMaxDevices = 64;
 constexpr size_t kMaxP = MTR_NOALLOC_MAX_PARTICLES;
 constexpr size_t kMaxNodes = MTR_NOALLOC_MAX_NODES;
-constexpr size_t kMaxTiles = MTR_NOALLOC_MAX_NODES;  // a tile holds at least one node
-constexpr size_t kSortBlocks = (kMaxP + kSortTile - 1) / kSortTile;
+// Most tiles of a grid of kMaxNodes nodes with at least 4 per axis: an axis of n
+// nodes has ceil(n / 4) tiles in 3D, at most 2/5 n (n = 5), so at most 0.064
+// tiles per node; in 2D ceil(n / 8), at most n / 4 (n = 4), so at most 0.0625.
+constexpr size_t kMaxTiles = kMaxNodes * 64 / 1000 + 1;
+constexpr size_t kMaxSupers = (kMaxTiles * 64 + 1 + kSuperCells - 1) / kSuperCells;
+constexpr size_t kMaxCells = kMaxSupers * kSuperCells;
 
 constexpr size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 
@@ -52,15 +56,13 @@ constexpr size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 constexpr size_t kOffHeader = 0;
 constexpr size_t kOffParams = kOffHeader + align256(sizeof(StepHeader));
 constexpr size_t kOffKeys0 = kOffParams + align256(sizeof(DevParams));
-constexpr size_t kOffKeysA = kOffKeys0 + align256(kMaxP * 4);
-constexpr size_t kOffValsA = kOffKeysA + align256(kMaxP * 4);
-constexpr size_t kOffKeysB = kOffValsA + align256(kMaxP * 4);
-constexpr size_t kOffValsB = kOffKeysB + align256(kMaxP * 4);
-constexpr size_t kOffHist = kOffValsB + align256(kMaxP * 4);
-constexpr size_t kOffDtot = kOffHist + align256(256 * kSortBlocks * 4);
-constexpr size_t kOffTileB = kOffDtot + align256(256 * 4);
-constexpr size_t kOffTileE = kOffTileB + align256(kMaxTiles * 4);
-constexpr size_t kOffAcc = kOffTileE + align256(kMaxTiles * 4);
+constexpr size_t kOffRank = kOffKeys0 + align256(kMaxP * 4);
+constexpr size_t kOffTmp = kOffRank + align256(kMaxP * 4);
+constexpr size_t kOffBig = kOffTmp + align256(kMaxP * 4);
+constexpr size_t kOffStart = kOffBig + align256((kMaxP / kBigCell + 1) * 4);
+constexpr size_t kOffCount = kOffStart + align256((kMaxCells + 4) * 4);
+constexpr size_t kOffSuper = kOffCount + align256(kMaxCells * 4);
+constexpr size_t kOffAcc = kOffSuper + align256(kMaxSupers * 4);
 constexpr size_t kScratchBytes = kOffAcc + align256(4 * kMaxNodes * sizeof(double));  // mass + momentum[3]
 
 }  // namespace
@@ -85,7 +87,8 @@ __global__ void __launch_bounds__(kChunk) k_p2g_noalloc(StepArgs A, const uint32
   const StepHeader* H = A.H;
   const uint32_t t = blockIdx.x;
   if (t >= H->ntiles) return;
-  const uint32_t pb = A.tile_begin[t], pe = A.tile_end[t];
+  uint32_t pb, pe;
+  tile_range(A, t, pb, pe);
   if (pb >= pe) return;
   const DevParams& P = *A.P;
   extern __shared__ double smem[];
@@ -223,18 +226,20 @@ __global__ void __launch_bounds__(kChunk) k_p2g_noalloc(StepArgs A, const uint32
   }
 }
 
-// Cell keys of the first sort pass.  A particle whose cell lies outside the
-// caller's grid (or whose position is not finite) gets the sentinel key
-// ntiles * 64, one past every real tile: it sorts behind all real particles,
-// no tile range names it, and it is reported through the status word.  The
-// test is written on the same expression cell_key floors, so a particle kept
-// here has a tile index below ntiles.
+// Cell keys.  A particle whose cell lies outside the caller's grid (or whose
+// position is not finite) gets the sentinel key ntiles * 64, one past every
+// real tile: it sorts behind all real particles, no tile names it, and it is
+// reported through the status word.  The test is written on the same
+// expression cell_key floors, so a particle kept here has a tile index below
+// ntiles.
 template <int D>
-__global__ void __launch_bounds__(256) k_noalloc_keys(StepCommon A) {
+__global__ void __launch_bounds__(kSortThreads) k_noalloc_keys(StepCommon A) {
   const StepHeader* H = A.H;
   const double ioh = A.P->one_over_dx;
-  const uint32_t sentinel = H->ntiles * 64u;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < A.Np; i += gridDim.x * blockDim.x) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = i < A.Np;
+  uint32_t key = H->ntiles * 64u;
+  if (valid) {
     double x[3] = {0.0, 0.0, 0.0};
     bool inside = true;
 #pragma unroll
@@ -244,13 +249,14 @@ __global__ void __launch_bounds__(256) k_noalloc_keys(StepCommon A) {
       if (!(u >= 0.0 && u < (double)H->N[a])) inside = false;
     }
     if (inside) {
-      A.keys0[i] = cell_key<D>(H, ioh, x);
+      key = cell_key<D>(H, ioh, x);
     } else {
-      A.keys0[i] = sentinel;
       atomicOr(&A.H->status, MTR_STATUS_STENCIL_OOB);
       atomicMin(&A.H->first_bad, i);
     }
+    A.keys0[i] = key;
   }
+  sort_count(A, i, valid, key);
 }
 
 template <int D>
@@ -259,12 +265,18 @@ constexpr size_t noalloc_smem_bytes() {
 }
 
 // Writes the grid description and the few constants the kernels read into
-// the scratch header and parameter block (passed by value: no host copy).
+// the scratch header and parameter block (passed by value: no host copy), and
+// clears the accumulators and the sort's counts.
 __global__ void k_noalloc_setup(StepHeader* H, DevParams* P, const double* gx, const double* gy, const double* gz,
                                 uint32_t nx, uint32_t ny, uint32_t nz, uint32_t tx, uint32_t ty, uint32_t tz,
                                 double one_over_dx, double apicD, double flip_ratio, double particle_mass, uint32_t Np,
-                                int dim) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+                                int dim, double* acc, uint32_t nacc, uint32_t* count, uint32_t ncount,
+                                uint32_t* super, uint32_t nsuper) {
+  const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  for (uint32_t i = i0; i < nacc; i += step) acc[i] = 0.0;
+  for (uint32_t i = i0; i < ncount; i += step) count[i] = 0u;
+  for (uint32_t i = i0; i < nsuper; i += step) super[i] = 0u;
+  if (i0 != 0) return;
   H->done = 0;
   H->abort = 0;
   H->frame = 0;
@@ -284,6 +296,7 @@ __global__ void k_noalloc_setup(StepHeader* H, DevParams* P, const double* gx, c
   H->T[1] = ty;
   H->T[2] = tz;
   H->ntiles = tx * ty * tz;
+  H->nbig = 0;
   P->one_over_dx = one_over_dx;
   P->apicDinverse = apicD;
   P->flip_ratio = flip_ratio;
@@ -357,53 +370,36 @@ int run_noalloc(unsigned char* base, const mtr_params& p, const double* x, const
   A.gx = const_cast<double*>(gx);
   A.gy = const_cast<double*>(gy);
   A.gz = const_cast<double*>(gz ? gz : gy);
-  A.cap_nodes = (uint32_t)kMaxNodes;
-  A.cap_tiles = (uint32_t)ntiles;  // k_tile_ranges skips the sentinel tile (index ntiles)
+  A.cap_nodes = (uint32_t)G;
+  A.cap_tiles = (uint32_t)ntiles;
   A.acc = reinterpret_cast<double*>(base + kOffAcc);
   A.keys0 = reinterpret_cast<uint32_t*>(base + kOffKeys0);
-  A.keysA = reinterpret_cast<uint32_t*>(base + kOffKeysA);
-  A.valsA = reinterpret_cast<uint32_t*>(base + kOffValsA);
-  A.keysB = reinterpret_cast<uint32_t*>(base + kOffKeysB);
-  A.valsB = reinterpret_cast<uint32_t*>(base + kOffValsB);
-  A.hist = reinterpret_cast<uint32_t*>(base + kOffHist);
-  A.dtot = reinterpret_cast<uint32_t*>(base + kOffDtot);
-  A.sort_blocks = (int)((Np + kSortTile - 1) / kSortTile);
-  A.tile_begin = reinterpret_cast<uint32_t*>(base + kOffTileB);
-  A.tile_end = reinterpret_cast<uint32_t*>(base + kOffTileE);
+  A.perm_rank = reinterpret_cast<uint32_t*>(base + kOffRank);
+  A.perm = A.perm_rank;
+  A.perm_tmp = reinterpret_cast<uint32_t*>(base + kOffTmp);
+  A.big_cells = reinterpret_cast<uint32_t*>(base + kOffBig);
+  A.cell_start = reinterpret_cast<uint32_t*>(base + kOffStart);
+  A.cell_count = reinterpret_cast<uint32_t*>(base + kOffCount);
+  A.super = reinterpret_cast<uint32_t*>(base + kOffSuper);
   A.in.x = const_cast<double*>(x);
   A.xin = x;
   A.in.v = const_cast<double*>(v);
   A.in.B = const_cast<double*>(B);
-  // what must start at zero: the accumulators and the tile ranges of this grid
-  // (memsets first, so that a failure leaves nothing of this call queued)
-  if (cudaMemsetAsync(A.acc, 0, sizeof(double) * 4 * kMaxNodes, st) != cudaSuccess) return MTR_ERR_CUDA;
-  if (cudaMemsetAsync(A.tile_begin, 0, sizeof(uint32_t) * ntiles, st) != cudaSuccess) return MTR_ERR_CUDA;
-  if (cudaMemsetAsync(A.tile_end, 0, sizeof(uint32_t) * ntiles, st) != cudaSuccess) return MTR_ERR_CUDA;
-  k_noalloc_setup<<<1, 32, 0, st>>>(H, P, gx, gy, gz, nx, ny, nz, tx, ty, tz, 1.0 / p.dx, apicD, p.flip_ratio,
-                                    p.particle_mass, Np, D);
-  k_noalloc_keys<D><<<(uint32_t)std::min<uint64_t>((Np + 255) / 256, 148 * 8), 256, 0, st>>>(A);
-  // enough digits for every real key (below ntiles * 64) and the sentinel (ntiles * 64)
-  uint64_t keybits = 1;
-  while ((1ull << keybits) < ntiles * 64ull + 1ull) ++keybits;
-  const int passes = (int)((keybits + 7) / 8);
-  const uint32_t* skeys = nullptr;
-  const uint32_t* perm = nullptr;
-  for (int pass = 0; pass < passes; ++pass) {
-    const int shift = 8 * pass;
-    const uint32_t* ksrc = pass == 0 ? A.keys0 : ((pass & 1) ? A.keysB : A.keysA);
-    const uint32_t* vsrc = pass == 0 ? nullptr : ((pass & 1) ? A.valsB : A.valsA);
-    uint32_t* kdst = (pass & 1) ? A.keysA : A.keysB;
-    uint32_t* vdst = (pass & 1) ? A.valsA : A.valsB;
-    k_sort_hist<D, false><<<A.sort_blocks, kSortThreads, 0, st>>>(A, ksrc, shift);
-    k_sort_scan<<<256, 256, 0, st>>>(A);
-    k_sort_scatter<<<A.sort_blocks, kSortThreads, 0, st>>>(A, ksrc, vsrc, kdst, vdst, shift);
-    skeys = kdst;
-    perm = vdst;
-  }
-  k_tile_ranges<<<(Np + 255) / 256, 256, 0, st>>>(A, skeys);
-  k_p2g_noalloc<D, DEG><<<(uint32_t)ntiles, kChunk, noalloc_smem_bytes<D>(), st>>>(A, perm);
+  if (ntiles > kMaxTiles) return MTR_ERR_TOO_LARGE;  // cannot happen (see kMaxTiles)
+  const uint32_t supers = (uint32_t)((ntiles * 64 + 1 + kSuperCells - 1) / kSuperCells);
+  const uint32_t pblocks = (Np + kSortThreads - 1) / kSortThreads;
+  // sets the header up and clears what must start at zero: this grid's cell
+  // counts and accumulators
+  k_noalloc_setup<<<(uint32_t)std::min<uint64_t>((G * (1 + D) + 255) / 256, 148 * 4), 256, 0, st>>>(
+      H, P, gx, gy, gz, nx, ny, nz, tx, ty, tz, 1.0 / p.dx, apicD, p.flip_ratio, p.particle_mass, Np, D, A.acc,
+      (uint32_t)(G * (1 + D)), A.cell_count, supers * kSuperCells, A.super, supers);
+  k_noalloc_keys<D><<<pblocks, kSortThreads, 0, st>>>(A);
+  k_sort_scan<<<supers, kSortThreads, 0, st>>>(A);
+  k_sort_place<<<pblocks, kSortThreads, 0, st>>>(A);
+  k_sort_rank<<<pblocks, kSortThreads, 0, st>>>(A);
+  k_p2g_noalloc<D, DEG><<<(uint32_t)ntiles, kChunk, noalloc_smem_bytes<D>(), st>>>(A, A.perm);
   k_noalloc_finalize<D><<<(uint32_t)std::min<uint64_t>((G + 255) / 256, 148 * 8), 256, 0, st>>>(
-      A.acc, (uint32_t)kMaxNodes, (uint32_t)G, p.particle_mass, grid_mass, grid_v, H, status);
+      A.acc, (uint32_t)G, (uint32_t)G, p.particle_mass, grid_mass, grid_v, H, status);
   return cudaGetLastError() == cudaSuccess ? MTR_OK : MTR_ERR_CUDA;
 }
 
