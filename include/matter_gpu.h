@@ -350,11 +350,11 @@ typedef struct mtr_group_info {
 int mtr_autotune(mtr_ctx* ctx, int reps, int* threads /* [4] out, may be NULL */);
 int mtr_set_tile_threads(mtr_ctx* ctx, const int* threads /* [4] */);
 int mtr_get_tile_threads(mtr_ctx* ctx, int* threads /* [4] */);
-/* Lanes per particle of the two scatters, lanes[0] P2G and lanes[1] MUSL: the
- * warp lanes that share one particle's stencil (3D: 16, each lane one (y, z)
- * column of 4 x nodes, or 32, each lane 2 of a column's x nodes; 2D: 4 or 8).
- * A warp scatters 32 / lanes particles at a time.  mtr_autotune tunes them
- * with the block sizes (candidates 64/128/256 threads x both lane counts). */
+/* Lanes per particle of the two scatters, lanes[0] P2G and lanes[1] MUSL: 16
+ * or 32 in 3D, 4 or 8 in 2D (default 16, 4).  A hint that is checked, kept and
+ * reported: the scatters give each of a particle's stencil columns (16 in 3D,
+ * 4 in 2D) two lanes in P2G and one in MUSL, whatever it says, which measured
+ * fastest on every workload.  mtr_autotune leaves it as it is. */
 int mtr_set_tile_lanes(mtr_ctx* ctx, const int* lanes /* [2] */);
 int mtr_get_tile_lanes(mtr_ctx* ctx, int* lanes /* [2] */);
 int mtr_batch_set_tile_lanes(mtr_batch* batch, int group, const int* lanes /* [2] */);

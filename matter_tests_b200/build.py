@@ -21,7 +21,7 @@ NVCC_FLAGS = [
     "-O3", "-lineinfo", "-std=c++17",
     "-Xcompiler", "-fPIC", "-shared",
     "--expt-relaxed-constexpr",
-    "--threads", "0", "--split-compile", "0",  # the sources and the kernels within each on all host cores
+    "--threads", "0",  # the sources in parallel (--split-compile changes the code of the tile kernels, by up to 8% in time)
 ]
 
 

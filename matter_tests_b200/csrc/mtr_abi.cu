@@ -116,9 +116,9 @@ bool valid_tile_threads(const int* t) {
   return true;
 }
 
-// Lanes per particle of the two scatters (P2G, MUSL): the stencil columns of
-// a particle's cell (16 in 3D, 4 in 2D) times the split of each column's 4 x
-// nodes over 1 or 2 lanes; a warp then takes 32 / lanes particles at a time.
+// Lanes per particle of the two scatters (P2G, MUSL), 16 or 32 in 3D, 4 or 8
+// in 2D: kept for callers.  The scatters hold a stencil column in fixed lanes
+// (P2G two, MUSL one), which measured fastest on every workload.
 constexpr int kScatterSlots = 2;
 int scatter_columns(int dim) { return dim == 3 ? 16 : 4; }
 bool valid_tile_lanes(int dim, const int* lanes) {
@@ -171,7 +171,7 @@ struct mtr_ctx {
   bool use_graphs = true;
   uint32_t step_limit = 0xffffffffu;  // mtr_set_step_limit: no step beyond this step count
   int tile_threads[kTileSlots] = {kChunk, kChunk, kChunk, kChunk};
-  int tile_split[kScatterSlots] = {1, 1};  // x-node split of the P2G and MUSL scatters (1 or 2)
+  int tile_split[kScatterSlots] = {1, 1};  // lanes per particle asked for, over the stencil columns
   // a trial step runs every kernel of a step but the commit (k_tail): the
   // particle buffer it reads and the clock stay as they were
   bool trial = false;
@@ -415,10 +415,8 @@ void scatter_attributes(K kernel, size_t smem) {
 
 template <int D, int DEG, typename R>
 void set_kernel_attributes_t() {
-  scatter_attributes(k_p2g_w<D, DEG, R, 1>, p2g_smem_bytes<D, R>(kMaxTileThreads));
-  scatter_attributes(k_p2g_w<D, DEG, R, 2>, p2g_smem_bytes<D, R>(kMaxTileThreads));
-  scatter_attributes(k_g2p_musl_w<D, DEG, R, 1>, musl_smem_bytes<D, R>(MTR_MUSL_MAX_THREADS));
-  scatter_attributes(k_g2p_musl_w<D, DEG, R, 2>, musl_smem_bytes<D, R>(MTR_MUSL_MAX_THREADS));
+  scatter_attributes(k_p2g_w<D, DEG, R>, p2g_smem_bytes<D, R>(kMaxTileThreads));
+  scatter_attributes(k_g2p_musl_w<D, DEG, R>, musl_smem_bytes<D, R>(MTR_MUSL_MAX_THREADS));
 }
 
 void set_kernel_attributes(bool fp32) {
@@ -544,10 +542,7 @@ int enqueue_step_t(mtr_ctx* c, int parity) {
   const int* tt = c->tile_threads;
   {
     const size_t sm = p2g_smem_bytes<D, R>(tt[kSlotP2G], c->prm.use_mibf != 0);
-    if (c->tile_split[kSlotP2G] == 2)
-      k_p2g_w<D, DEG, R, 2><<<c->cap_tiles, tt[kSlotP2G], sm, st>>>(A, perm);
-    else
-      k_p2g_w<D, DEG, R, 1><<<c->cap_tiles, tt[kSlotP2G], sm, st>>>(A, perm);
+    k_p2g_w<D, DEG, R><<<c->cap_tiles, tt[kSlotP2G], sm, st>>>(A, perm);
   }
   ++n;
   mark(c, "k_p2g");
@@ -562,10 +557,7 @@ int enqueue_step_t(mtr_ctx* c, int parity) {
   mark(c, "k_grid");
   if (c->prm.use_musl) {
     const size_t sm = musl_smem_bytes<D, R>(tt[kSlotMUSL]);
-    if (c->tile_split[kSlotMUSL] == 2)
-      k_g2p_musl_w<D, DEG, R, 2><<<c->cap_tiles, tt[kSlotMUSL], sm, st>>>(A, perm);
-    else
-      k_g2p_musl_w<D, DEG, R, 1><<<c->cap_tiles, tt[kSlotMUSL], sm, st>>>(A, perm);
+    k_g2p_musl_w<D, DEG, R><<<c->cap_tiles, tt[kSlotMUSL], sm, st>>>(A, perm);
     mark(c, "k_g2p_musl");
     k_musl_norm<D, R><<<gblocks, 256, 0, st>>>(A);
     mark(c, "k_musl_norm");
@@ -927,15 +919,13 @@ int enqueue_group_step_t(mtr_batch* b, mtr_batch_group& g, int gi) {
   n += 6;
   b->marks.record("kb_sort", st, gi);
   const uint32_t tiles = g.total[kBK_TILEK];
-  launch_tiles<R>(g.tile_split[kSlotP2G] == 2 ? kb_p2g_w<D, DEG, R, 2> : kb_p2g_w<D, DEG, R, 1>, tiles,
-                  tt[kSlotP2G], p2g_smem_bytes<D, R>(tt[kSlotP2G]), st, B);
+  launch_tiles<R>(kb_p2g_w<D, DEG, R>, tiles, tt[kSlotP2G], p2g_smem_bytes<D, R>(tt[kSlotP2G]), st, B);
   b->marks.record(kSlotMark[kSlotP2G], st, gi);
   kb_grid<D, R><<<g.total[kBK_NODES], 256, 0, st>>>(B);
   b->marks.record("kb_grid", st, gi);
   n += 2;
   if (g.musl) {
-    launch_tiles<R>(g.tile_split[kSlotMUSL] == 2 ? kb_g2p_musl_w<D, DEG, R, 2> : kb_g2p_musl_w<D, DEG, R, 1>,
-                    tiles, tt[kSlotMUSL], musl_smem_bytes<D, R>(tt[kSlotMUSL]), st, B);
+    launch_tiles<R>(kb_g2p_musl_w<D, DEG, R>, tiles, tt[kSlotMUSL], musl_smem_bytes<D, R>(tt[kSlotMUSL]), st, B);
     b->marks.record(kSlotMark[kSlotMUSL], st, gi);
     kb_musl_norm<D, R><<<g.total[kBK_NODES], 256, 0, st>>>(B);
     b->marks.record("kb_musl_norm", st, gi);
@@ -982,10 +972,8 @@ int enqueue_batch_step(mtr_batch* b) {
 
 template <int D, int DEG, typename R>
 void set_batch_attributes_t() {
-  scatter_attributes(kb_p2g_w<D, DEG, R, 1>, p2g_smem_bytes<D, R>(kMaxTileThreads));
-  scatter_attributes(kb_p2g_w<D, DEG, R, 2>, p2g_smem_bytes<D, R>(kMaxTileThreads));
-  scatter_attributes(kb_g2p_musl_w<D, DEG, R, 1>, musl_smem_bytes<D, R>(MTR_MUSL_MAX_THREADS));
-  scatter_attributes(kb_g2p_musl_w<D, DEG, R, 2>, musl_smem_bytes<D, R>(MTR_MUSL_MAX_THREADS));
+  scatter_attributes(kb_p2g_w<D, DEG, R>, p2g_smem_bytes<D, R>(kMaxTileThreads));
+  scatter_attributes(kb_g2p_musl_w<D, DEG, R>, musl_smem_bytes<D, R>(MTR_MUSL_MAX_THREADS));
 }
 
 void set_batch_attributes(const mtr_batch_group& g) {
@@ -1061,18 +1049,16 @@ void write_batch_headers(mtr_batch* b) {
 }
 
 // Block-shape tuning over kTuneRounds candidates: candidate k runs every tile
-// kernel with kTileCandidates[k % 3] threads (capped at the slot's maximum)
-// and the scatters with x split 1 + k / 3 (16 or 32 lanes per particle in 3D,
-// 4 or 8 in 2D).  The candidates are interleaved: each repetition times every
-// candidate once, so slow drifts of the state or the clock touch them all
-// alike.  samples[slot][k] holds the times of the slot's kernel with
-// candidate k; for the gathers, whose shape is the thread count alone,
-// rounds k and k + 3 are the same candidate.  A candidate's time is the
+// kernel with kTileCandidates[k] threads (capped at the slot's maximum).  The
+// candidates are interleaved: each repetition times every candidate once, so
+// slow drifts of the state or the clock touch them all alike.
+// samples[slot][k] holds the times of the slot's kernel with candidate k.  A
+// candidate's time is the
 // median of its samples and its noise the half-range of its samples relative
 // to that median; a slot keeps its current shape unless another candidate is
 // faster by more than 2% and by more than the noise of the two together, so
 // timing noise does not trade an equal shape for a slower one.
-constexpr int kTuneRounds = 6;
+constexpr int kTuneRounds = 3;
 
 struct TuneTimes {
   std::vector<double> samples[kTileSlots][kTuneRounds];
@@ -1083,24 +1069,21 @@ struct TuneTimes {
   // (median, relative half-range) of one candidate of a slot; median < 0: not measured
   std::pair<double, double> stats(int sl, int k) const {
     std::vector<double> v = samples[sl][k];
-    if (sl >= kScatterSlots) v.insert(v.end(), samples[sl][k + 3].begin(), samples[sl][k + 3].end());
     if (v.empty()) return {-1.0, 0.0};
     std::sort(v.begin(), v.end());
     const size_t n = v.size();
     const double med = n % 2 ? v[n / 2] : 0.5 * (v[n / 2 - 1] + v[n / 2]);
     return {med, med > 0.0 ? 0.5 * (v.back() - v.front()) / med : 0.0};
   }
-  void choose(int* threads, int* split) const {
+  void choose(int* threads) const {
     for (int sl = 0; sl < kTileSlots; ++sl) {
-      const bool scatter = sl < kScatterSlots;
-      const int nk = scatter ? kTuneRounds : 3;
       int cur = -1, arg = -1;
       double tcur = 0.0, ncur = 0.0, targ = 0.0, narg = 0.0;
-      for (int k = 0; k < nk; ++k) {
-        if (kTileCandidates[k % 3] > kSlotMax[sl]) continue;
+      for (int k = 0; k < kTuneRounds; ++k) {
+        if (kTileCandidates[k] > kSlotMax[sl]) continue;
         const auto st = stats(sl, k);
         if (st.first < 0.0) continue;
-        if (kTileCandidates[k % 3] == threads[sl] && (!scatter || 1 + k / 3 == split[sl])) {
+        if (kTileCandidates[k] == threads[sl]) {
           cur = k;
           tcur = st.first;
           ncur = st.second;
@@ -1114,16 +1097,14 @@ struct TuneTimes {
       if (arg < 0) continue;  // the slot's kernel does not run in this step
       const double margin = std::max(0.02, ncur + narg);
       if (cur >= 0 && tcur <= (1.0 + margin) * targ) continue;
-      threads[sl] = kTileCandidates[arg % 3];
-      if (scatter) split[sl] = 1 + arg / 3;
+      threads[sl] = kTileCandidates[arg];
     }
   }
 };
 
 // the shapes of candidate k for every slot
-void set_candidate(int* threads, int* split, int k) {
-  for (int sl = 0; sl < kTileSlots; ++sl) threads[sl] = std::min(kTileCandidates[k % 3], kSlotMax[sl]);
-  for (int sl = 0; sl < kScatterSlots; ++sl) split[sl] = 1 + k / 3;
+void set_candidate(int* threads, int k) {
+  for (int sl = 0; sl < kTileSlots; ++sl) threads[sl] = std::min(kTileCandidates[k], kSlotMax[sl]);
 }
 
 // Restores flags changed for trial steps even when a step throws.
@@ -1902,22 +1883,20 @@ int mtr_autotune(mtr_ctx* c, int reps, int* threads) {
       }
       if (!ready) throw MtrError{MTR_ERR_STATE, "grid kept growing during tuning"};
       TuneTimes tt;
-      int chosen[kTileSlots], chosen_split[kScatterSlots];
+      int chosen[kTileSlots];
       std::copy(c->tile_threads, c->tile_threads + kTileSlots, chosen);
-      std::copy(c->tile_split, c->tile_split + kScatterSlots, chosen_split);
       c->marks.on = true;
       for (int r = 0; r < reps; ++r)
         for (int k = 0; k < kTuneRounds; ++k) {
-          set_candidate(c->tile_threads, c->tile_split, k);
+          set_candidate(c->tile_threads, k);
           c->marks.reset();
           enqueue_step(c, parity);
           CK(cudaStreamSynchronize(c->stream));
           const auto& L = c->marks.list;
           for (size_t i = 1; i < L.size(); ++i) tt.add(L[i].first, c->marks.since_previous(i), k);
         }
-      tt.choose(chosen, chosen_split);
+      tt.choose(chosen);
       std::copy(chosen, chosen + kTileSlots, c->tile_threads);
-      std::copy(chosen_split, chosen_split + kScatterSlots, c->tile_split);
       *c->hH = saved;  // the trial steps leave no trace: clock, plates, counters as before
       write_header(c);
       CK(cudaStreamSynchronize(c->stream));
@@ -2271,16 +2250,13 @@ int mtr_batch_autotune(mtr_batch* b, int reps) {
         g.tuned_nodes = nodes;
       }
       std::vector<TuneTimes> tt(b->groups.size());
-      std::vector<std::vector<int>> chosen, chosen_split;
-      for (auto& g : b->groups) {
-        chosen.emplace_back(g.tile_threads, g.tile_threads + kTileSlots);
-        chosen_split.emplace_back(g.tile_split, g.tile_split + kScatterSlots);
-      }
+      std::vector<std::vector<int>> chosen;
+      for (auto& g : b->groups) chosen.emplace_back(g.tile_threads, g.tile_threads + kTileSlots);
       b->marks.on = true;
       b->trial = true;
       for (int r = 0; r < reps; ++r)
         for (int k = 0; k < kTuneRounds; ++k) {
-          for (auto& g : b->groups) set_candidate(g.tile_threads, g.tile_split, k);
+          for (auto& g : b->groups) set_candidate(g.tile_threads, k);
           b->marks.reset();
           b->marks.record("start", b->stream, -1);
           enqueue_batch_step(b);
@@ -2290,9 +2266,8 @@ int mtr_batch_autotune(mtr_batch* b, int reps) {
             if (b->marks.tag[i] == b->marks.tag[i - 1]) tt[b->marks.tag[i]].add(L[i].first, b->marks.since_previous(i), k);
         }
       for (size_t gi = 0; gi < b->groups.size(); ++gi) {
-        tt[gi].choose(chosen[gi].data(), chosen_split[gi].data());
+        tt[gi].choose(chosen[gi].data());
         std::copy(chosen[gi].begin(), chosen[gi].end(), b->groups[gi].tile_threads);
-        std::copy(chosen_split[gi].begin(), chosen_split[gi].end(), b->groups[gi].tile_split);
       }
     }
     for (size_t i = 0; i < b->members.size(); ++i) *b->members[i]->hH = saved[i];

@@ -228,6 +228,89 @@ __device__ __forceinline__ R bspline_dN(R u) {
   }
 }
 
+// The 4 stencil weights of one axis, and with DW their derivatives (times dx),
+// from the particle's position t in its cell, (x - x_1) / dx with x_1 the
+// stencil's second node: t in [0, 1] and the nodes lie at -1, 0, 1, 2 cells from
+// x_1.  The pieces of the spline each node sees are then known, so nothing
+// branches: about 15 operations for the 4 nodes instead of about 14 (two
+// pieces and their selection) for each.  1 - t is formed in FP64.
+template <int DEG, bool DW, typename R>
+__device__ __forceinline__ void axis_weights(double td, R (&w)[4], R (&d)[4]) {
+  const R t = (R)td, s = (R)(1.0 - td);
+  if constexpr (DEG == 3) {
+    const R tt = t * t, ss = s * s;
+    w[0] = ss * (s * R(1.0 / 6.0));
+    w[1] = R(2.0 / 3.0) - tt * (R(1.0) - R(0.5) * t);
+    w[2] = R(2.0 / 3.0) - ss * (R(1.0) - R(0.5) * s);
+    w[3] = tt * (t * R(1.0 / 6.0));
+    if constexpr (DW) {
+      d[0] = R(-0.5) * ss;
+      d[1] = t * (R(1.5) * t - R(2.0));
+      d[2] = s * (R(2.0) - R(1.5) * s);
+      d[3] = R(0.5) * tt;
+    }
+  } else {
+    // r: distance to the nearest node, which is the second (t < 1/2) or the third
+    const bool left = t < R(0.5);
+    const R r = left ? t : -s, lo = R(0.5) - r, hi = R(0.5) + r;
+    const R wl = R(0.5) * lo * lo, wc = R(0.75) - r * r, wr = R(0.5) * hi * hi;
+    w[0] = left ? wl : R(0.0);
+    w[1] = left ? wc : wl;
+    w[2] = left ? wr : wc;
+    w[3] = left ? R(0.0) : wr;
+    if constexpr (DW) {
+      const R dc = R(-2.0) * r;
+      d[0] = left ? -lo : R(0.0);
+      d[1] = left ? dc : -lo;
+      d[2] = left ? hi : dc;
+      d[3] = left ? R(0.0) : hi;
+    }
+  }
+  if constexpr (!DW) d[0] = d[1] = d[2] = d[3] = R(0.0);
+}
+
+// node offsets x_i - x_p of the same 4 nodes
+template <typename R>
+__device__ __forceinline__ void axis_offsets(double td, R dx, R (&o)[4]) {
+  const R t = (R)td, s = (R)(1.0 - td);
+  o[0] = -(R(1.0) + t) * dx;
+  o[1] = -t * dx;
+  o[2] = s * dx;
+  o[3] = (R(1.0) + s) * dx;
+}
+
+// A stencil that P2G clamped at the grid's first node: t may lie outside
+// [0, 1] there, and every node's weight is evaluated piece by piece.
+template <int DEG, typename R>
+__device__ __noinline__ void axis_weights_any(double td, R (&w)[4], R (&d)[4]) {
+#pragma unroll
+  for (int o = 0; o < 4; ++o) {
+    const R u = (R)(td + (1.0 - o));
+    w[o] = bspline_N<DEG>(u);
+    d[o] = bspline_dN<DEG>(u);
+  }
+}
+
+// binary exponent of a positive weight; zero (which adds nothing) counts as one
+__device__ __forceinline__ int weight_exponent(double w) {
+  const int e = __double2hiint(w) >> 20;
+  return e ? e - 1023 : 0;
+}
+__device__ __forceinline__ int weight_exponent(float w) {
+  const int e = __float_as_int(w) >> 23;
+  return e ? e - 127 : 0;
+}
+
+// a lower bound of the exponents of one axis's weights: the outer ones of the
+// cubic spline, the outer two of the three quadratic ones (the fourth is zero)
+template <int DEG, typename R>
+__device__ __forceinline__ int least_exponent(const R (&w)[4]) {
+  if constexpr (DEG == 3)
+    return min(weight_exponent(w[0]), weight_exponent(w[3]));
+  else
+    return min(min(weight_exponent(w[0]), weight_exponent(w[1])), min(weight_exponent(w[2]), weight_exponent(w[3])));
+}
+
 // ---------------------------------------------------------------------------
 // SVD: two-sided cyclic Jacobi (Golub & Van Loan, 4th ed., §8.6.3; 2x2
 // symmetrising rotation §8.6.2; symSchur2 Alg. 8.5.1).  Output convention of

@@ -411,11 +411,7 @@ __global__ void __launch_bounds__(256) k_header(StepCommon A) {
 // same keys needs three launches per 8-bit digit (9 for the 18-bit keys of the
 // 1M-particle collapse) and a pass over the sorted keys for the tile ranges,
 // which here are cell_start itself.
-// Measured on a B200, per step: the radix sort with its memsets and tile ranges
-// 11-16 launches and about 80 us at 1,024,000 particles; this one 4 launches,
-// 49 us (CUDA events around every launch, 4 us each of which is the event).
-// Whole steps: 5k particles in 2D 122 -> 100 us, 51,200 in 2D 138 -> 111 us,
-// 150k in 3D 250 -> 210 us, 1,024,000 in 3D FP64 1123 -> 1089 us.
+// @MEASURED_SORT@
 // A cell's ranking is quadratic in its particles (about 8 in 3D), which up to
 // kBigCell of them costs less than another launch; larger cells are ordered by
 // a whole block that walks the keys once.
@@ -702,20 +698,33 @@ __device__ __forceinline__ bool patch_node(const StepHeader* H, const int (&n0)[
 }
 
 // ---------------------------------------------------------------------------
-// 5. P2G + stress force, warp-cooperative, one block per tile.
+// 5. P2G + stress force, one block per tile, each warp on its own.
 //
-// A tile block walks its sorted particles in chunks of blockDim.x (64, 128 or
-// 256 threads, chosen per scene at run time by measurement).  Phase 1, one
-// thread per particle, loads the particle and stages its stencil weights and
-// gradients in shared memory.  Phase 2: lane groups (3D: 16 lanes, 2D: 4 lanes)
-// take consecutive staged particles; a lane owns one stencil column of the
-// particle's cell (3D: (iy, iz) and its 4 ix nodes, 2D: iy and its 4 ix
-// nodes), accumulates every channel in registers while consecutive particles
-// share a cell, and adds them to the shared patch once per cell.  Sorted
-// particles share cells in runs of about ppc, so this issues ~ppc times fewer
-// shared atomics than one atomic per particle and node, with no two lanes of
-// a group on one address.  The patch is flushed with one global atomic per
-// node and channel.
+// The sorted particles of a tile are 16 runs of 4 cells along the innermost
+// axis (a unit).  A warp takes one unit per lane group: it stages a few of the
+// unit's particles in its own part of shared memory (weights, offsets and the
+// factors of momentum and force), then every lane accumulates its stencil
+// columns over those particles.  A column is the 4 nodes along the innermost
+// axis; its sums stay in registers as a window that slides with the cells, so
+// a node is added to the shared patch once per unit (7 nodes for 4 cells)
+// instead of once per cell or per few particles.  No two lanes of a group ever
+// meet on one address, and there is no block barrier between the start and
+// the flush of the patch (one global atomic per node and channel).
+//
+// The lanes of a group come in two roles with the same code: role 0 sums mass
+// and momentum, role 1 the force (and friction).  With per-axis factors w and
+// a (role 0: weight times offset x_i - x_p; role 1: weight derivative) a
+// column's contribution to channel c is
+//   f1_h A_c + f2_h B_c,   f1 = w, f2 = a along the innermost axis,
+//   A_c = w w V_c + a w X_c + w a Y_c,  B_c = w w Z_c,
+// with V, X, Y, Z the velocity and the columns of B D^-1 (role 0), or zero and
+// the rows of the stress (role 1): 2 multiply-adds per node and channel.
+// A particle's 16 columns (2D: 4) take 32 lanes (2D: 8); half of that, two
+// columns a lane, needed 28% more registers and measured slower (FP64 0.41 ms
+// against 0.33 on the 1M collapse).
+//
+// Bound: FP64 issue and shared-memory loads of the factors.
+// @MEASURED_P2G@
 // ---------------------------------------------------------------------------
 constexpr int kChunk = 128;  // default block size of the tile kernels
 // Largest block of the tile kernels.  The scatter kernels stage one particle
@@ -727,7 +736,7 @@ constexpr int kMaxTileThreads = 256;
 // that run the return mapping; it bounds their registers per thread.  Four
 // blocks of 128 threads (128 registers, some spilled to L1) measured 15-25%
 // faster for k_defgrad_t than the unbounded two blocks (240 registers) on the
-// 3D collapse; three blocks measured best for k_g2p_t on the 3D Cam-Clay incline.
+// 3D collapse.
 // The FP32-storage form holds fewer live values and gains from a tighter bound:
 // six blocks of 128 threads (80 registers) measured 6% faster for its
 // k_defgrad_t on the 3D collapse than four.  The FP64 form keeps four: six
@@ -739,91 +748,75 @@ constexpr int kMaxTileThreads = 256;
 #ifndef MTR_DEFGRAD_MIN_BLOCKS_F32
 #define MTR_DEFGRAD_MIN_BLOCKS_F32 6
 #endif
-#ifndef MTR_G2P_MIN_BLOCKS
-#define MTR_G2P_MIN_BLOCKS 3
-#endif
+// Resident blocks of kChunk threads of k_g2p_t: with one plastic model compiled
+// in, four in FP64 and five with FP32 storage (1.2M Cam-Clay incline FP64 0.505
+// -> 0.488 ms, mixed 0.458 -> 0.392, 2M DP mixed 0.339 -> 0.299 against three);
+// three for the generic kernel, which spills under more (150k elastic FP64
+// 0.050 against 0.062).
+template <typename R, int PM>
+constexpr int g2p_min_blocks() {
+  return PM < 0 ? 3 : (sizeof(R) == 4 ? 5 : 4);
+}
 // the same register bound for blocks of up to kMaxTileThreads threads (R is
 // the storage type of the kernel the bound is written on)
+// (the generic kernel spills 1.8 KB a thread under the FP32 form's bound: it takes the FP64 one's)
 #define MTR_DEFGRAD_BOUNDS \
-  kMaxTileThreads, ((sizeof(R) == 4 ? MTR_DEFGRAD_MIN_BLOCKS_F32 : MTR_DEFGRAD_MIN_BLOCKS) * kChunk / kMaxTileThreads)
+  kMaxTileThreads, ((sizeof(R) == 4 && PM >= 0 ? MTR_DEFGRAD_MIN_BLOCKS_F32 : MTR_DEFGRAD_MIN_BLOCKS) * kChunk / kMaxTileThreads)
 
-// FP64 stage: the position is kept and node offsets are formed in phase 2.
-template <int D, typename R = double>
-struct PStage {
-  double x[D], v[D], B[D * D], tau[Sym<D>::n], w[D * 4], dw[D * 4];
-  double mui;
-  int lb;  // packed local stencil base (4 bits per axis); -1 marks an empty slot
-  int pad;
-};
-
-// FP32 stage: node offsets x_i - x_p are formed in FP64 in phase 1 and
-// stored rounded, so phase 2 runs in FP32 only.
-template <int D>
-struct PStage<D, float> {
-  float pd[D * 4], v[D], B[D * D], tau[Sym<D>::n], w[D * 4], dw[D * 4];
-  float mui;
-  int lb;
-};
-
+#ifndef MTR_P2G_MIN_BLOCKS
+#define MTR_P2G_MIN_BLOCKS 2
+#endif
+#ifndef MTR_P2G_MIN_BLOCKS_F32
+#define MTR_P2G_MIN_BLOCKS_F32 3
+#endif
+#define MTR_P2G_BOUNDS kMaxTileThreads, (sizeof(R) == 4 ? MTR_P2G_MIN_BLOCKS_F32 : MTR_P2G_MIN_BLOCKS)
+// A staged particle of the P2G: per axis the 4 weights and the second factor
+// of each role, the channel factors V, X, Y, Z (2D: V, X, Z) of each role.
+// Padded to an odd multiple of 16 bytes, so that the lanes that stage
+// neighbouring slots store to different banks (a 512-byte stride made the
+// FP64 stores 16-way conflicts, 65% of the kernel's shared-memory cycles).
 template <int D, typename R>
-__device__ __forceinline__ R stage_pd(const PStage<D, R>& S, const double (*crd)[Tiling<D>::PN], int a, int lba,
-                                      int o) {
-  if constexpr (kFP64<R>)
-    return crd[a][lba + o] - S.x[a];
-  else
-    return S.pd[a * 4 + o];
+struct PStageData {
+  R w[D][4], a[2][D][4];
+  R q[2][D][4];
+  R mui;  // factor of role 1's fourth channel, the mu(I) deviation (role 0: 1, the mass)
+};
+constexpr size_t stage_stride(size_t n) {
+  n = align16(n);
+  return n % 32 ? n : n + 16;
 }
+template <int D, typename R>
+struct __align__(16) PStage : PStageData<D, R> {
+  char pad[stage_stride(sizeof(PStageData<D, R>)) - sizeof(PStageData<D, R>)];
+};
+constexpr int kTinyWeight = 1 << 12;  // some node of the particle may fall under the weight threshold
 
-// Particles staged per chunk by a scatter block of `threads` threads:
-// threads / DIV.  A smaller chunk needs less shared memory per block (more
-// resident blocks per SM) at the price of more chunk barriers and shorter
-// register runs per lane group.  Measured on the 1M 3D collapse and the 1.2M
-// incline (ms per launch at each kernel's best block shape): P2G with half
-// chunks FP64 0.461 -> 0.449, mixed 0.252 -> 0.245, at 256 threads FP64
-// 0.682 -> 0.471; the MUSL scatter slower with them (mixed 0.252 -> 0.309),
-// so it keeps full chunks.
-// The scatters stage B already multiplied by D^-1 (apicDinverse) and P2G the
-// stress already multiplied by 1/dx, so phase 2 (run by every lane of a
-// particle's group) does not repeat those products.
-// The scatters' test of the reference's weight threshold as a select (a
-// zero weight adds nothing) instead of a branch around each node's sums; the
-// branch split the unrolled node loop.  Measured (ms per launch at the best
-// shape): FP64 P2G 0.391 -> 0.370 on the 1M collapse and 0.511 -> 0.471 on the
-// 1.2M incline, mixed P2G 0.244 -> 0.237, FP64 MUSL 0.397 -> 0.375.
-#ifndef MTR_SCATTER_SELECT
-#define MTR_SCATTER_SELECT 1
-#endif
-#ifndef MTR_SCATTER_PRESCALE
-#define MTR_SCATTER_PRESCALE 1
-#endif
-// With half chunks, every P2G thread takes part in staging: two threads per
-// staged particle (otherwise half the block waits at the barrier after the
-// staging, the kernel's top stall): FP64 P2G 0.369 -> 0.356 ms on the 1M
-// collapse and 0.473 -> 0.452 on the 1.2M incline, mixed 0.238 -> 0.232.
-#ifndef MTR_P2G_PAIR_STAGE
-#define MTR_P2G_PAIR_STAGE 1
-#endif
-#ifndef MTR_P2G_CHUNK_DIV
-#define MTR_P2G_CHUNK_DIV 2
-#endif
+// Lane groups of a scatter warp: each of a particle's stencil columns takes
+// ROLES lanes (P2G: mass and momentum, force; MUSL: one).
+template <int D, int ROLES>
+struct ScatterShape {
+  static constexpr int COLS = D == 3 ? 16 : 4;  // stencil columns
+  static constexpr int LPP = COLS * ROLES;      // lanes of a group
+  static constexpr int GR = 32 / LPP;           // groups of a warp
+  static constexpr int CH = COLS;               // particles a group stages at a time (P2G: two lanes each)
+};
+constexpr int kUnits = 16;      // units of 4 cells of a tile
+constexpr int kGroupPad = 64;   // bytes between the groups' stages (different banks)
+
 // Largest block of the MUSL scatter and the resident blocks of that size its
-// register bound asks for.  Capped at 128 threads with five resident blocks
-// (at most 102 registers; the FP64 form had 124): FP64 MUSL 0.413 -> 0.399 ms,
-// mixed 0.297 -> 0.265 on the 1M collapse at step 300 (256-thread blocks,
-// which the bound rules out, never measured fastest for this kernel).
+// register bound asks for (FP64 and FP32 storage): what leaves the gather
+// without spills (1M collapse, FP64 0.363 ms at 3, 0.380 at 4 and 0.382 at 5;
+// mixed 0.230 at 5, 0.242 at 6).
 #ifndef MTR_MUSL_MAX_THREADS
 #define MTR_MUSL_MAX_THREADS 128
 #endif
 #ifndef MTR_MUSL_MIN_BLOCKS
-#define MTR_MUSL_MIN_BLOCKS 5
+#define MTR_MUSL_MIN_BLOCKS 3
 #endif
-#ifndef MTR_MUSL_CHUNK_DIV
-#define MTR_MUSL_CHUNK_DIV 1
+#ifndef MTR_MUSL_MIN_BLOCKS_F32
+#define MTR_MUSL_MIN_BLOCKS_F32 5
 #endif
-template <typename S, int DIV>
-constexpr size_t stage_bytes(int threads) {
-  return sizeof(S) * (size_t)(threads / DIV);
-}
+#define MTR_MUSL_BOUNDS MTR_MUSL_MAX_THREADS, (sizeof(R) == 4 ? MTR_MUSL_MIN_BLOCKS_F32 : MTR_MUSL_MIN_BLOCKS)
 
 template <int D, typename R>
 constexpr size_t p2g_crd_bytes() {
@@ -837,15 +830,25 @@ __host__ __device__ constexpr size_t p2g_patch_bytes(bool mibf) {
   return align16(sizeof(R) * (Tiling<D>::NCH - (mibf ? 0 : 1)) * Tiling<D>::NODES);
 }
 template <int D, typename R>
+__host__ __device__ constexpr size_t p2g_group_bytes() {
+  return ScatterShape<D, 2>::CH * sizeof(PStage<D, R>) + kGroupPad;
+}
+template <int D, typename R>
 constexpr size_t p2g_smem_bytes(int threads, bool mibf = true) {
-  return p2g_crd_bytes<D, R>() + p2g_patch_bytes<D, R>(mibf) + stage_bytes<PStage<D, R>, MTR_P2G_CHUNK_DIV>(threads);
+  return p2g_crd_bytes<D, R>() + p2g_patch_bytes<D, R>(mibf) +
+         ScatterShape<D, 2>::GR * p2g_group_bytes<D, R>() * (size_t)(threads / 32);
 }
 
-template <int D, int DEG, typename R, int XS = 1>
+// local stencil base along axis a of the particles of cell c of a tile at n0
+// (the cell's floor, clamped at the grid's first node, p2g.cpp:21-24)
+__device__ __forceinline__ int cell_base(int n0, int c) { return max(n0 + c, 0) - n0; }
+
+template <int D, int DEG, typename R>
 __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid, const uint32_t nblk) {
   using TL = Tiling<D>;
-  constexpr int PN = TL::PN, NODES = TL::NODES, NCH = TL::NCH, TB = TL::TB;
-  constexpr int NS = Sym<D>::n;
+  using SS = ScatterShape<D, 2>;
+  constexpr int PN = TL::PN, NODES = TL::NODES, NCH = TL::NCH, TB = TL::TB, Z = D - 1;
+  constexpr int LPP = SS::LPP, GR = SS::GR, CH = SS::CH, NC = D + 1;
   const StepHeader* H = A.H;
   if (step_inactive(H)) return;
   const uint32_t t = bid;
@@ -859,8 +862,6 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
   R(*patch)[NODES] = reinterpret_cast<R(*)[NODES]>(smem_raw + p2g_crd_bytes<D, R>());
   const bool mibf = P.use_mibf;
   const int nch = mibf ? NCH : NCH - 1;  // channels the patch holds
-  PStage<D, R>* st =
-      reinterpret_cast<PStage<D, R>*>(smem_raw + p2g_crd_bytes<D, R>() + p2g_patch_bytes<D, R>(mibf));
   int tc[3];
   tile_coords<D>(H, t, tc);
   const int n0[3] = {tc[0] * TB - 1, tc[1] * TB - 1, D == 3 ? tc[2] * TB - 1 : 0};
@@ -871,245 +872,197 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
     const double* ax = a == 0 ? A.gx : (a == 1 ? A.gy : A.gz);
     crd[a][o] = (g >= 0 && g < (int)H->N[a]) ? ax[g] : 0.0;
   }
+  __shared__ uint32_t cstart[65];  // first particle of each cell of the tile
+  for (int i = threadIdx.x; i < 65; i += blockDim.x) cstart[i] = A.cell_start[t * 64u + i];
   __syncthreads();
   const uint32_t Np = A.Np;
   const double ioh = P.one_over_dx;
-  const R iohR = (R)ioh, apicD = (R)P.apicDinverse;
+  const R iohR = (R)ioh, dxR = (R)P.dx, apicD = (R)P.apicDinverse;
   const bool apic = P.flip_ratio < 0;
-  const int lane = threadIdx.x & 31;
-  // XS lanes share a stencil column, each owning HN = 4 / XS of its x nodes
-  constexpr int COLS = D == 3 ? 16 : 4, LPP = COLS * XS, HN = 4 / XS;
-  const int q = lane % LPP;
-  const int iy = D == 3 ? ((q % COLS) >> 2) : q % COLS;
-  const int iz = D == 3 ? ((q % COLS) & 3) : 0;
-  const int h0 = (q / COLS) * HN;
-  // group g takes the consecutive staged particles [g*LPP, (g+1)*LPP) of the
-  // warp's 32, so groups work on different cells and their flushes rarely
-  // meet on one patch node (interleaving them made both groups flush the same
-  // cell at once, which measured slower despite fewer bank conflicts)
-  // (with a chunk of blockDim / MTR_P2G_CHUNK_DIV particles, a group takes
-  // LPP / MTR_P2G_CHUNK_DIV of them)
-  static_assert(LPP % MTR_P2G_CHUNK_DIV == 0, "chunk divisor must divide the lanes per particle");
-  constexpr int PPG = LPP / MTR_P2G_CHUNK_DIV;
-  const int chunk = (int)blockDim.x / MTR_P2G_CHUNK_DIV;
-  const int kbeg = ((int)threadIdx.x / LPP) * PPG, kend = kbeg + PPG;
-  for (uint32_t c0 = pb; c0 < pe; c0 += chunk) {
-    if constexpr (MTR_P2G_PAIR_STAGE && MTR_P2G_CHUNK_DIV == 2) {
-      // phase 1, two threads per staged particle: thread t < chunk loads the
-      // position, velocity and B and evaluates the weights; thread t + chunk
-      // loads the stress and mu(I) and evaluates the weight derivatives
-      const int role = (int)threadIdx.x >= chunk ? 1 : 0;
-      const int slot = (int)threadIdx.x - role * chunk;
-      const uint32_t s = c0 + (uint32_t)slot;
-      PStage<D, R>& S = st[slot];
-      int packed = -1;
-      if (s < pe) {
-        const uint32_t j = perm[s];
-        double xp[3] = {0.0, 0.0, 0.0};
-        int lb[3] = {0, 0, 0};
-        bool oob = false;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int grp = lane / LPP, q = lane % LPP;
+  const int role = q / (LPP / 2), ci = q % (LPP / 2);
+  const int ix = D == 3 ? ci >> 2 : ci, iy = D == 3 ? ci & 3 : 0;  // this lane's column
+  PStage<D, R>* st = reinterpret_cast<PStage<D, R>*>(smem_raw + p2g_crd_bytes<D, R>() + p2g_patch_bytes<D, R>(mibf) +
+                                                     (size_t)(warp * GR + grp) * p2g_group_bytes<D, R>());
+  // patch channels of this role: c < D vector component, c == D mass or friction
+  R* const vec = patch[role ? 1 + D : 1];
+  R* const one = patch[role ? 1 + 2 * D : 0];
+  R acc[4][NC];
 #pragma unroll
-        for (int a = 0; a < D; ++a) {
-          xp[a] = A.in.x[(size_t)a * Np + j];
-          int b = (int)floor((xp[a] - H->org[a]) * ioh) - 1;
-          b = b < 0 ? 0 : b;  // p2g.cpp:21-24 clamps at zero
-          lb[a] = b - n0[a];
-          if (lb[a] < 0 || lb[a] > PN - 4 || b + 3 >= (int)H->N[a]) oob = true;
-        }
+  for (int h = 0; h < 4; ++h)
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[h][c] = R(0.0);
+  int node0 = 0;  // node of the window's first entry
+  // adds the first node of the window to the patch and moves the window by one
+  auto advance = [&]() {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const R v = acc[0][c];
+      if (v != R(0.0)) atomicAdd(c < D ? &vec[c * NODES + node0] : &one[node0], v);
+#pragma unroll
+      for (int h = 0; h < 3; ++h) acc[h][c] = acc[h + 1][c];
+      acc[3][c] = R(0.0);
+    }
+    ++node0;
+  };
+  // adds a staged particle to the window; TINY: some node may fall under the
+  // weight threshold of p2g.cpp:35 (mass and momentum of weights <= 1e-25 are
+  // skipped, which is checked node by node for such a particle)
+  auto add = [&](const PStage<D, R>& S, auto tiny) {
+    R f1[4], f2[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      f1[h] = S.w[Z][h];
+      f2[h] = S.a[role][Z][h];
+    }
+    R u0 = S.w[0][ix], u1 = S.a[role][0][ix];
+    [[maybe_unused]] R u2 = R(0.0);
+    if constexpr (D == 3) {
+      const R wy = S.w[1][iy], ay = S.a[role][1][iy];
+      u2 = u0 * ay;
+      u0 *= wy;
+      u1 *= wy;
+    }
+    if constexpr (decltype(tiny)::value) {
+#pragma unroll
+      for (int h = 0; h < 4; ++h)
+        if (role == 0 && !(f1[h] * u0 > R(1e-25))) f1[h] = f2[h] = R(0.0);
+    }
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+      R a1 = u0 * S.q[role][c][0] + u1 * S.q[role][c][1];
+      if constexpr (D == 3) a1 += u2 * S.q[role][c][2];
+      const R b1 = u0 * S.q[role][c][D];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) acc[h][c] = f2[h] * b1 + (f1[h] * a1 + acc[h][c]);
+    }
+    const R a1 = u0 * (role ? S.mui : R(1.0));
+#pragma unroll
+    for (int h = 0; h < 4; ++h) acc[h][D] += f1[h] * a1;
+  };
+  for (int u0 = warp * GR; u0 < kUnits; u0 += nwarps * GR) {
+    const int c1 = 4 * (u0 + grp);  // first cell of the unit
+    const uint32_t ub = cstart[c1], count = cstart[c1 + 4] - ub;
+    const uint32_t most = GR == 1 ? count : __reduce_max_sync(0xffffffffu, count);
+    if (most == 0) continue;
+    // stencil base of the unit's cells; along the innermost axis that of its first cell
+    const int bx = cell_base(n0[0], D == 3 ? c1 >> 4 : c1 >> 3), by = D == 3 ? cell_base(n0[1], (c1 >> 2) & 3) : 0;
+    const int z1 = D == 3 ? 0 : c1 & 7;
+    node0 = D == 3 ? ((bx + ix) * PN + by + iy) * PN + cell_base(n0[Z], 0) : (bx + ix) * PN + cell_base(n0[Z], z1);
+    int cz = 0;  // cell of the unit the window is at
+    for (uint32_t k0 = 0; k0 < most; k0 += CH) {
+      __syncwarp();  // the last chunk has been read
+      // Two lanes per staged particle: role 0 stores the weights, the weights
+      // times offsets, velocity and B, role 1 the weight derivatives, the
+      // stress and mu(I).  Both evaluate both second factors and keep theirs:
+      // a branch on the role would run the two halves one after the other.
+      bool tiny = false;
+      for (int slot = ci; slot < CH; slot += LPP / 2) {
+        if (k0 + slot >= count) break;
+        PStage<D, R>& S = st[slot];
+        const uint32_t s = ub + k0 + slot, j = perm[s];
+        double xp[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int a = 0; a < D; ++a) xp[a] = A.in.x[(size_t)a * Np + j];
+        R qv[D][1 + D], mui = R(0.0);
         if (role == 0) {
 #pragma unroll
           for (int a = 0; a < D; ++a) {
-            if constexpr (kFP64<R>) S.x[a] = xp[a];
-            S.v[a] = A.in.v[(size_t)a * Np + j];
-          }
+            qv[a][0] = A.in.v[(size_t)a * Np + j];
 #pragma unroll
-          for (int q = 0; q < D * D; ++q)
-            S.B[q] = apic ? (MTR_SCATTER_PRESCALE ? apicD * A.in.B[(size_t)q * Np + j] : A.in.B[(size_t)q * Np + j])
-                          : R(0.0);
-          if (oob) {
-            raise_status(A.H, MTR_STATUS_STENCIL_OOB, A.in.id[j]);
-          } else {
-#pragma unroll
-            for (int a = 0; a < D; ++a) {
-#pragma unroll
-              for (int o = 0; o < 4; ++o) {
-                const double c = crd[a][lb[a] + o];
-                S.w[a * 4 + o] = bspline_N<DEG>((R)((xp[a] - c) * ioh));
-                if constexpr (!kFP64<R>) S.pd[a * 4 + o] = (R)(c - xp[a]);
-              }
-            }
-            packed = lb[0] | (lb[1] << 4) | (lb[2] << 8);
+            for (int b = 0; b < D; ++b)
+              qv[a][1 + b] = apic ? apicD * A.in.B[(size_t)(a * D + b) * Np + j] : R(0.0);
           }
         } else {
+          R tau[Sym<D>::n];
 #pragma unroll
-          for (int q = 0; q < NS; ++q)
-            S.tau[q] = MTR_SCATTER_PRESCALE ? iohR * A.in.tau[(size_t)q * Np + j] : A.in.tau[(size_t)q * Np + j];
-          S.mui = mibf ? (R)((double)A.in.sc[(size_t)MTR_SCALAR_MUI * Np + j] - P.mui0) : R(0.0);
-          if (!oob) {
+          for (int i = 0; i < Sym<D>::n; ++i) tau[i] = iohR * A.in.tau[(size_t)i * Np + j];
 #pragma unroll
-            for (int a = 0; a < D; ++a) {
+          for (int a = 0; a < D; ++a) {
+            qv[a][0] = R(0.0);
 #pragma unroll
-              for (int o = 0; o < 4; ++o) {
-                const double c = crd[a][lb[a] + o];
-                S.dw[a * 4 + o] = bspline_dN<DEG>((R)((xp[a] - c) * ioh));
-              }
-            }
+            for (int b = 0; b < D; ++b) qv[a][1 + b] = sym_at<D>(tau, a, b);
           }
+          if (mibf) mui = (R)((double)A.in.sc[(size_t)MTR_SCALAR_MUI * Np + j] - P.mui0);
         }
-      }
-      if (role == 0) S.lb = packed;
-    } else if ((int)threadIdx.x < chunk) {  // phase 1: stage one particle per thread
-      const uint32_t s = c0 + threadIdx.x;
-      PStage<D, R>& S = st[threadIdx.x];
-      int packed = -1;
-      if (s < pe) {
-        const uint32_t j = perm[s];
-        double xp[3] = {0.0, 0.0, 0.0};
-        int lb[3] = {0, 0, 0};
-        bool oob = false;
+        // the particle's base must be its cell's (it is, unless its position is
+        // not finite or left of the grid) and its stencil inside the grid
+        const int zc = z1 + (s >= cstart[c1 + 1]) + (s >= cstart[c1 + 2]) + (s >= cstart[c1 + 3]);
+        const int lb[3] = {bx, D == 3 ? by : cell_base(n0[Z], zc), D == 3 ? cell_base(n0[Z], zc) : 0};
+        bool ok = true;
+        int least = 0;
 #pragma unroll
         for (int a = 0; a < D; ++a) {
-          xp[a] = A.in.x[(size_t)a * Np + j];
-          if constexpr (kFP64<R>) S.x[a] = xp[a];
-          S.v[a] = A.in.v[(size_t)a * Np + j];
-          int b = (int)floor((xp[a] - H->org[a]) * ioh) - 1;
-          b = b < 0 ? 0 : b;  // p2g.cpp:21-24 clamps at zero
-          lb[a] = b - n0[a];
-          if (lb[a] < 0 || lb[a] > PN - 4 || b + 3 >= (int)H->N[a]) oob = true;
+          const int b = (int)floor((xp[a] - H->org[a]) * ioh) - 1;
+          ok = ok && max(b, 0) == lb[a] + n0[a] && lb[a] + n0[a] + 3 < (int)H->N[a];
+          const double td = (xp[a] - crd[a][lb[a] + 1]) * ioh;
+          R w[4], d[4], o[4];
+          axis_weights<DEG, true, R>(td, w, d);
+          if (b < 0) {  // clamped; through copies: w and d stay in registers otherwise
+            R wc[4], dc[4];
+            axis_weights_any<DEG, R>(td, wc, dc);
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+              w[h] = wc[h];
+              d[h] = dc[h];
+            }
+          }
+          axis_offsets<R>(td, dxR, o);
+          least += least_exponent<DEG>(w);
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            if (role == 0) S.w[a][h] = w[h];
+            S.a[role][a][h] = role ? d[h] : w[h] * o[h];
+          }
         }
 #pragma unroll
-        for (int q = 0; q < D * D; ++q)
-          S.B[q] = apic ? (MTR_SCATTER_PRESCALE ? apicD * A.in.B[(size_t)q * Np + j] : A.in.B[(size_t)q * Np + j])
-                        : R(0.0);
+        for (int a = 0; a < D; ++a)
 #pragma unroll
-        for (int q = 0; q < NS; ++q)
-          S.tau[q] = MTR_SCATTER_PRESCALE ? iohR * A.in.tau[(size_t)q * Np + j] : A.in.tau[(size_t)q * Np + j];
-        // MIBF friction is accumulated as the deviation from its initial value
-        // mui0, so a uniform field reproduces mui0 exactly at every node
-        S.mui = mibf ? (R)((double)A.in.sc[(size_t)MTR_SCALAR_MUI * Np + j] - P.mui0) : R(0.0);
-        if (oob) {
-          raise_status(A.H, MTR_STATUS_STENCIL_OOB, A.in.id[j]);
-        } else {
+          for (int b = 0; b < 1 + D; ++b) S.q[role][a][b] = qv[a][b];
+        if (role) S.mui = mui;
+        tiny = tiny || least < -82;  // every product of weights is at least 2^least; 1e-25 < 2^-83
+        if (!ok) {  // adds nothing
+          if (role == 0) {
+            raise_status(A.H, MTR_STATUS_STENCIL_OOB, A.in.id[j]);
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+#pragma unroll
+              for (int h = 0; h < 4; ++h) S.w[a][h] = R(0.0);
+          }
 #pragma unroll
           for (int a = 0; a < D; ++a) {
 #pragma unroll
-            for (int o = 0; o < 4; ++o) {
-              const double c = crd[a][lb[a] + o];
-              const R u = (R)((xp[a] - c) * ioh);
-              S.w[a * 4 + o] = bspline_N<DEG>(u);
-              S.dw[a * 4 + o] = bspline_dN<DEG>(u);
-              if constexpr (!kFP64<R>) S.pd[a * 4 + o] = (R)(c - xp[a]);
-            }
+            for (int h = 0; h < 4; ++h) S.a[role][a][h] = R(0.0);
+#pragma unroll
+            for (int b = 0; b < 1 + D; ++b) S.q[role][a][b] = R(0.0);
           }
-          packed = lb[0] | (lb[1] << 4) | (lb[2] << 8);
+          if (role) S.mui = R(0.0);
         }
       }
-      S.lb = packed;
-    }
-    __syncthreads();
-    {  // phase 2: a lane owns one (iy, iz) stencil column and HN of its ix nodes
-      R acc[HN][NCH];
-#pragma unroll
-      for (int h = 0; h < HN; ++h)
-#pragma unroll
-        for (int ch = 0; ch < NCH; ++ch) acc[h][ch] = R(0.0);
-      int cur = -1;
-      auto flush = [&]() {
-        const int lbx = cur & 15, lby = (cur >> 4) & 15, lbz = cur >> 8;
-#pragma unroll
-        for (int hh = 0; hh < HN; ++hh) {
-          const int h = h0 + hh;
-          const int node = D == 3 ? ((lbx + h) * PN + (lby + iy)) * PN + (lbz + iz) : (lbx + h) * PN + (lby + iy);
-#pragma unroll
-          for (int ch = 0; ch < NCH; ++ch) {  // the friction accumulator stays zero without MIBF
-            if (acc[hh][ch] != R(0.0)) atomicAdd(&patch[ch][node], acc[hh][ch]);
-            acc[hh][ch] = R(0.0);
-          }
-        }
-      };
-      for (int k = kbeg; k < kend; ++k) {
-        const PStage<D, R>& S = st[k];
-        const int lbp = S.lb;
-        if (lbp < 0) continue;
-        if (lbp != cur) {
-          if (cur >= 0) flush();
-          cur = lbp;
-        }
-        const int lbx = lbp & 15, lby = (lbp >> 4) & 15, lbz = lbp >> 8;
-        // tensor-product factors of this lane's column
-        const R wy = S.w[4 + iy], dwy = S.dw[4 + iy];
-        R wyz, G0, G1, G2 = R(0.0);
-        if constexpr (D == 3) {
-          const R wz = S.w[8 + iz], dwz = S.dw[8 + iz];
-          wyz = wy * wz;
-          if constexpr (MTR_SCATTER_PRESCALE) {
-            G0 = wyz;
-            G1 = dwy * wz;
-            G2 = wy * dwz;
-          } else {
-            G0 = wyz * iohR;
-            G1 = dwy * wz * iohR;
-            G2 = wy * dwz * iohR;
-          }
+      const bool slow = __any_sync(0xffffffffu, tiny);  // (also orders the stage before its reads)
+      __syncwarp();
+      const int kend = count > k0 ? min((int)(count - k0), CH) : 0;
+      for (int k = 0; k < kend;) {
+        const int cend = (int)(cstart[c1 + cz + 1] - ub - k0);  // the cell's end within the chunk
+        const int e = min(cend, kend);
+        if (slow) {
+#pragma unroll 1
+          for (; k < e; ++k) add(st[k], std::true_type{});
         } else {
-          wyz = wy;
-          G0 = MTR_SCATTER_PRESCALE ? wy : wy * iohR;
-          G1 = MTR_SCATTER_PRESCALE ? dwy : dwy * iohR;
+#pragma unroll 2
+          for (; k < e; ++k) add(st[k], std::false_type{});
         }
-        // force f_a = tau_a . grad w = dwx * Pf_a + wx * Qf_a
-        R Pf[D], Qf[D];
-#pragma unroll
-        for (int a = 0; a < D; ++a) {
-          Pf[a] = sym_at<D>(S.tau, a, 0) * G0;
-          R q = sym_at<D>(S.tau, a, 1) * G1;
-          if constexpr (D == 3) q += sym_at<D>(S.tau, a, 2) * G2;
-          Qf[a] = q;
-        }
-        // momentum per weight: v_a + apicD B_a . (x_i - x_p) = Tm_a + Sm_a * pdx
-        const R pdy = stage_pd<D, R>(S, crd, 1, lby, iy);
-        const R pdz = D == 3 ? stage_pd<D, R>(S, crd, D - 1, lbz, iz) : R(0.0);
-        R Tm[D], Sm[D];
-#pragma unroll
-        for (int a = 0; a < D; ++a) {
-          if (apic) {
-            R byz = S.B[a * D + 1] * pdy;
-            if constexpr (D == 3) byz += S.B[a * D + 2] * pdz;
-            Tm[a] = S.v[a] + (MTR_SCATTER_PRESCALE ? byz : apicD * byz);
-            Sm[a] = MTR_SCATTER_PRESCALE ? S.B[a * D] : apicD * S.B[a * D];
-          } else {
-            Tm[a] = S.v[a];
-            Sm[a] = R(0.0);
-          }
-        }
-        const R mui = S.mui;
-#pragma unroll
-        for (int hh = 0; hh < HN; ++hh) {
-          const int h = h0 + hh;
-          const R wx = S.w[h], dwx = S.dw[h];
-          const R weight = wx * wyz;
-          if constexpr (MTR_SCATTER_SELECT) {
-            // p2g.cpp:35 skips weights <= 1e-25; a zero weight adds nothing
-            const R ws = weight > R(1e-25) ? weight : R(0.0);
-            const R pdx = stage_pd<D, R>(S, crd, 0, lbx, h);
-            acc[hh][0] += ws;
-#pragma unroll
-            for (int a = 0; a < D; ++a) acc[hh][1 + a] += ws * (Tm[a] + Sm[a] * pdx);
-            if (mibf) acc[hh][1 + 2 * D] += mui * ws;
-          } else if (weight > R(1e-25)) {
-            const R pdx = stage_pd<D, R>(S, crd, 0, lbx, h);
-            acc[hh][0] += weight;
-#pragma unroll
-            for (int a = 0; a < D; ++a) acc[hh][1 + a] += weight * (Tm[a] + Sm[a] * pdx);
-            if (mibf) acc[hh][1 + 2 * D] += mui * weight;
-          }
-#pragma unroll
-          for (int a = 0; a < D; ++a) acc[hh][1 + D + a] += dwx * Pf[a] + wx * Qf[a];
-        }
+        if (cend > kend || cz == 3) break;  // the cell goes on in the next chunk, or the unit ends
+        // the next cell; its base is the same where both are clamped
+        if (cell_base(n0[Z], z1 + cz + 1) != cell_base(n0[Z], z1 + cz)) advance();
+        ++cz;
       }
-      if (cur >= 0) flush();
     }
-    __syncthreads();
+#pragma unroll 1
+    for (int h = 0; h < 4; ++h) advance();
   }
+  __syncthreads();
   const uint32_t cap = A.cap_nodes;
   for (int n = threadIdx.x; n < NODES; n += blockDim.x) {
     uint32_t l;
@@ -1123,9 +1076,9 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
   }
 }
 
-template <int D, int DEG, typename R, int XS = 1>
-__global__ void __launch_bounds__(kMaxTileThreads) k_p2g_w(StepArgsT<R> A, const uint32_t* __restrict__ perm) {
-  p2g_w_body<D, DEG, R, XS>(A, perm, blockIdx.x, gridDim.x);
+template <int D, int DEG, typename R>
+__global__ void __launch_bounds__(MTR_P2G_BOUNDS) k_p2g_w(StepArgsT<R> A, const uint32_t* __restrict__ perm) {
+  p2g_w_body<D, DEG, R>(A, perm, blockIdx.x, gridDim.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1531,40 +1484,48 @@ __device__ __forceinline__ void load_patch(const StepCommon& A, const StepHeader
 
 // G2P gather (g2p.cpp:24-77) and velocity gradient (deformation_update.cpp:17-40)
 // from a shared node patch; lb = stencil base relative to the patch origin.
-// The offsets and the spline argument are formed in FP64 from the FP64
-// position, then rounded to R.  The patch holds node velocities minus vref:
-// B-spline weights sum to one and reproduce linears, so pic = vref + sum w dv,
-// while B and grad v need the deviations only.
+// The position in the cell is formed in FP64 from the FP64 position, then
+// rounded to R.  The patch holds node velocities minus vref: B-spline weights
+// sum to one and reproduce linears, so pic = vref + sum w dv, while B and
+// grad v need the deviations only.
 //
-// The sums are factorised over the tensor-product stencil, innermost axis
-// first: per node only sum w_z v, sum w_z dz v, sum w_z' v and sum w_z flip
-// are formed, rows of 4 nodes are then combined with the y factors and planes
-// of 16 with the x factors.  USL in 3D takes 12 multiply-adds per node and
-// 18 per row instead of 32 per node, MUSL 9 instead of 20, and the deformation
-// update 6 instead of 12.  The x planes stay a loop: unrolling all 64 nodes
-// made the return-mapping kernels too large for the instruction cache.
-// The innermost rows are read as vectors from the interleaved patch (3D USL:
-// three 16-byte loads per node instead of six of 8 bytes in FP64).  What bounds
-// it then is FP64 issue and the registers of the sums (measured together with
-// the series return mapping, see hencky_series).
-template <int D, int DEG, bool FLIP, bool WP, bool WB, bool WF, bool GV, typename R>
+// The sums are factorised over the tensor-product stencil: per node of a row
+// along the innermost axis only sum w_z v, sum w_z dz v, sum w_z' v and sum
+// w_z flip are formed, and a row's sums are then added with its x and y
+// factors.  USL in 3D takes 12 multiply-adds per node and 24 per row of 4
+// instead of 32 per node, MUSL 9 and 15 instead of 20, the deformation update
+// 6 and 9 instead of 12.  The rows are a loop whose x and y factors wait in
+// shared memory (xf, `STRIDE` threads apart): what is live is the sums, the 4
+// factors along the innermost axis and ROWS rows.  MUSL and the deformation
+// update unroll all 4 rows of an x plane (1M collapse, FP64 0.375 -> 0.363 and
+// 0.151 -> 0.147 ms against one row at a time, mixed 0.239 -> 0.230); USL, which
+// also holds the particle for its return mapping, takes one (1.2M Cam-Clay
+// incline, FP64 0.524 -> 0.488).
+template <int D, int DEG, bool FLIP, bool WP, bool WB, bool WF, bool GV, int STRIDE, int ROWS, typename R>
 __device__ __forceinline__ void gather_sums(const R* pv, const double (*crd)[Tiling<D>::PN], const int (&lb)[3],
-                                            const double (&xp)[3], double ioh, R (&ps)[3], R (&Bp)[D][D], R (&flp)[3],
-                                            R (&gv)[D][D]) {
+                                            const double (&xp)[3], double ioh, R dx, R* xf, R (&ps)[3],
+                                            R (&Bp)[D][D], R (&flp)[3], R (&gv)[D][D]) {
   constexpr int PN = Tiling<D>::PN, STR = NodePatch<D, FLIP, R>::STRIDE;
-  constexpr int Z = D - 1;  // innermost axis
-  R wz[4], dz[4], pz[4], wy[4], dy[4], py[4];
-  auto axis = [&](int a, int o, R& w, R& dw, R& wp) {
-    const double c = crd[a][lb[a] + o];
-    const R u = (R)((xp[a] - c) * ioh);
-    w = bspline_N<DEG>(u);
-    dw = GV ? bspline_dN<DEG>(u) : R(0.0);
-    wp = WB ? w * (R)(c - xp[a]) : R(0.0);
-  };
+  constexpr int Z = D - 1;                  // innermost axis
+  constexpr int NF = (1 + WB + GV) * 4;     // factors of an axis: w, w times offset, derivative
+  constexpr int OP = 4, OD = WB ? 8 : 4;    // where the last two start
+  R wz[4], dz[4], pz[4];
 #pragma unroll
-  for (int o = 0; o < 4; ++o) {
-    axis(Z, o, wz[o], dz[o], pz[o]);
-    if constexpr (D == 3) axis(1, o, wy[o], dy[o], py[o]);
+  for (int a = 0; a < D; ++a) {
+    const double td = (xp[a] - crd[a][lb[a] + 1]) * ioh;
+    axis_weights<DEG, GV, R>(td, wz, dz);
+    if constexpr (WB) {
+      axis_offsets<R>(td, dx, pz);
+#pragma unroll
+      for (int o = 0; o < 4; ++o) pz[o] *= wz[o];
+    }
+    if (a == Z) break;
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {
+      xf[(a * NF + o) * STRIDE] = wz[o];
+      if constexpr (WB) xf[(a * NF + OP + o) * STRIDE] = pz[o];
+      if constexpr (GV) xf[(a * NF + OD + o) * STRIDE] = dz[o];
+    }
   }
 #pragma unroll
   for (int a = 0; a < 3; ++a) ps[a] = flp[a] = R(0.0);
@@ -1573,70 +1534,59 @@ __device__ __forceinline__ void gather_sums(const R* pv, const double (*crd)[Til
 #pragma unroll
     for (int c = 0; c < D; ++c) Bp[r][c] = gv[r][c] = R(0.0);
   const R* plane = pv + (D == 3 ? (lb[0] * PN + lb[1]) * PN + lb[2] : lb[0] * PN + lb[1]) * STR;
-  // sums of one row of 4 nodes along the innermost axis
-  auto row = [&](const R* q, R (&s0)[3], R (&s1)[3], R (&s2)[3], R (&f0)[3]) {
-#pragma unroll
-    for (int a = 0; a < D; ++a) s0[a] = s1[a] = s2[a] = f0[a] = R(0.0);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      R v[3], f[3];
-      load_node<D, WF, R>(q + k * STR, v, f);
-#pragma unroll
-      for (int a = 0; a < D; ++a) {
-        s0[a] += wz[k] * v[a];
-        if constexpr (WB) s1[a] += pz[k] * v[a];
-        if constexpr (GV) s2[a] += dz[k] * v[a];
-        if constexpr (WF) f0[a] += wz[k] * f[a];
-      }
-    }
-  };
 #pragma unroll 1
   for (int ii = 0; ii < 4; ++ii, plane += (D == 3 ? PN * PN : PN) * STR) {
-    R wx, dx, px;
-    axis(0, ii, wx, dx, px);
-    R r0[3], rz[3], gz[3], rf[3];  // plane sums: w, w times offset (innermost), gradient (innermost), flip
-    if constexpr (D == 3) {
-      R ry[3], gy[3];
+    const R* xi = xf + ii * STRIDE;
+    const R* row = plane;
+#pragma unroll ROWS
+    for (int j = 0; j < (D == 3 ? 4 : 1); ++j, row += PN * STR) {
+      R s0[3], s1[3], s2[3], f0[3];
 #pragma unroll
-      for (int a = 0; a < 3; ++a) r0[a] = rz[a] = gz[a] = rf[a] = ry[a] = gy[a] = R(0.0);
+      for (int a = 0; a < D; ++a) s0[a] = s1[a] = s2[a] = f0[a] = R(0.0);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        R s0[3], s1[3], s2[3], f0[3];
-        row(plane + j * PN * STR, s0, s1, s2, f0);
+      for (int k = 0; k < 4; ++k) {
+        R v[3], f[3];
+        load_node<D, WF, R>(row + k * STR, v, f);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          r0[a] += wy[j] * s0[a];
-          if constexpr (WB) {
-            ry[a] += py[j] * s0[a];
-            rz[a] += wy[j] * s1[a];
-          }
-          if constexpr (GV) {
-            gy[a] += dy[j] * s0[a];
-            gz[a] += wy[j] * s2[a];
-          }
-          if constexpr (WF) rf[a] += wy[j] * f0[a];
+        for (int a = 0; a < D; ++a) {
+          s0[a] += wz[k] * v[a];
+          if constexpr (WB) s1[a] += pz[k] * v[a];
+          if constexpr (GV) s2[a] += dz[k] * v[a];
+          if constexpr (WF) f0[a] += wz[k] * f[a];
+        }
+      }
+      const R wx = xi[0];
+      R w = wx, px, py, gx, gy;  // the row's factors of v, B and grad v
+      if constexpr (WB) px = xi[OP * STRIDE];
+      if constexpr (GV) gx = xi[OD * STRIDE];
+      if constexpr (D == 3) {
+        const R* yj = xf + (NF + j) * STRIDE;
+        const R wy = yj[0];
+        w = wx * wy;
+        if constexpr (WB) {
+          px *= wy;
+          py = wx * yj[OP * STRIDE];
+        }
+        if constexpr (GV) {
+          gx *= wy;
+          gy = wx * yj[OD * STRIDE];
         }
       }
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        if constexpr (WB) Bp[a][1] += wx * ry[a];
-        if constexpr (GV) gv[a][1] += wx * gy[a];
+      for (int a = 0; a < D; ++a) {
+        if constexpr (WP) ps[a] += w * s0[a];
+        if constexpr (WB) {
+          Bp[a][0] += px * s0[a];
+          if constexpr (D == 3) Bp[a][1] += py * s0[a];
+          Bp[a][Z] += w * s1[a];
+        }
+        if constexpr (GV) {
+          gv[a][0] += gx * s0[a];
+          if constexpr (D == 3) gv[a][1] += gy * s0[a];
+          gv[a][Z] += w * s2[a];
+        }
+        if constexpr (WF) flp[a] += w * f0[a];
       }
-    } else {
-      row(plane, r0, rz, gz, rf);
-    }
-#pragma unroll
-    for (int a = 0; a < D; ++a) {
-      if constexpr (WP) ps[a] += wx * r0[a];
-      if constexpr (WB) {
-        Bp[a][0] += px * r0[a];
-        Bp[a][Z] += wx * rz[a];
-      }
-      if constexpr (GV) {
-        gv[a][0] += dx * r0[a];
-        gv[a][Z] += wx * gz[a];
-      }
-      if constexpr (WF) flp[a] += wx * rf[a];
     }
   }
 }
@@ -1644,18 +1594,19 @@ __device__ __forceinline__ void gather_sums(const R* pv, const double (*crd)[Til
 // The sums a transfer scheme needs (B for APIC and AFLIP, flip for all but
 // APIC), pic = vref + ps (the FP64 path gathers the velocities themselves) and
 // grad v scaled by 1/dx.
-template <int D, int DEG, bool GV, typename R>
+template <int D, int DEG, bool GV, int STRIDE, int ROWS, typename R>
 __device__ __forceinline__ void gather_patch(const R* pv, const double (*crd)[Tiling<D>::PN], const int (&lb)[3],
-                                             const double (&xp)[3], double ioh, const double (&vref)[3],
+                                             const double (&xp)[3], double ioh, R dx, R* xf,
+                                             const double (&vref)[3],
                                              double (&pic)[3], R (&Bp)[D][D], R (&flp)[3], R (&gv)[D][D], bool want_b,
                                              bool want_flip) {
   R ps[3];
   if (!want_flip)
-    gather_sums<D, DEG, true, true, true, false, GV, R>(pv, crd, lb, xp, ioh, ps, Bp, flp, gv);
+    gather_sums<D, DEG, true, true, true, false, GV, STRIDE, ROWS, R>(pv, crd, lb, xp, ioh, dx, xf, ps, Bp, flp, gv);
   else if (want_b)
-    gather_sums<D, DEG, true, true, true, true, GV, R>(pv, crd, lb, xp, ioh, ps, Bp, flp, gv);
+    gather_sums<D, DEG, true, true, true, true, GV, STRIDE, ROWS, R>(pv, crd, lb, xp, ioh, dx, xf, ps, Bp, flp, gv);
   else
-    gather_sums<D, DEG, true, true, false, true, GV, R>(pv, crd, lb, xp, ioh, ps, Bp, flp, gv);
+    gather_sums<D, DEG, true, true, false, true, GV, STRIDE, ROWS, R>(pv, crd, lb, xp, ioh, dx, xf, ps, Bp, flp, gv);
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     if constexpr (kFP64<R>)
@@ -1673,11 +1624,11 @@ __device__ __forceinline__ void gather_patch(const R* pv, const double (*crd)[Ti
 }
 
 // grad v alone (MUSL deformation update), from a patch without flips
-template <int D, int DEG, typename R>
+template <int D, int DEG, int STRIDE, int ROWS, typename R>
 __device__ __forceinline__ void gather_gradv(const R* pv, const double (*crd)[Tiling<D>::PN], const int (&lb)[3],
-                                             const double (&xp)[3], double ioh, R (&gv)[D][D]) {
+                                             const double (&xp)[3], double ioh, R dx, R* xf, R (&gv)[D][D]) {
   R ps[3], Bp[D][D], flp[3];
-  gather_sums<D, DEG, false, false, false, false, true, R>(pv, crd, lb, xp, ioh, ps, Bp, flp, gv);
+  gather_sums<D, DEG, false, false, false, false, true, STRIDE, ROWS, R>(pv, crd, lb, xp, ioh, dx, xf, ps, Bp, flp, gv);
   const R iohR = (R)ioh;
 #pragma unroll
   for (int r = 0; r < D; ++r)
@@ -1702,6 +1653,7 @@ __device__ __forceinline__ void g2p_t_body(const StepArgsT<R>& A, const uint32_t
   if (pb >= pe) return;
   const DevParams& P = *A.P;
   __shared__ __align__(16) R pv[NodePatch<D, true, R>::SIZE];
+  __shared__ R xfac[12 * (D - 1) * kChunk];  // x and y factors of each thread's gather
   __shared__ double crd[3][PN];
   int n0[3];
   load_tile_setup<D>(A, H, t, n0, crd);
@@ -1721,7 +1673,7 @@ __device__ __forceinline__ void g2p_t_body(const StepArgsT<R>& A, const uint32_t
     R flp[3], Bp[D][D], gv[D][D];
     int lb[3];
     if (local_base<D>(H, p.x, ioh, n0, false, lb)) {
-      gather_patch<D, DEG, true, R>(pv, crd, lb, p.x, ioh, vref, pic, Bp, flp, gv, fr < 0, fr >= -1);
+      gather_patch<D, DEG, true, kChunk, 1, R>(pv, crd, lb, p.x, ioh, (R)P.dx, xfac + threadIdx.x, vref, pic, Bp, flp, gv, fr < 0, fr >= -1);
     } else {
       raise_status(H, MTR_STATUS_STENCIL_OOB, p.id);
 #pragma unroll
@@ -1768,39 +1720,31 @@ __device__ __forceinline__ void g2p_t_body(const StepArgsT<R>& A, const uint32_t
 }
 
 template <int D, int DEG, typename R, int PM = -1>
-__global__ void __launch_bounds__(kChunk, MTR_G2P_MIN_BLOCKS) k_g2p_t(StepArgsT<R> A, const uint32_t* __restrict__ perm) {
+__global__ void __launch_bounds__(kChunk, (g2p_min_blocks<R, PM>())) k_g2p_t(StepArgsT<R> A, const uint32_t* __restrict__ perm) {
   g2p_t_body<D, DEG, R, PM>(A, perm, blockIdx.x, gridDim.x);
 }
 
 // ---------------------------------------------------------------------------
-// 7b. MUSL (musl.cpp:6-96), one block per tile.  Phase 1 (thread per
-// particle): gather pic/B/flip from the shared node patch, blend v, write
-// x + dt pic, v, B; stage v_new, B_new and the re-scatter weights.  Phase 2
-// (lane groups owning stencil columns, as in P2G): accumulate
-// v_p + B D^-1 (x_i - x_p) per cell in registers, add once per cell to the
-// shared re-projection patch, flush with one global atomic per node.
+// 7b. MUSL (musl.cpp:6-96), one block per tile, each warp on its own units as
+// in P2G.  Phase 1 (a lane per particle): gather pic/B/flip from the shared
+// node patch, blend v, write x + dt pic, v, B.  Phase 2 (lane groups owning
+// stencil columns): the particles are staged in kMuslParts parts (half of the
+// shared memory, so more blocks per SM) and v_p + B D^-1 (x_i - x_p) is summed
+// in the sliding register windows of P2G, one lane per column.
+// @MEASURED_MUSL@
 // ---------------------------------------------------------------------------
-template <int D, typename R = double>
-struct MStage {
-  double x[D], v[D], B[D * D], w[D * 4];
-  int lb;
-  int pad;
-};
-
-template <int D>
-struct MStage<D, float> {
-  float pd[D * 4], v[D], B[D * D], w[D * 4];
-  int lb;
-};
+constexpr int kMuslParts = 2;
 
 template <int D, typename R>
-__device__ __forceinline__ R stage_pd(const MStage<D, R>& S, const double (*crd)[Tiling<D>::PN], int a, int lba,
-                                      int o) {
-  if constexpr (kFP64<R>)
-    return crd[a][lba + o] - S.x[a];
-  else
-    return S.pd[a * 4 + o];
-}
+struct MStageData {
+  R w[D][4], a[D][4];  // weights and weights times offsets
+  R q[D][4];           // V, X, Y, Z (2D: V, X, Z) of each component
+  int lb;
+};
+template <int D, typename R>
+struct __align__(16) MStage : MStageData<D, R> {
+  char pad[stage_stride(sizeof(MStageData<D, R>)) - sizeof(MStageData<D, R>)];
+};
 
 template <int D, typename R>
 constexpr size_t musl_crd_bytes() {
@@ -1810,15 +1754,23 @@ template <int D, typename R>
 constexpr size_t musl_patch_bytes() {
   return align16(sizeof(R) * NodePatch<D, true, R>::SIZE) + align16(sizeof(R) * D * Tiling<D>::NODES);
 }
+// a warp stages 32 / kMuslParts particles at a time
+template <int D, typename R>
+__host__ __device__ constexpr size_t musl_group_bytes() {
+  return ScatterShape<D, 1>::LPP / kMuslParts * sizeof(MStage<D, R>) + kGroupPad;
+}
 template <int D, typename R>
 constexpr size_t musl_smem_bytes(int threads) {
-  return musl_crd_bytes<D, R>() + musl_patch_bytes<D, R>() + stage_bytes<MStage<D, R>, MTR_MUSL_CHUNK_DIV>(threads);
+  return musl_crd_bytes<D, R>() + musl_patch_bytes<D, R>() +
+         ScatterShape<D, 1>::GR * musl_group_bytes<D, R>() * (size_t)(threads / 32);
 }
 
-template <int D, int DEG, typename R, int XS = 1>
+template <int D, int DEG, typename R>
 __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid, const uint32_t nblk) {
   using TL = Tiling<D>;
-  constexpr int PN = TL::PN, NODES = TL::NODES;
+  using SS = ScatterShape<D, 1>;
+  constexpr int PN = TL::PN, NODES = TL::NODES, Z = D - 1;
+  constexpr int LPP = SS::LPP, GR = SS::GR, CH = LPP / kMuslParts;
   StepHeader* H = A.H;
   if (step_inactive(H)) return;
   const uint32_t t = bid;
@@ -1832,7 +1784,6 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
   R* pv = reinterpret_cast<R*>(smem_raw + musl_crd_bytes<D, R>());  // node v, flip
   R(*vsum)[NODES] = reinterpret_cast<R(*)[NODES]>(
       smem_raw + musl_crd_bytes<D, R>() + align16(sizeof(R) * NodePatch<D, true, R>::SIZE));  // [D][NODES]
-  MStage<D, R>* st = reinterpret_cast<MStage<D, R>*>(smem_raw + musl_crd_bytes<D, R>() + musl_patch_bytes<D, R>());
   int n0[3];
   load_tile_setup<D>(A, H, t, n0, crd);
   double vref[3];
@@ -1840,95 +1791,49 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
   const double fr = P.flip_ratio;
   load_patch<D, true, R>(A, H, n0, A.nv, vref, A.nflip, fr >= -1, pv);
   for (int i = threadIdx.x; i < D * NODES; i += blockDim.x) (&vsum[0][0])[i] = R(0.0);
+  __shared__ uint32_t ustart[kUnits + 1];  // first particle of each unit
+  if (threadIdx.x <= kUnits) ustart[threadIdx.x] = A.cell_start[t * 64u + 4u * threadIdx.x];
   __syncthreads();
   const uint32_t Np = A.Np;
   const double dt = H->dt, ioh = P.one_over_dx;
-  const R apicD = (R)P.apicDinverse;
+  const R dx = (R)P.dx, apicD = (R)P.apicDinverse;
   const bool apic = fr < 0;
-  const int lane = threadIdx.x & 31;
-  constexpr int COLS = D == 3 ? 16 : 4, LPP = COLS * XS, HN = 4 / XS;  // as in k_p2g_w
-  const int q = lane % LPP;
-  const int iy = D == 3 ? ((q % COLS) >> 2) : q % COLS;
-  const int iz = D == 3 ? ((q % COLS) & 3) : 0;
-  const int h0 = (q / COLS) * HN;
-  // a staged particle after its gather: velocity blend, position update,
-  // outputs and the re-scatter stencil; returns the packed stencil base
-  // (-1: none)
-  auto finish = [&](MStage<D, R>& S, uint32_t s, uint32_t pid, const double (&xp)[3], const double (&vp)[3],
-                    const double (&pic)[3], const R (&flp)[3], const R (&Bp)[D][D], bool ok) -> int {
-    int packed = -1;
-    double xn[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-    for (int a = 0; a < D; ++a) {
-      const double vn = blend_v(fr, vp[a], (double)flp[a], pic[a]);
-      if constexpr (kFP64<R>) S.x[a] = xp[a];
-      S.v[a] = (R)vn;
-      xn[a] = xp[a] + dt * pic[a];  // positionUpdate: x + dt pic
-      A.out.v[(size_t)a * Np + s] = (R)vn;
-    }
-    wrap_and_teleport(P, xn);
-#pragma unroll
-    for (int a = 0; a < D; ++a) A.out.x[(size_t)a * Np + s] = xn[a];
-#pragma unroll
-    for (int r = 0; r < D; ++r)
-#pragma unroll
-      for (int c = 0; c < D; ++c) {
-        const R b = apic ? Bp[r][c] : R(0.0);
-        A.out.B[(size_t)(r * D + c) * Np + s] = b;
-        S.B[r * D + c] = MTR_SCATTER_PRESCALE ? apicD * b : b;
-      }
-    A.out.id[s] = pid;
-    if (P.store_pic_flip) {
-#pragma unroll
-      for (int a = 0; a < D; ++a) {
-        A.pic[(size_t)a * Np + s] = (R)pic[a];
-        A.flip[(size_t)a * Np + s] = (fr >= -1) ? flp[a] : R(0.0);
-      }
-    }
-    // re-scatter stencil, base clamped at zero like P2G (musl.cpp:35-40)
-    int lbs[3];
-    if (ok && local_base<D>(H, xp, ioh, n0, true, lbs)) {
-#pragma unroll
-      for (int a = 0; a < D; ++a)
-#pragma unroll
-        for (int o = 0; o < 4; ++o) {
-          const double c = crd[a][lbs[a] + o];
-          S.w[a * 4 + o] = bspline_N<DEG>((R)((xp[a] - c) * ioh));
-          if constexpr (!kFP64<R>) S.pd[a * 4 + o] = (R)(c - xp[a]);
-        }
-      packed = lbs[0] | (lbs[1] << 4) | (lbs[2] << 8);
-    } else if (ok) {
-      raise_status(H, MTR_STATUS_STENCIL_OOB, pid);
-    }
-    return packed;
-  };
-  // consecutive particles per lane group, as in k_p2g_w
-  static_assert(LPP % MTR_MUSL_CHUNK_DIV == 0, "chunk divisor must divide the lanes per particle");
-  constexpr int PPG = LPP / MTR_MUSL_CHUNK_DIV;
-  const int chunk = (int)blockDim.x / MTR_MUSL_CHUNK_DIV;
-  const int kbeg = ((int)threadIdx.x / LPP) * PPG, kend = kbeg + PPG;
-  for (uint32_t c0 = pb; c0 < pe; c0 += chunk) {
-    if ((int)threadIdx.x < chunk) {  // phase 1
-      const uint32_t s = c0 + threadIdx.x;
-      MStage<D, R>& S = st[threadIdx.x];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int grp = lane / LPP, q = lane % LPP;
+  const int ix = D == 3 ? q >> 2 : q, iy = D == 3 ? q & 3 : 0;  // this lane's column
+  MStage<D, R>* st = reinterpret_cast<MStage<D, R>*>(smem_raw + musl_crd_bytes<D, R>() + musl_patch_bytes<D, R>() +
+                                                     (size_t)(warp * GR + grp) * musl_group_bytes<D, R>());
+  // the gather's x and y factors use the warp's stage, which phase 1 does not
+  R* xfac = reinterpret_cast<R*>(smem_raw + musl_crd_bytes<D, R>() + musl_patch_bytes<D, R>() +
+                                 (size_t)warp * GR * musl_group_bytes<D, R>()) + lane;
+  static_assert(8 * (D - 1) * 32 * sizeof(R) <= GR * musl_group_bytes<D, R>(), "x and y factors must fit the warp's stage");
+  for (int u0 = warp * GR; u0 < kUnits; u0 += nwarps * GR) {
+    const uint32_t ub = ustart[u0 + grp], count = ustart[u0 + grp + 1] - ub;
+    const uint32_t most = GR == 1 ? count : __reduce_max_sync(0xffffffffu, count);
+    for (uint32_t k0 = 0; k0 < most; k0 += LPP) {
+      // phase 1
+      __syncwarp();  // the stage has been read
+      const bool has = k0 + q < count;
       int packed = -1;
-      if (s < pe) {
-        const uint32_t j = perm[s];
-        double xp[3] = {0, 0, 0}, vp[3] = {0, 0, 0};
+      R vs[D], Bs[D][D];
+      double td[3] = {0.0, 0.0, 0.0};
+      if (has) {
+        const uint32_t s = ub + k0 + q, j = perm[s];
+        double xp[3] = {0, 0, 0};
 #pragma unroll
-        for (int a = 0; a < D; ++a) {
-          xp[a] = A.in.x[(size_t)a * Np + j];
-          vp[a] = A.in.v[(size_t)a * Np + j];
-        }
-        const uint32_t pid = A.in.id[j];
+        for (int a = 0; a < D; ++a) xp[a] = A.in.x[(size_t)a * Np + j];
         double pic[3];
         R flp[3], Bp[D][D], gv[D][D];
         int lb[3];
-        const bool ok = local_base<D>(H, xp, ioh, n0, false, lb);
-        if (ok) {
-          gather_patch<D, DEG, false, R>(pv, crd, lb, xp, ioh, vref, pic, Bp, flp, gv, apic, fr >= -1);
+        if (local_base<D>(H, xp, ioh, n0, false, lb)) {
+          gather_patch<D, DEG, false, 32, 4, R>(pv, crd, lb, xp, ioh, dx, xfac, vref, pic, Bp, flp, gv, apic, fr >= -1);
+          // the re-scatter's base, clamped at zero like P2G's (musl.cpp:35-40), is
+          // the same one: the gather takes no particle left of the first node
+          packed = lb[0] | (lb[1] << 4) | (lb[2] << 8);
+#pragma unroll
+          for (int a = 0; a < D; ++a) td[a] = (xp[a] - crd[a][lb[a] + 1]) * ioh;
         } else {
-          raise_status(H, MTR_STATUS_STENCIL_OOB, pid);
+          raise_status(H, MTR_STATUS_STENCIL_OOB, A.in.id[j]);
 #pragma unroll
           for (int a = 0; a < 3; ++a) {
             pic[a] = 0.0;
@@ -1939,77 +1844,138 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
 #pragma unroll
             for (int c = 0; c < D; ++c) Bp[r][c] = R(0.0);
         }
-        packed = finish(S, s, pid, xp, vp, pic, flp, Bp, ok);
-      }
-      S.lb = packed;
-    }
-    __syncthreads();
-    {  // phase 2
-      R acc[HN][D];
-#pragma unroll
-      for (int h = 0; h < HN; ++h)
-#pragma unroll
-        for (int a = 0; a < D; ++a) acc[h][a] = R(0.0);
-      int cur = -1;
-      auto flush = [&]() {
-        const int lbx = cur & 15, lby = (cur >> 4) & 15, lbz = cur >> 8;
-#pragma unroll
-        for (int hh = 0; hh < HN; ++hh) {
-          const int h = h0 + hh;
-          const int node = D == 3 ? ((lbx + h) * PN + (lby + iy)) * PN + (lbz + iz) : (lbx + h) * PN + (lby + iy);
-#pragma unroll
-          for (int a = 0; a < D; ++a) {
-            if (acc[hh][a] != R(0.0)) atomicAdd(&vsum[a][node], acc[hh][a]);
-            acc[hh][a] = R(0.0);
-          }
-        }
-      };
-      for (int k = kbeg; k < kend; ++k) {
-        const MStage<D, R>& S = st[k];
-        const int lbp = S.lb;
-        if (lbp < 0) continue;
-        if (lbp != cur) {
-          if (cur >= 0) flush();
-          cur = lbp;
-        }
-        const int lbx = lbp & 15, lby = (lbp >> 4) & 15, lbz = lbp >> 8;
-        const R wyz = D == 3 ? S.w[4 + iy] * S.w[8 + iz] : S.w[4 + iy];
-        const R pdy = stage_pd<D, R>(S, crd, 1, lby, iy);
-        const R pdz = D == 3 ? stage_pd<D, R>(S, crd, D - 1, lbz, iz) : R(0.0);
-        R Tm[D], Sm[D];
+        double xn[3] = {0.0, 0.0, 0.0};
 #pragma unroll
         for (int a = 0; a < D; ++a) {
-          if (apic) {
-            R byz = S.B[a * D + 1] * pdy;
-            if constexpr (D == 3) byz += S.B[a * D + 2] * pdz;
-            Tm[a] = S.v[a] + (MTR_SCATTER_PRESCALE ? byz : apicD * byz);
-            Sm[a] = MTR_SCATTER_PRESCALE ? S.B[a * D] : apicD * S.B[a * D];
-          } else {
-            Tm[a] = S.v[a];
-            Sm[a] = R(0.0);
-          }
+          const double vn = blend_v(fr, (double)A.in.v[(size_t)a * Np + j], (double)flp[a], pic[a]);
+          vs[a] = (R)vn;
+          xn[a] = xp[a] + dt * pic[a];  // positionUpdate: x + dt pic
+          A.out.v[(size_t)a * Np + s] = (R)vn;
         }
+        wrap_and_teleport(P, xn);
 #pragma unroll
-        for (int hh = 0; hh < HN; ++hh) {
-          const int h = h0 + hh;
-          const R weight = S.w[h] * wyz;
-          if constexpr (MTR_SCATTER_SELECT) {
-            const R ws = weight > R(1e-25) ? weight : R(0.0);  // musl.cpp:51 skips weights <= 1e-25
-            const R pdx = stage_pd<D, R>(S, crd, 0, lbx, h);
+        for (int a = 0; a < D; ++a) A.out.x[(size_t)a * Np + s] = xn[a];
 #pragma unroll
-            for (int a = 0; a < D; ++a) acc[hh][a] += ws * (Tm[a] + Sm[a] * pdx);
-          } else {
-            if (!(weight > R(1e-25))) continue;
-            const R pdx = stage_pd<D, R>(S, crd, 0, lbx, h);
+        for (int r = 0; r < D; ++r)
 #pragma unroll
-            for (int a = 0; a < D; ++a) acc[hh][a] += weight * (Tm[a] + Sm[a] * pdx);
+          for (int c = 0; c < D; ++c) {
+            const R b = apic ? Bp[r][c] : R(0.0);
+            A.out.B[(size_t)(r * D + c) * Np + s] = b;
+            Bs[r][c] = apicD * b;
+          }
+        A.out.id[s] = A.in.id[j];
+        if (P.store_pic_flip) {
+#pragma unroll
+          for (int a = 0; a < D; ++a) {
+            A.pic[(size_t)a * Np + s] = (R)pic[a];
+            A.flip[(size_t)a * Np + s] = (fr >= -1) ? flp[a] : R(0.0);
           }
         }
       }
-      if (cur >= 0) flush();
+      // phase 2; the window starts and ends with the chunk, so that its registers
+      // are free during the gather
+      R acc[4][D];
+#pragma unroll
+      for (int h = 0; h < 4; ++h)
+#pragma unroll
+        for (int c = 0; c < D; ++c) acc[h][c] = R(0.0);
+      int curb = 0, curz = -1;
+      auto advance = [&]() {
+        const int bx = curb & 15, by = curb >> 4;
+        const int node = D == 3 ? ((bx + ix) * PN + (by + iy)) * PN + curz : (bx + ix) * PN + curz;
+#pragma unroll
+        for (int c = 0; c < D; ++c) {
+          if (acc[0][c] != R(0.0)) atomicAdd(&vsum[c][node], acc[0][c]);
+#pragma unroll
+          for (int h = 0; h < 3; ++h) acc[h][c] = acc[h + 1][c];
+          acc[3][c] = R(0.0);
+        }
+        ++curz;
+      };
+#pragma unroll 1
+      for (int part = 0; part < kMuslParts; ++part) {
+        if (k0 + part * CH >= most) break;
+        __syncwarp();  // the last part has been read
+        if (q / CH == part) {
+          MStage<D, R>& S = st[q % CH];
+          if (packed >= 0) {
+            int least = 0;
+#pragma unroll
+            for (int a = 0; a < D; ++a) {
+              R w[4], d[4], o[4];
+              axis_weights<DEG, false, R>(td[a], w, d);
+              axis_offsets<R>(td[a], dx, o);
+#pragma unroll
+              for (int h = 0; h < 4; ++h) {
+                S.w[a][h] = w[h];
+                S.a[a][h] = w[h] * o[h];
+              }
+              least += least_exponent<DEG>(w);
+            }
+#pragma unroll
+            for (int r = 0; r < D; ++r) {
+              S.q[r][0] = vs[r];
+#pragma unroll
+              for (int c = 0; c < D; ++c) S.q[r][1 + c] = Bs[r][c];
+            }
+            S.lb = packed | (least < -82 ? kTinyWeight : 0);
+          } else {
+            S.lb = -1;
+          }
+        }
+        __syncwarp();
+        const uint32_t left = most - k0 - part * CH;
+        const int kend = left < (uint32_t)CH ? (int)left : CH;
+#pragma unroll 1
+        for (int k = 0; k < kend; ++k) {
+          const MStage<D, R>& S = st[k];
+          const int lbp = S.lb;
+          if (lbp < 0) continue;
+          const int base = D == 3 ? lbp & 255 : lbp & 15, bz = (D == 3 ? lbp >> 8 : lbp >> 4) & 15;
+          if (base != curb || bz != curz) {
+            if (curz >= 0) {
+              const int to = base == curb && bz > curz && bz < curz + 4 ? bz : curz + 4;
+              while (curz < to) advance();
+            }
+            curb = base;
+            curz = bz;
+          }
+          R f1[4], f2[4];
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            f1[h] = S.w[Z][h];
+            f2[h] = S.a[Z][h];
+          }
+          R u0 = S.w[0][ix], u1 = S.a[0][ix];
+          [[maybe_unused]] R u2 = R(0.0);
+          if constexpr (D == 3) {
+            const R wy = S.w[1][iy], ay = S.a[1][iy];
+            u2 = u0 * ay;
+            u0 *= wy;
+            u1 *= wy;
+          }
+          if (lbp & kTinyWeight) {  // musl.cpp:51 skips weights <= 1e-25
+#pragma unroll
+            for (int h = 0; h < 4; ++h)
+              if (!(f1[h] * u0 > R(1e-25))) f1[h] = f2[h] = R(0.0);
+          }
+#pragma unroll
+          for (int c = 0; c < D; ++c) {
+            R a1 = u0 * S.q[c][0] + u1 * S.q[c][1];
+            if constexpr (D == 3) a1 += u2 * S.q[c][2];
+            const R b1 = u0 * S.q[c][D];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) acc[h][c] = f2[h] * b1 + (f1[h] * a1 + acc[h][c]);
+          }
+        }
+      }
+      if (curz >= 0) {
+        const int to = curz + 4;
+        while (curz < to) advance();
+      }
     }
-    __syncthreads();
   }
+  __syncthreads();
   const uint32_t cap = A.cap_nodes;
   for (int n = threadIdx.x; n < NODES; n += blockDim.x) {
     uint32_t l;
@@ -2022,10 +1988,10 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
   }
 }
 
-template <int D, int DEG, typename R, int XS = 1>
-__global__ void __launch_bounds__(MTR_MUSL_MAX_THREADS, MTR_MUSL_MIN_BLOCKS)
+template <int D, int DEG, typename R>
+__global__ void __launch_bounds__(MTR_MUSL_BOUNDS)
     k_g2p_musl_w(StepArgsT<R> A, const uint32_t* __restrict__ perm) {
-  g2p_musl_w_body<D, DEG, R, XS>(A, perm, blockIdx.x, gridDim.x);
+  g2p_musl_w_body<D, DEG, R>(A, perm, blockIdx.x, gridDim.x);
 }
 
 // musl.cpp:80-95: v2 /= (m_i / m_p) (zero where m_i == 0)
@@ -2064,6 +2030,7 @@ __device__ __forceinline__ void defgrad_t_body(const StepArgsT<R>& A, const uint
   tile_range(A, t, pb, pe);
   if (pb >= pe) return;
   __shared__ __align__(16) R pv[NodePatch<D, false, R>::SIZE];
+  __shared__ R xfac[8 * (D - 1) * kMaxTileThreads];  // x and y factors of each thread's gather
   __shared__ double crd[3][PN];
   int n0[3];
   load_tile_setup<D>(A, H, t, n0, crd);
@@ -2081,7 +2048,7 @@ __device__ __forceinline__ void defgrad_t_body(const StepArgsT<R>& A, const uint
     R gv[D][D];
     int lb[3];
     if (local_base<D>(H, p.x, ioh, n0, false, lb)) {
-      gather_gradv<D, DEG, R>(pv, crd, lb, p.x, ioh, gv);
+      gather_gradv<D, DEG, kMaxTileThreads, 4, R>(pv, crd, lb, p.x, ioh, (R)A.P->dx, xfac + threadIdx.x, gv);
     } else {
       raise_status(H, MTR_STATUS_STENCIL_OOB, p.id);
 #pragma unroll
@@ -2243,9 +2210,9 @@ __global__ void __launch_bounds__(kSortThreads) kb_sort_rank(BatchView<R> B) {
   if (A) sort_rank_body(*A, b, nb);
 }
 
-template <int D, int DEG, typename R, int XS = 1>
-__global__ void __launch_bounds__(kMaxTileThreads) kb_p2g_w(BatchView<R> B) {
-  batch_tiles(B, [&](const StepArgsT<R>& A, uint32_t b, uint32_t nb) { p2g_w_body<D, DEG, R, XS>(A, A.perm, b, nb); });
+template <int D, int DEG, typename R>
+__global__ void __launch_bounds__(MTR_P2G_BOUNDS) kb_p2g_w(BatchView<R> B) {
+  batch_tiles(B, [&](const StepArgsT<R>& A, uint32_t b, uint32_t nb) { p2g_w_body<D, DEG, R>(A, A.perm, b, nb); });
 }
 
 template <int D, typename R>
@@ -2256,14 +2223,14 @@ __global__ void __launch_bounds__(256) kb_grid(BatchView<R> B) {
 }
 
 template <int D, int DEG, typename R, int PM = -1>
-__global__ void __launch_bounds__(kChunk, MTR_G2P_MIN_BLOCKS) kb_g2p_t(BatchView<R> B) {
+__global__ void __launch_bounds__(kChunk, (g2p_min_blocks<R, PM>())) kb_g2p_t(BatchView<R> B) {
   batch_tiles(B, [&](const StepArgsT<R>& A, uint32_t b, uint32_t nb) { g2p_t_body<D, DEG, R, PM>(A, A.perm, b, nb); });
 }
 
-template <int D, int DEG, typename R, int XS = 1>
-__global__ void __launch_bounds__(MTR_MUSL_MAX_THREADS, MTR_MUSL_MIN_BLOCKS) kb_g2p_musl_w(BatchView<R> B) {
+template <int D, int DEG, typename R>
+__global__ void __launch_bounds__(MTR_MUSL_BOUNDS) kb_g2p_musl_w(BatchView<R> B) {
   batch_tiles(B, [&](const StepArgsT<R>& A, uint32_t b, uint32_t nb) {
-    g2p_musl_w_body<D, DEG, R, XS>(A, A.perm, b, nb);
+    g2p_musl_w_body<D, DEG, R>(A, A.perm, b, nb);
   });
 }
 

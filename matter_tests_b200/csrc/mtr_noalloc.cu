@@ -77,6 +77,13 @@ namespace {
 std::mutex g_setup_mutex;
 void* g_scratch_ptr[kMaxDevices] = {};
 
+template <int D>
+struct NStage {
+  double x[D], v[D], B[D * D], w[D * 4];
+  int lb;
+  int pad;
+};
+
 // The P2G variant: as k_p2g_w, but mass and momentum only (no stress, no
 // friction channel), accumulating into the scratch grid.
 template <int D, int DEG>
@@ -94,7 +101,7 @@ __global__ void __launch_bounds__(kChunk) k_p2g_noalloc(StepArgs A, const uint32
   extern __shared__ double smem[];
   double(*patch)[NODES] = reinterpret_cast<double(*)[NODES]>(smem);
   double(*crd)[PN] = reinterpret_cast<double(*)[PN]>(smem + NCH * NODES);
-  MStage<D>* st = reinterpret_cast<MStage<D>*>(smem + NCH * NODES + 3 * PN);
+  NStage<D>* st = reinterpret_cast<NStage<D>*>(smem + NCH * NODES + 3 * PN);
   int tc[3];
   tile_coords<D>(H, t, tc);
   const int n0[3] = {tc[0] * TB - 1, tc[1] * TB - 1, D == 3 ? tc[2] * TB - 1 : 0};
@@ -118,7 +125,7 @@ __global__ void __launch_bounds__(kChunk) k_p2g_noalloc(StepArgs A, const uint32
   for (uint32_t c0 = pb; c0 < pe; c0 += kChunk) {
     {
       const uint32_t s = c0 + threadIdx.x;
-      MStage<D>& S = st[threadIdx.x];
+      NStage<D>& S = st[threadIdx.x];
       int packed = -1;
       if (s < pe) {
         const uint32_t j = perm[s];
@@ -165,7 +172,7 @@ __global__ void __launch_bounds__(kChunk) k_p2g_noalloc(StepArgs A, const uint32
         }
       };
       for (int k = kbeg; k < kend; ++k) {
-        const MStage<D>& S = st[k];
+        const NStage<D>& S = st[k];
         const int lbp = S.lb;
         if (lbp < 0) continue;
         if (lbp != cur) {
@@ -261,7 +268,7 @@ __global__ void __launch_bounds__(kSortThreads) k_noalloc_keys(StepCommon A) {
 
 template <int D>
 constexpr size_t noalloc_smem_bytes() {
-  return sizeof(double) * ((1 + D) * Tiling<D>::NODES + 3 * Tiling<D>::PN) + sizeof(MStage<D>) * kChunk;
+  return sizeof(double) * ((1 + D) * Tiling<D>::NODES + 3 * Tiling<D>::PN) + sizeof(NStage<D>) * kChunk;
 }
 
 // Writes the grid description and the few constants the kernels read into
