@@ -515,8 +515,10 @@ void launch_g2p(int spm, uint32_t blocks, int threads, cudaStream_t st, const St
   k_g2p_t<D, DEG, R><<<blocks, threads, 0, st>>>(A, perm);
 }
 
+// `follows`: the step enqueued just before left its commit to this one;
+// `commit`: this step commits itself (k_tail).
 template <int D, int DEG, typename R>
-int enqueue_step_t(mtr_ctx* c, int parity) {
+int enqueue_step_t(mtr_ctx* c, int parity, bool follows, bool commit) {
   cudaStream_t st = c->stream;
   StepArgsT<R> A = make_args<R>(c, parity);
   int n = 0;
@@ -524,7 +526,10 @@ int enqueue_step_t(mtr_ctx* c, int parity) {
   k_bbox<D, R><<<c->npartials, 256, 0, st>>>(A);
   ++n;
   mark(c, "k_bbox");
-  k_header<D><<<1, 256, 0, st>>>(A);
+  if (follows)
+    k_header<D, true><<<1, 256, 0, st>>>(A);
+  else
+    k_header<D><<<1, 256, 0, st>>>(A);
   ++n;
   mark(c, "k_header");
   // sort
@@ -571,7 +576,7 @@ int enqueue_step_t(mtr_ctx* c, int parity) {
     ++n;
     mark(c, "k_g2p");
   }
-  if (!c->trial) {
+  if (!c->trial && commit) {
     k_tail<D><<<1, 32, 0, st>>>(A, 1 - parity);
     ++n;
     mark(c, "k_tail");
@@ -581,13 +586,17 @@ int enqueue_step_t(mtr_ctx* c, int parity) {
 }
 
 template <typename R>
-int enqueue_step_r(mtr_ctx* c, int parity) {
-  if (c->dim == 3) return c->deg == 3 ? enqueue_step_t<3, 3, R>(c, parity) : enqueue_step_t<3, 2, R>(c, parity);
-  return c->deg == 3 ? enqueue_step_t<2, 3, R>(c, parity) : enqueue_step_t<2, 2, R>(c, parity);
+int enqueue_step_r(mtr_ctx* c, int parity, bool follows, bool commit) {
+  if (c->dim == 3)
+    return c->deg == 3 ? enqueue_step_t<3, 3, R>(c, parity, follows, commit)
+                       : enqueue_step_t<3, 2, R>(c, parity, follows, commit);
+  return c->deg == 3 ? enqueue_step_t<2, 3, R>(c, parity, follows, commit)
+                     : enqueue_step_t<2, 2, R>(c, parity, follows, commit);
 }
 
-int enqueue_step(mtr_ctx* c, int parity) {
-  return c->fp32 ? enqueue_step_r<float>(c, parity) : enqueue_step_r<double>(c, parity);
+int enqueue_step(mtr_ctx* c, int parity, bool follows = false, bool commit = true) {
+  return c->fp32 ? enqueue_step_r<float>(c, parity, follows, commit)
+                 : enqueue_step_r<double>(c, parity, follows, commit);
 }
 
 void build_graphs(mtr_ctx* c) {
@@ -598,7 +607,7 @@ void build_graphs(mtr_ctx* c) {
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     int n = 0;
     try {
-      for (int s = 0; s < kGraphSteps; ++s) n += enqueue_step(c, (p0 + s) & 1);
+      for (int s = 0; s < kGraphSteps; ++s) n += enqueue_step(c, (p0 + s) & 1, s > 0, s + 1 == kGraphSteps);
     } catch (...) {
       cudaStreamEndCapture(c->stream, &g);
       if (g) cudaGraphDestroy(g);
@@ -1216,7 +1225,7 @@ int mtr_upload(mtr_ctx* c, const double* x, const double* v, const double* F, co
       c->perm_rank = dalloc<uint32_t>(Np);
       c->perm_tmp = dalloc<uint32_t>(Np);
       c->big_cells = dalloc<uint32_t>(Np / kBigCell + 1);
-      c->npartials = (int)std::min<uint32_t>((Np + 255) / 256, 148 * 8);
+      c->npartials = (int)std::min<uint32_t>((Np + 256 * kBBoxItems - 1) / (256 * kBBoxItems), 148 * 8);
       c->partials = dalloc<BBoxPartial>(c->npartials);
       c->staging = dalloc<double>((size_t)Np * std::max<int>(dd, (int)MTR_NUM_SCALARS));
     }
@@ -1358,13 +1367,15 @@ int mtr_step(mtr_ctx* c, int nsteps) {
       if (c->use_graphs && (!c->graph[0] || !c->graph[1])) build_graphs(c);
       int parity = c->host_parity;
       int todo = remaining;
+      bool follows = false;  // the step before was enqueued directly and left its commit
       while (todo > 0) {
         if (c->use_graphs && todo >= kGraphSteps) {
           CK(cudaGraphLaunch(c->graph[parity], c->stream));
           launches += (int64_t)c->launches_per_step * kGraphSteps;
           todo -= kGraphSteps;  // kGraphSteps is even: parity unchanged
         } else {
-          launches += enqueue_step(c, parity);
+          launches += enqueue_step(c, parity, follows, todo == 1);
+          follows = true;
           parity ^= 1;
           todo -= 1;
         }

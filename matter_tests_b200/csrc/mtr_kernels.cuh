@@ -150,24 +150,41 @@ __device__ __forceinline__ void block_count(unsigned n, unsigned long long* dst)
 // ---------------------------------------------------------------------------
 // 1. bbox / vmax / sum v partials
 // ---------------------------------------------------------------------------
+// Bound: the latency of its loads.  A thread takes kBBoxItems particles and
+// issues all their loads before it uses one.
+constexpr int kBBoxItems = 4;
 template <int D, typename R>
 __device__ __forceinline__ void bbox_body(const StepArgsT<R>& A, const uint32_t bid, const uint32_t nblk) {
   if (step_inactive(A.H)) return;
   double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300}, v2 = 0.0, vs[3] = {0.0, 0.0, 0.0};
-#pragma unroll 4
-  for (uint32_t i = bid * blockDim.x + threadIdx.x; i < A.Np; i += nblk * blockDim.x) {
-    double vv[3];
+  for (uint32_t i0 = bid * (256 * kBBoxItems) + threadIdx.x; i0 < A.Np; i0 += nblk * (256 * kBBoxItems)) {
+    double x[kBBoxItems][D];
+    R v[kBBoxItems][D];
 #pragma unroll
-    for (int a = 0; a < D; ++a) {
-      double xa = A.in.x[(size_t)a * A.Np + i];
-      mn[a] = fmin(mn[a], xa);
-      mx[a] = fmax(mx[a], xa);
-      vv[a] = A.in.v[(size_t)a * A.Np + i];
-      vs[a] += vv[a];
+    for (int k = 0; k < kBBoxItems; ++k) {
+      // past the end: the first particle again, counted once below
+      const uint32_t i = i0 + k * 256 < A.Np ? i0 + k * 256 : i0;
+#pragma unroll
+      for (int a = 0; a < D; ++a) {
+        x[k][a] = A.in.x[(size_t)a * A.Np + i];
+        v[k][a] = A.in.v[(size_t)a * A.Np + i];
+      }
     }
-    double s = __dadd_rn(__dmul_rn(vv[0], vv[0]), __dmul_rn(vv[1], vv[1]));
-    if constexpr (D == 3) s = __dadd_rn(s, __dmul_rn(vv[2], vv[2]));
-    v2 = fmax(v2, s);
+#pragma unroll
+    for (int k = 0; k < kBBoxItems; ++k) {
+      const bool in = i0 + k * 256 < A.Np;
+      double vv[3];
+#pragma unroll
+      for (int a = 0; a < D; ++a) {
+        mn[a] = fmin(mn[a], x[k][a]);
+        mx[a] = fmax(mx[a], x[k][a]);
+        vv[a] = v[k][a];
+        vs[a] += in ? vv[a] : 0.0;
+      }
+      double s = __dadd_rn(__dmul_rn(vv[0], vv[0]), __dmul_rn(vv[1], vv[1]));
+      if constexpr (D == 3) s = __dadd_rn(s, __dmul_rn(vv[2], vv[2]));
+      v2 = fmax(v2, s);
+    }
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
@@ -214,13 +231,41 @@ __global__ void __launch_bounds__(256) k_bbox(StepArgsT<R> A) {
 // ---------------------------------------------------------------------------
 // 2. step header: dt (update_dt.cpp:5-66) and grid (remesh.cpp:38-311)
 // ---------------------------------------------------------------------------
+// value, value + dx, (value + dx) + dx, ... up to stop, each sum rounded as in
+// the serial loop it restates, by one warp: within a binade the increment is a
+// constant, so the lanes guess 32 values at once and keep the leading ones that
+// each follow from the one before by the rounded addition.  Returns the count,
+// exact up to kMaxAxisNodes so that the host can size a regrowth in one go; the
+// bound also ends the loop for non-finite extents.
+// The serial loop's addition, test and store took 25 cycles a node; with the
+// commit of the step before in the same kernel, us per step: 211,777 particles
+// on a 2D grid of 450 x 230 nodes 100 -> 86, 51,200 in 2D 69 -> 65.
+__device__ __forceinline__ uint32_t arange_axis(double value, double stop, double dx, uint32_t cap, double* ax) {
+  const int lane = threadIdx.x & 31;
+  if (!isfinite(value)) return value < stop ? kMaxAxisNodes : 0u;
+  uint32_t n = 0;
+  for (;;) {
+    const double d = __dsub_rn(__dadd_rn(value, dx), value);
+    const double guess = lane == 0 ? value : __fma_rn((double)lane, d, value);
+    const double before = __shfl_up_sync(0xffffffffu, guess, 1);
+    const unsigned good = __ballot_sync(0xffffffffu, lane == 0 || __dadd_rn(before, dx) == guess);
+    const int len = good == 0xffffffffu ? 32 : __ffs(~good) - 1;
+    const unsigned in = __ballot_sync(0xffffffffu, lane < len && guess < stop && n + lane < kMaxAxisNodes);
+    const int cnt = in == 0xffffffffu ? 32 : __ffs(~in) - 1;
+    if (lane < cnt && n + lane < cap) ax[n + lane] = guess;
+    n += (uint32_t)cnt;
+    if (cnt < len) return n;
+    value = __dadd_rn(__shfl_sync(0xffffffffu, guess, len - 1), dx);
+  }
+}
+
 template <int D>
 __device__ __forceinline__ void header_body(const StepCommon& A) {
   StepHeader* H = A.H;
   const DevParams& P = *A.P;
   if (step_inactive(H)) return;
-  // the block (blockDim.x a multiple of 32, at most 256) reduces the bbox
-  // partials; warp 0 then does the rest
+  // the block (256 threads) reduces the bbox partials; thread 0 then does the
+  // step's scalars and one warp per axis the grid coordinates
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300}, v2 = 0.0, vs[3] = {0.0, 0.0, 0.0};
   for (int b = threadIdx.x; b < A.npartials; b += blockDim.x) {
@@ -255,8 +300,7 @@ __device__ __forceinline__ void header_body(const StepCommon& A) {
       wred[wid].v2 = v2;
     }
     __syncthreads();
-    if (wid != 0) return;
-    for (int w = 1; w < nw; ++w) {
+    for (int w = 1; w < nw && wid == 0; ++w) {
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         mn[a] = fmin(mn[a], wred[w].mn[a]);
@@ -268,7 +312,7 @@ __device__ __forceinline__ void header_body(const StepCommon& A) {
   }
   __shared__ double s_low[3], s_high[3], s_stop[3];
   __shared__ int s_ok;
-  if (lane == 0) {
+  if (threadIdx.x == 0) {
     H->nbig = 0;
     // balances of this step (read back by mtr_balance)
     H->grid_mass = 0.0;
@@ -352,26 +396,20 @@ __device__ __forceinline__ void header_body(const StepCommon& A) {
     }
     s_ok = 1;
   }
-  __syncwarp();
-  // arange (tools.hpp:291-296): one lane per axis accumulates value += step
-  if (lane < D) {
-    const double dx = P.dx;
-    double* ax = lane == 0 ? A.gx : (lane == 1 ? A.gy : A.gz);
-    const uint32_t cap = A.cap_axis[lane];
-    const double stop = s_stop[lane];
-    uint32_t n = 0;
-    // counted exactly up to kMaxAxisNodes so the host can size the regrowth in
-    // one go; the bound also ends the loop for non-finite extents
-    for (double value = s_low[lane]; value < stop && n < kMaxAxisNodes; value = __dadd_rn(value, dx)) {
-      if (n < cap) ax[n] = value;
-      ++n;
+  __syncthreads();
+  // arange (tools.hpp:291-296): one warp per axis
+  if (wid < D) {
+    double* ax = wid == 0 ? A.gx : (wid == 1 ? A.gy : A.gz);
+    const uint32_t cap = A.cap_axis[wid];
+    const uint32_t n = arange_axis(s_low[wid], s_stop[wid], P.dx, cap, ax);
+    if (lane == 0) {
+      H->N[wid] = n;
+      H->org[wid] = s_low[wid];
+      if (n > cap || n < 4 || n >= kMaxAxisNodes) atomicExch(&s_ok, 0);
     }
-    H->N[lane] = n;
-    H->org[lane] = s_low[lane];
-    if (n > cap || n < 4 || n >= kMaxAxisNodes) atomicExch(&s_ok, 0);
   }
-  __syncwarp();
-  if (lane == 0) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
     if (D == 2) {
       H->N[2] = 1;
       H->org[2] = 0.0;
@@ -392,7 +430,16 @@ __device__ __forceinline__ void header_body(const StepCommon& A) {
 }
 
 template <int D>
+__device__ __forceinline__ void tail_body(const StepCommon& A, int out_parity);
+
+// AFTER_TAIL: commits the step before first (its k_tail), for steps enqueued
+// one behind the other: one launch less per step
+template <int D, bool AFTER_TAIL = false>
 __global__ void __launch_bounds__(256) k_header(StepCommon A) {
+  if constexpr (AFTER_TAIL) {
+    tail_body<D>(A, 1 - A.out_parity);  // the step before wrote what this one reads
+    __syncthreads();
+  }
   header_body<D>(A);
 }
 
@@ -411,7 +458,11 @@ __global__ void __launch_bounds__(256) k_header(StepCommon A) {
 // same keys needs three launches per 8-bit digit (9 for the 18-bit keys of the
 // 1M-particle collapse) and a pass over the sorted keys for the tile ranges,
 // which here are cell_start itself.
-// @MEASURED_SORT@
+// Measured on a B200, per step: the radix sort with its memsets and tile ranges
+// 11-16 launches and about 80 us at 1,024,000 particles; this one 4 launches,
+// 49 us (CUDA events around every launch, 4 us each of which is the event).
+// Whole steps: 5k particles in 2D 122 -> 100 us, 51,200 in 2D 138 -> 111 us,
+// 150k in 3D 250 -> 210 us, 1,024,000 in 3D FP64 1123 -> 1089 us.
 // A cell's ranking is quadratic in its particles (about 8 in 3D), which up to
 // kBigCell of them costs less than another launch; larger cells are ordered by
 // a whole block that walks the keys once.
@@ -724,7 +775,12 @@ __device__ __forceinline__ bool patch_node(const StepHeader* H, const int (&n0)[
 // against 0.33 on the 1M collapse).
 //
 // Bound: FP64 issue and shared-memory loads of the factors.
-// @MEASURED_P2G@
+// In the sum phase the shared-memory pipe is 73% busy in FP64 (32 wavefronts a
+// particle, most of them 16-byte loads of the factors; ncu).  ms per launch:
+// 1,024,000 particles, cubic, FP64 0.403 -> 0.291, mixed 0.242 -> 0.191; 2M
+// quadratic mixed 0.465 -> 0.351; 51,200 in 2D FP64 0.062 -> 0.024.
+// Tried: holding the next chunk's particles in registers while one is summed
+// (spills, 0.35 -> 0.52), a third register bound (80 registers, 0.45).
 // ---------------------------------------------------------------------------
 constexpr int kChunk = 128;  // default block size of the tile kernels
 // Largest block of the tile kernels.  The scatter kernels stage one particle
@@ -1731,7 +1787,9 @@ __global__ void __launch_bounds__(kChunk, (g2p_min_blocks<R, PM>())) k_g2p_t(Ste
 // stencil columns): the particles are staged in kMuslParts parts (half of the
 // shared memory, so more blocks per SM) and v_p + B D^-1 (x_i - x_p) is summed
 // in the sliding register windows of P2G, one lane per column.
-// @MEASURED_MUSL@
+// Measured, ms per launch at 1,024,000 particles, cubic: FP64 0.393 -> 0.363,
+// mixed 0.258 -> 0.230.  Timing copies without one part each: the gather takes
+// about 80 us of the FP64 launch, the staging and sums 176, the shared adds 25.
 // ---------------------------------------------------------------------------
 constexpr int kMuslParts = 2;
 
