@@ -143,9 +143,10 @@ struct mtr_ctx {
   // storage type of particle and grid state: double (MTR_PREC_FP64) or float (MTR_PREC_MIXED)
   bool fp32 = false;
   size_t rsize = sizeof(double);
-  // particle buffers (two sets, positions FP64, the rest of type R) and their backing allocations
+  // particle buffers (two sets, positions FP64, the rest of type R); they and the
+  // sort's and copies' arrays lie in one allocation
   PBufT<void> buf[2]{};
-  std::vector<void*> pallocs;
+  unsigned char* arena = nullptr;
   void *pic = nullptr, *flip = nullptr;
   // grid (axes FP64, node channels of type R)
   uint32_t cap_axis[3] = {0, 0, 0};
@@ -279,11 +280,19 @@ HostStage& host_stage(int device) {
   return S;
 }
 
-// bytes host -> device on the context's stream; returns when the copy is done
+// Waits for the stream at the end of a scope, also when a call throws: nothing
+// reads or writes the caller's memory after the entry point has returned.
+struct Drain {
+  cudaStream_t st;
+  ~Drain() { cudaStreamSynchronize(st); }
+};
+
+// bytes host -> device on the context's stream, ordered behind the work queued on
+// it.  Pinned memory is read until the caller synchronises the stream; pageable
+// memory has been read (into the staging chunks) on return.
 void copy_to_device(mtr_ctx* c, void* dst, const void* host, size_t bytes) {
   if (is_pinned(host)) {
     CK(cudaMemcpyAsync(dst, host, bytes, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
     return;
   }
   HostStage& S = g_stage[c->device < 64 && c->device >= 0 ? c->device : 0];
@@ -295,17 +304,16 @@ void copy_to_device(mtr_ctx* c, void* dst, const void* host, size_t bytes) {
     CK(cudaEventSynchronize(S.done[k]));  // the chunk's previous DMA has finished
     std::memcpy(S.buf[k], (const char*)host + off, n);
     CK(cudaMemcpyAsync((char*)dst + off, S.buf[k], n, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaEventRecord(S.done[k], c->stream));
+    CK(cudaEventRecord(S.done[k], c->stream));  // the chunk's next user waits for it
   }
-  CK(cudaStreamSynchronize(c->stream));
 }
 
 // bytes device -> host on the context's stream (work already queued on it
-// comes first); returns when the data is in host memory
+// comes first).  Pinned memory is written by the time the caller has
+// synchronised the stream, pageable memory on return.
 void copy_to_host(mtr_ctx* c, void* host, const void* src, size_t bytes) {
   if (is_pinned(host)) {
     CK(cudaMemcpyAsync(host, src, bytes, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
     return;
   }
   HostStage& S = g_stage[c->device < 64 && c->device >= 0 ? c->device : 0];
@@ -314,6 +322,7 @@ void copy_to_host(mtr_ctx* c, void* host, const void* src, size_t bytes) {
   const size_t nchunks = (bytes + kStageChunk - 1) / kStageChunk;
   auto issue = [&](size_t j) {
     const size_t off = j * kStageChunk, n = std::min(kStageChunk, bytes - off);
+    CK(cudaEventSynchronize(S.done[j & 1]));  // an upload's DMA may still read the chunk
     CK(cudaMemcpyAsync(S.buf[j & 1], (const char*)src + off, n, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaEventRecord(S.done[j & 1], c->stream));
   };
@@ -754,8 +763,9 @@ void derive_constants(mtr_ctx* c) {  // simulation.cpp:94-136
 }
 
 // The first step's grid extents, as remeshFixedInit(2,2,2) will compute them
-// (remesh.cpp:38-182), to size the initial grid allocation.
-void grid_extent(const mtr_params& p, uint32_t Np, const double* x, uint32_t want[3]) {
+// (remesh.cpp:38-182), to size the initial grid allocation; lo and hi are the
+// least and largest coordinate per axis.
+void grid_extent(const mtr_params& p, const double* lo, const double* hi, uint32_t want[3]) {
   const int d = p.dim;
   const double dx = p.dx;
   for (int a = 0; a < 3; ++a) want[a] = 1;
@@ -764,12 +774,7 @@ void grid_extent(const mtr_params& p, uint32_t Np, const double* x, uint32_t wan
     return;
   }
   for (int a = 0; a < d; ++a) {
-    double mn = x[a], mx = x[a];
-    for (uint32_t q = 1; q < Np; ++q) {
-      double v = x[(size_t)q * d + a];
-      mn = std::min(mn, v);
-      mx = std::max(mx, v);
-    }
+    double mn = lo[a], mx = hi[a];
     const double g = p.grid_reference_point[a];
     if (p.grid_reference_point[0] < 1e10) {
       mn = std::min(mn, g);
@@ -780,7 +785,20 @@ void grid_extent(const mtr_params& p, uint32_t Np, const double* x, uint32_t wan
   }
 }
 
-void initial_grid_extent(mtr_ctx* c, const double* x, uint32_t want[3]) { grid_extent(c->prm, c->Np, x, want); }
+// The extents of the uploaded positions, from the reductions over the buffer on
+// the device (a scan of the host array took 4 ms for 1.2M particles).
+void initial_grid_extent(mtr_ctx* c, uint32_t want[3]) {
+  std::vector<BBoxPartial> part(c->npartials);
+  CK(cudaMemcpyAsync(part.data(), c->partials, sizeof(BBoxPartial) * part.size(), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  BBoxPartial r = part[0];
+  for (const BBoxPartial& q : part)
+    for (int a = 0; a < c->dim; ++a) {
+      r.mn[a] = std::min(r.mn[a], q.mn[a]);
+      r.mx[a] = std::max(r.mx[a], q.mx[a]);
+    }
+  grid_extent(c->prm, r.mn, r.mx, want);
+}
 
 // SoA device array of the current particle order -> AoS host array in the
 // caller's order (kinds as k_soa_to_aos); f64 marks an FP64 array on either path.
@@ -1187,47 +1205,59 @@ int mtr_upload(mtr_ctx* c, const double* x, const double* v, const double* F, co
   return guarded([&]() -> int {
     if (!c || !x || Np == 0) throw MtrError{MTR_ERR_INVALID, "null context/positions or Np == 0"};
     CK(cudaSetDevice(c->device));
+    const Drain drain{c->stream};
     const int d = c->dim, dd = d * d, ns = nsym(d);
     // A new scene of the same particle count refills the buffers it already
     // has: their addresses, and with them the captured step graphs, stay valid
     // (freeing and allocating them again costs more than the copies).
-    const bool reuse = c->uploaded && c->Np == Np && !c->pallocs.empty();
+    const bool reuse = c->uploaded && c->Np == Np && c->arena;
     c->uploaded = false;
     if (!reuse) {
       free_graphs(c);
-      for (void* p : c->pallocs) dfree(p);
-      c->pallocs.clear();
-      for (void* p : {(void*)c->keys0, (void*)c->perm_rank, (void*)c->perm_tmp, (void*)c->big_cells,
-                      (void*)c->partials, (void*)c->staging})
-        dfree(p);
+      dfree(c->arena);
+      c->arena = nullptr;
       c->Np = Np;
       c->hp.Np = Np;
-      const size_t rs = c->rsize;
-      for (int s = 0; s < 2; ++s) {
-        double* xb = dalloc<double>((size_t)Np * d);  // positions: FP64 on both paths
-        unsigned char* blk = dalloc<unsigned char>(rs * Np * (d + 2 * dd + MTR_NUM_SCALARS + ns));
-        c->pallocs.push_back(xb);
-        c->pallocs.push_back(blk);
-        c->buf[s].x = xb;
-        c->buf[s].v = blk;
-        c->buf[s].F = blk + rs * Np * d;
-        c->buf[s].B = blk + rs * Np * (d + dd);
-        c->buf[s].sc = blk + rs * Np * (d + 2 * dd);
-        c->buf[s].tau = blk + rs * Np * (d + 2 * dd + MTR_NUM_SCALARS);
-        c->buf[s].id = dalloc<uint32_t>(Np);
-        c->pallocs.push_back(c->buf[s].id);
+      c->npartials =
+          (int)std::min<uint32_t>((Np + 256 * kBBoxItems - 1) / (256 * kBBoxItems), 148 * 8);
+      // every array of the particles in one allocation (one driver call, whose
+      // cost varies by milliseconds, instead of fifteen): sizes first, then places
+      const size_t rs = c->rsize, n = Np;
+      size_t total = 0;
+      for (int pass = 0; pass < 2; ++pass) {
+        size_t at = 0;
+        auto take = [&](auto*& p, size_t bytes) {
+          p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(c->arena + (pass ? at : 0));
+          at += (bytes + 255) & ~size_t(255);
+        };
+        for (int s = 0; s < 2; ++s) {
+          PBufT<void>& q = c->buf[s];
+          unsigned char* blk = nullptr;
+          take(q.x, 8 * n * d);  // positions: FP64 on both paths
+          take(blk, rs * n * (d + 2 * dd + MTR_NUM_SCALARS + ns));
+          q.v = blk;
+          q.F = blk + rs * n * d;
+          q.B = blk + rs * n * (d + dd);
+          q.sc = blk + rs * n * (d + 2 * dd);
+          q.tau = blk + rs * n * (d + 2 * dd + MTR_NUM_SCALARS);
+          take(q.id, 4 * n);
+        }
+        unsigned char *pic = nullptr, *flip = nullptr;
+        take(pic, rs * n * d);
+        take(flip, rs * n * d);
+        c->pic = pic;
+        c->flip = flip;
+        take(c->keys0, 4 * n);
+        take(c->perm_rank, 4 * n);
+        take(c->perm_tmp, 4 * n);
+        take(c->big_cells, 4 * (n / kBigCell + 1));
+        take(c->partials, sizeof(BBoxPartial) * c->npartials);
+        take(c->staging, 8 * n * std::max<int>(dd, (int)MTR_NUM_SCALARS));
+        if (pass == 0) {
+          total = at;
+          c->arena = dalloc<unsigned char>(total);
+        }
       }
-      c->pic = dalloc<unsigned char>(rs * Np * d);
-      c->flip = dalloc<unsigned char>(rs * Np * d);
-      c->pallocs.push_back(c->pic);
-      c->pallocs.push_back(c->flip);
-      c->keys0 = dalloc<uint32_t>(Np);
-      c->perm_rank = dalloc<uint32_t>(Np);
-      c->perm_tmp = dalloc<uint32_t>(Np);
-      c->big_cells = dalloc<uint32_t>(Np / kBigCell + 1);
-      c->npartials = (int)std::min<uint32_t>((Np + 256 * kBBoxItems - 1) / (256 * kBBoxItems), 148 * 8);
-      c->partials = dalloc<BBoxPartial>(c->npartials);
-      c->staging = dalloc<double>((size_t)Np * std::max<int>(dd, (int)MTR_NUM_SCALARS));
     }
     c->uploads_reused += reuse ? 1 : 0;
     // state -> buffer 0 (AoS host layout -> SoA)
@@ -1256,7 +1286,6 @@ int mtr_upload(mtr_ctx* c, const double* x, const double* v, const double* F, co
           k_aos_to_soa<2, double><<<blocks, 256, 0, c->stream>>>(Np, src, (double*)dst, kind, eye);
       }
       CK(cudaGetLastError());
-      CK(cudaStreamSynchronize(c->stream));
     };
     put(x, c->buf[0].x, d, 0, false);
     put(v, c->buf[0].v, d, 0, false);
@@ -1273,9 +1302,27 @@ int mtr_upload(mtr_ctx* c, const double* x, const double* v, const double* F, co
       scp = sc.data();
     }
     put(scp, c->buf[0].sc, MTR_NUM_SCALARS, 2, false);
+    // the extents of the positions, by the step's own reduction (under a header
+    // that lets it run)
+    std::memset(c->hH, 0, sizeof(StepHeader));
+    c->hH->stop_frame = 0xffffffffu;
+    c->hH->stop_step = 0xffffffffu;
+    write_header(c);
+    auto bbox = [&](auto dimc, auto zero) {
+      constexpr int D = decltype(dimc)::value;
+      using R = decltype(zero);
+      k_bbox<D, R><<<c->npartials, 256, 0, c->stream>>>(make_args<R>(c, 0));
+    };
+    const std::integral_constant<int, 3> d3;
+    const std::integral_constant<int, 2> d2;
+    if (c->fp32)
+      d == 3 ? bbox(d3, 0.0f) : bbox(d2, 0.0f);
+    else
+      d == 3 ? bbox(d3, 0.0) : bbox(d2, 0.0);
+    CK(cudaGetLastError());
     // initial grid: kept when the new scene's extent fits the grid there is
     uint32_t want[3];
-    initial_grid_extent(c, x, want);
+    initial_grid_extent(c, want);
     bool fits = reuse && c->gx != nullptr;
     for (int a = 0; a < d; ++a) fits = fits && want[a] <= c->cap_axis[a];
     if (fits) {
@@ -1462,6 +1509,7 @@ int mtr_download(mtr_ctx* c, double* x, double* v, double* F, double* B, double*
   return guarded([&]() -> int {
     if (!c || !c->uploaded) throw MtrError{MTR_ERR_STATE, "nothing uploaded"};
     CK(cudaSetDevice(c->device));
+    const Drain drain{c->stream};
     read_header(c);
     const int d = c->dim, dd = d * d;
     const PBufT<void>& b = c->buf[c->hH->cur];
@@ -1470,6 +1518,7 @@ int mtr_download(mtr_ctx* c, double* x, double* v, double* F, double* B, double*
     get_soa(c, F, b.F, b.id, dd, c->fp32 ? 3 : 1, false);
     get_soa(c, B, b.B, b.id, dd, 1, false);
     get_soa(c, scalars, b.sc, b.id, MTR_NUM_SCALARS, 2, false);
+    CK(cudaStreamSynchronize(c->stream));
     return MTR_OK;
   });
 }
@@ -1479,10 +1528,12 @@ int mtr_download_pic_flip(mtr_ctx* c, double* pic, double* flip) {
     if (!c || !c->uploaded) throw MtrError{MTR_ERR_STATE, "nothing uploaded"};
     if (!c->hp.store_pic_flip) throw MtrError{MTR_ERR_STATE, "pic/flip are kept only after mtr_keep_pic_flip(ctx, 1)"};
     CK(cudaSetDevice(c->device));
+    const Drain drain{c->stream};
     read_header(c);
     const PBufT<void>& b = c->buf[c->hH->cur];
     get_soa(c, pic, c->pic, b.id, c->dim, 0, false);
     get_soa(c, flip, c->flip, b.id, c->dim, 0, false);
+    CK(cudaStreamSynchronize(c->stream));
     return MTR_OK;
   });
 }
@@ -1961,8 +2012,15 @@ int mtr_footprint(const mtr_params* params, uint32_t Np, const double* x, uint64
                      + 2 * rs * d * n                                                      // pic, flip
                      + 3 * 4 * n + 4 * (n / kBigCell + 1)                                    // sort
                      + 8 * n * std::max<uint64_t>(dd, MTR_NUM_SCALARS);                       // staging
+    double lo[3], hi[3];
+    for (int a = 0; a < p.dim; ++a) lo[a] = hi[a] = x[a];
+    for (uint32_t q = 1; q < Np; ++q)
+      for (int a = 0; a < p.dim; ++a) {
+        lo[a] = std::min(lo[a], x[(size_t)q * p.dim + a]);
+        hi[a] = std::max(hi[a], x[(size_t)q * p.dim + a]);
+      }
     uint32_t want[3];
-    grid_extent(p, Np, x, want);
+    grid_extent(p, lo, hi, want);
     const uint64_t tb = p.dim == 3 ? 4 : 8;
     uint64_t nodes = 1, tiles = 1, axes = 0;
     for (int a = 0; a < 3; ++a) {
@@ -2339,10 +2397,7 @@ void mtr_ctx_destroy(mtr_ctx* c) {
   }
   free_graphs(c);
   free_grid(c);
-  for (void* p : c->pallocs) dfree(p);
-  for (void* p : {(void*)c->keys0, (void*)c->perm_rank, (void*)c->perm_tmp, (void*)c->big_cells, (void*)c->partials,
-                  (void*)c->staging, (void*)c->dP, (void*)c->dH})
-    dfree(p);
+  for (void* p : {(void*)c->arena, (void*)c->dP, (void*)c->dH}) dfree(p);
   if (c->hH) cudaFreeHost(c->hH);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
