@@ -249,8 +249,6 @@ def kernel_bytes(name, p, Np, Ga, G, wr=8.0):
         return Np * (w8 * d + wr * (dd + 5)) + Ga * w8 * d + Np * wr * (dd + 6 + ns)
     if name == "k_grid":
         return G * (2 * wr * (2 + 2 * d) + w8 * d + wr * (d + 1))
-    if name == "k_musl_norm":
-        return G * (wr + 2 * w8 * d)
     if name == "k_sort_keys":
         return Np * (w8 * d + 8)
     if name == "k_sort_place":

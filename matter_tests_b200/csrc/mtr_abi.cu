@@ -573,12 +573,10 @@ int enqueue_step_t(mtr_ctx* c, int parity, bool follows, bool commit) {
     const size_t sm = musl_smem_bytes<D, R>(tt[kSlotMUSL]);
     k_g2p_musl_w<D, DEG, R><<<c->cap_tiles, tt[kSlotMUSL], sm, st>>>(A, perm);
     mark(c, "k_g2p_musl");
-    k_musl_norm<D, R><<<gblocks, 256, 0, st>>>(A);
-    mark(c, "k_musl_norm");
     launch_defgrad<D, DEG, R>(rm_specialization(D, true, c->prm.plastic_model), c->cap_tiles, tt[kSlotDefgrad], st,
                               A, perm);
     mark(c, "k_defgrad");
-    n += 3;
+    n += 2;
   } else {
     launch_g2p<D, DEG, R>(rm_specialization(D, false, c->prm.plastic_model), c->cap_tiles, tt[kSlotG2P], st, A,
                           perm);
@@ -954,15 +952,13 @@ int enqueue_group_step_t(mtr_batch* b, mtr_batch_group& g, int gi) {
   if (g.musl) {
     launch_tiles<R>(kb_g2p_musl_w<D, DEG, R>, tiles, tt[kSlotMUSL], musl_smem_bytes<D, R>(tt[kSlotMUSL]), st, B);
     b->marks.record(kSlotMark[kSlotMUSL], st, gi);
-    kb_musl_norm<D, R><<<g.total[kBK_NODES], 256, 0, st>>>(B);
-    b->marks.record("kb_musl_norm", st, gi);
     void (*kd)(BatchView<R>) = kb_defgrad_t<D, DEG, R>;
     if constexpr (D == 3) {
       if (g.spm == MTR_PM_DPMUI) kd = kb_defgrad_t<D, DEG, R, MTR_PM_DPMUI>;
     }
     launch_tiles<R>(kd, tiles, tt[kSlotDefgrad], 0, st, B);
     b->marks.record(kSlotMark[kSlotDefgrad], st, gi);
-    n += 3;
+    n += 2;
   } else {
     void (*kg)(BatchView<R>) = kb_g2p_t<D, DEG, R>;
     if constexpr (D == 3) {
@@ -1566,7 +1562,11 @@ int mtr_get_grid(mtr_ctx* c, uint32_t dims[3], double* gx, double* gy, double* g
     if (gy) CK(cudaMemcpy(gy, c->gy, sizeof(double) * H.N[1], cudaMemcpyDeviceToHost));
     if (gz && d == 3) CK(cudaMemcpy(gz, c->gz, sizeof(double) * H.N[2], cudaMemcpyDeviceToHost));
     if (mass) get_nodes(c, mass, c->nmass, G);
-    std::vector<double> tmp((size_t)G);
+    std::vector<double> tmp((size_t)G), mi;
+    if (v && c->prm.use_musl) {
+      mi.resize((size_t)G);
+      get_nodes(c, mi.data(), c->nmass, G);
+    }
     for (int w = 0; w < 2; ++w) {
       double* host = w == 0 ? v : flip;
       if (!host) continue;
@@ -1574,6 +1574,8 @@ int mtr_get_grid(mtr_ctx* c, uint32_t dims[3], double* gx, double* gy, double* g
         if (w == 0) {  // node velocities are FP64 on both paths
           const double* src = (c->prm.use_musl ? c->v2 : c->nv) + (size_t)a * c->cap_nodes;
           CK(cudaMemcpy(tmp.data(), src, sizeof(double) * G, cudaMemcpyDeviceToHost));
+          if (c->prm.use_musl)  // the step keeps the sums (musl.cpp:80-95)
+            for (uint32_t l = 0; l < G; ++l) tmp[l] = mi[l] > 0 ? tmp[l] / (mi[l] / c->prm.particle_mass) : 0.0;
         } else {
           get_nodes(c, tmp.data(), (const unsigned char*)c->nflip + c->rsize * a * c->cap_nodes, G);
         }

@@ -14,7 +14,7 @@
 //   USL:  k_g2p_t gather pic/B/flip/grad v, F update, return mapping, tau, x/v update, coalesced stores
 //                                                              g2p.cpp, deformation_update.cpp, plasticity.cpp,
 //                                                              position_update.cpp
-//   MUSL: k_g2p_musl_w (gather + v blend + re-scatter), k_musl_norm, k_defgrad_t
+//   MUSL: k_g2p_musl_w (gather + v blend + re-scatter), k_defgrad_t
 //                                                              musl.cpp:6-96
 //   k_tail        plate motion, clock, frame and end test     object_plate.hpp:136-162, simulation.cpp:176-200
 //
@@ -86,7 +86,7 @@ struct StepArgsT : StepCommon {
   R* nflip;       // [D][cap_nodes]
   R* nmass;       // [cap_nodes]
   R* nfric;       // [cap_nodes]
-  double* v2;     // [D][cap_nodes] MUSL re-projection accumulator (FP64 on both paths)
+  double* v2;     // [D][cap_nodes] MUSL re-projection accumulator (FP64 on both paths), not divided by m_i / m_p
   PBufT<R> in, out;
   R* pic;   // optional [D][Np] in output order
   R* flip;  // optional [D][Np]
@@ -120,19 +120,23 @@ __device__ __forceinline__ uint32_t node_index(const StepHeader* H, int i, int j
   return ((uint32_t)i * H->N[1] + (uint32_t)j) * H->N[2] + (uint32_t)k;
 }
 
-// sum over the block of a per-thread value, added once to *dst (all threads call)
-__device__ __forceinline__ void block_add(double v, double* dst) {
-  __shared__ double red[32];
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+// sums over the block of N per-thread values, each added once to dst[i] (all
+// threads call): one barrier for all of them
+template <int N>
+__device__ __forceinline__ void block_add(double (&v)[N], double* const (&dst)[N]) {
+  __shared__ double red[N][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], off);
+    if (lane == 0) red[i][warp] = v[i];
+  }
   __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < N) {
     double s = 0.0;
-    for (int w = 0; w < nw; ++w) s += red[w];
-    if (s != 0.0) atomicAdd(dst, s);
+    for (int w = 0; w < nw; ++w) s += red[threadIdx.x][w];
+    if (s != 0.0) atomicAdd(dst[threadIdx.x], s);
   }
 }
 
@@ -1249,7 +1253,7 @@ __device__ __forceinline__ void grid_body(const StepArgsT<R>& A, const uint32_t 
   const DevParams& P = *A.P;
   const uint32_t G = H->G, cap = A.cap_nodes;
   const double dt = H->dt;
-  const double dtpv = dt * P.particle_volume;
+  const double dtpv_mp = dt * P.particle_volume / P.particle_mass;
   double dtg[3];
 #pragma unroll
   for (int a = 0; a < D; ++a) dtg[a] = dt * H->gravity[a];
@@ -1275,20 +1279,21 @@ __device__ __forceinline__ void grid_body(const StepArgsT<R>& A, const uint32_t 
     double v[3] = {0, 0, 0}, vold[3] = {0, 0, 0};
     double fric = 0.0;
     sum_m += mraw;
+    const double rm = 1.0 / mraw;  // one division for the node's six quotients
     if (mraw > 0) {
 #pragma unroll
       for (int a = 0; a < D; ++a) {
         sum_p[a] += pacc[a];
-        v[a] = pacc[a] / mraw;
+        v[a] = pacc[a] * rm;
       }
     }
-    if (P.use_mibf) fric = P.mui0 + fracc / mraw;
+    if (P.use_mibf) fric = P.mui0 + fracc * rm;
     const double mi = mraw * P.particle_mass;
     double fl[3] = {0, 0, 0};
     if (mi > 0) {
 #pragma unroll
       for (int a = 0; a < D; ++a) {
-        double inc = -dtpv * facc[a] / mi + dtg[a];
+        double inc = -dtpv_mp * facc[a] * rm + dtg[a];
         vold[a] = v[a];
         v[a] = vold[a] + inc;
       }
@@ -1311,9 +1316,16 @@ __device__ __forceinline__ void grid_body(const StepArgsT<R>& A, const uint32_t 
 #pragma unroll
     for (int ch = 0; ch < Tiling<D>::NCH; ++ch) A.acc[(size_t)ch * cap + l] = R(0.0);  // ready for the next step
   }
-  block_add(sum_m * P.particle_mass, &H->grid_mass);
+  double sums[1 + D];
+  double* dst[1 + D];
+  sums[0] = sum_m * P.particle_mass;
+  dst[0] = &H->grid_mass;
 #pragma unroll
-  for (int a = 0; a < D; ++a) block_add(sum_p[a] * P.particle_mass, &H->grid_mom[a]);
+  for (int a = 0; a < D; ++a) {
+    sums[1 + a] = sum_p[a] * P.particle_mass;
+    dst[1 + a] = &H->grid_mom[a];
+  }
+  block_add<1 + D>(sums, dst);
 }
 
 template <int D, typename R>
@@ -1431,17 +1443,21 @@ __device__ __forceinline__ void defgrad_and_store(const StepArgsT<R>& A, uint32_
 // Reference velocity of a tile: the FP64 node velocity at the patch node
 // nearest the tile centre (zero outside the grid, and always zero on the FP64
 // path, which gathers the node velocities themselves).
-template <int D, typename R>
+// NORM: src is the MUSL accumulator, divided by m_i / m_p (nmass, mp).
+template <int D, typename R, bool NORM = false>
 __device__ __forceinline__ void tile_vref(const StepCommon& A, const StepHeader* H, const int (&n0)[3],
-                                          const double* src, double (&vref)[3]) {
+                                          const double* src, double (&vref)[3], const R* nmass = nullptr,
+                                          double mp = 0.0) {
   vref[0] = vref[1] = vref[2] = 0.0;
   if constexpr (!kFP64<R>) {
     constexpr int c = 1 + Tiling<D>::TB / 2;
     const int gi = n0[0] + c, gj = n0[1] + c, gk = D == 3 ? n0[2] + c : 0;
     if (gi < (int)H->N[0] && gj < (int)H->N[1] && gk < (int)H->N[2]) {
       const uint32_t l = node_index(H, gi, gj, gk);
+      double f = 1.0;
+      if constexpr (NORM) f = nmass[l] > R(0.0) ? mp / (double)nmass[l] : 0.0;
 #pragma unroll
-      for (int a = 0; a < D; ++a) vref[a] = src[(size_t)a * A.cap_nodes + l];
+      for (int a = 0; a < D; ++a) vref[a] = src[(size_t)a * A.cap_nodes + l] * f;
     }
   }
 }
@@ -1515,21 +1531,29 @@ __device__ __forceinline__ void load_node(const R* __restrict__ p, R (&v)[3], R 
 
 // fills a node patch from the node velocities src (minus vref) and, with
 // FLIP and want_flip, the node flips
-template <int D, bool FLIP, typename R>
+template <int D, bool FLIP, typename R, bool NORM = false>
 __device__ __forceinline__ void load_patch(const StepCommon& A, const StepHeader* H, const int (&n0)[3],
                                            const double* src, const double (&vref)[3], const R* flip, bool want_flip,
-                                           R* dst) {
+                                           R* dst, const R* nmass = nullptr, double mp = 0.0) {
   const uint32_t cap = A.cap_nodes;
   for (int n = threadIdx.x; n < Tiling<D>::NODES; n += blockDim.x) {
     uint32_t l = 0;
     const bool in = patch_node<D>(H, n0, n, l);
     R* q = dst + n * NodePatch<D, FLIP, R>::STRIDE;
+    double v[D], f = 1.0;
+#pragma unroll
+    for (int a = 0; a < D; ++a) v[a] = in ? src[(size_t)a * cap + l] : 0.0;
+    if constexpr (NORM) {
+      const double mi = in ? (double)nmass[l] : 0.0;
+      f = mi > 0 ? mp / mi : 0.0;
+    }
 #pragma unroll
     for (int a = 0; a < D; ++a) {
+      if constexpr (NORM) v[a] *= f;
       if constexpr (kFP64<R>)
-        q[a] = in ? src[(size_t)a * cap + l] : 0.0;
+        q[a] = v[a];
       else
-        q[a] = in ? (R)(src[(size_t)a * cap + l] - vref[a]) : R(0.0);
+        q[a] = in ? (R)(v[a] - vref[a]) : R(0.0);
     }
     if constexpr (FLIP) {
 #pragma unroll
@@ -2052,30 +2076,11 @@ __global__ void __launch_bounds__(MTR_MUSL_BOUNDS)
   g2p_musl_w_body<D, DEG, R>(A, perm, blockIdx.x, gridDim.x);
 }
 
-// musl.cpp:80-95: v2 /= (m_i / m_p) (zero where m_i == 0)
-template <int D, typename R>
-__device__ __forceinline__ void musl_norm_body(const StepArgsT<R>& A, const uint32_t bid, const uint32_t nblk) {
-  StepHeader* H = A.H;
-  if (step_inactive(H)) return;
-  const uint32_t G = H->G, cap = A.cap_nodes;
-  const double mp = A.P->particle_mass;
-  for (uint32_t l = bid * blockDim.x + threadIdx.x; l < G; l += nblk * blockDim.x) {
-    const double mi = A.nmass[l];
-#pragma unroll
-    for (int a = 0; a < D; ++a) {
-      double* p = &A.v2[(size_t)a * cap + l];
-      *p = (mi > 0) ? *p / (mi / mp) : 0.0;
-    }
-  }
-}
-
-template <int D, typename R>
-__global__ void __launch_bounds__(256) k_musl_norm(StepArgsT<R> A) {
-  musl_norm_body<D, R>(A, blockIdx.x, gridDim.x);
-}
-
-// MUSL: deformation update from the normalised re-projected velocity v2 and
-// the old positions (deformation_update.cpp:6), then the return mapping.
+// MUSL: deformation update from the re-projected velocity v2 and the old
+// positions (deformation_update.cpp:6), then the return mapping.  v2 is divided
+// by m_i / m_p (zero where m_i == 0, musl.cpp:80-95) as the patch is loaded: 1
+// division a patch node, where a kernel of its own over the grid took 6 us at
+// 172,000 nodes and a launch.
 template <int D, int DEG, typename R, int PM>
 __device__ __forceinline__ void defgrad_t_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid, const uint32_t nblk) {
   using TL = Tiling<D>;
@@ -2093,8 +2098,9 @@ __device__ __forceinline__ void defgrad_t_body(const StepArgsT<R>& A, const uint
   int n0[3];
   load_tile_setup<D>(A, H, t, n0, crd);
   double vref[3];
-  tile_vref<D, R>(A, H, n0, A.v2, vref);
-  load_patch<D, false, R>(A, H, n0, A.v2, vref, (const R*)nullptr, false, pv);
+  const double mp = A.P->particle_mass;
+  tile_vref<D, R, true>(A, H, n0, A.v2, vref, A.nmass, mp);
+  load_patch<D, false, R, true>(A, H, n0, A.v2, vref, (const R*)nullptr, false, pv, A.nmass, mp);
   __syncthreads();
   const uint32_t Np = A.Np;
   const double dt = H->dt, ioh = A.P->one_over_dx;
@@ -2290,13 +2296,6 @@ __global__ void __launch_bounds__(MTR_MUSL_BOUNDS) kb_g2p_musl_w(BatchView<R> B)
   batch_tiles(B, [&](const StepArgsT<R>& A, uint32_t b, uint32_t nb) {
     g2p_musl_w_body<D, DEG, R>(A, A.perm, b, nb);
   });
-}
-
-template <int D, typename R>
-__global__ void __launch_bounds__(256) kb_musl_norm(BatchView<R> B) {
-  uint32_t b, nb;
-  const StepArgsT<R>* A = batch_locate(B, kBK_NODES, b, nb);
-  if (A) musl_norm_body<D, R>(*A, b, nb);
 }
 
 template <int D, int DEG, typename R, int PM = -1>
