@@ -682,6 +682,13 @@ __device__ __forceinline__ void tile_range(const StepCommon& A, uint32_t t, uint
   pe = A.cell_start[t * 64u + 64u];
 }
 
+// Share `part` of `parts` of a tile's particles [pb, pe): even, cut at whole warps.
+__device__ __forceinline__ void part_range(uint32_t part, uint32_t parts, uint32_t& pb, uint32_t& pe) {
+  const uint32_t n = pe - pb, b = pb;
+  pb = b + (n * part / parts & ~31u);
+  if (part + 1 < parts) pe = b + (n * (part + 1) / parts & ~31u);
+}
+
 template <int D>
 __device__ __forceinline__ void tile_coords(const StepHeader* H, uint32_t t, int (&tc)[3]) {
   if constexpr (D == 3) {
@@ -753,18 +760,22 @@ __device__ __forceinline__ bool patch_node(const StepHeader* H, const int (&n0)[
 }
 
 // ---------------------------------------------------------------------------
-// 5. P2G + stress force, one block per tile, each warp on its own.
+// 5. P2G + stress force, one block per tile (or per part of one), each warp on
+// its own.
 //
-// The sorted particles of a tile are 16 runs of 4 cells along the innermost
-// axis (a unit).  A warp takes one unit per lane group: it stages a few of the
-// unit's particles in its own part of shared memory (weights, offsets and the
-// factors of momentum and force), then every lane accumulates its stencil
-// columns over those particles.  A column is the 4 nodes along the innermost
-// axis; its sums stay in registers as a window that slides with the cells, so
-// a node is added to the shared patch once per unit (7 nodes for 4 cells)
-// instead of once per cell or per few particles.  No two lanes of a group ever
-// meet on one address, and there is no block barrier between the start and
-// the flush of the patch (one global atomic per node and channel).
+// A warp takes a run of the tile's cells, whose sorted particles lie together.
+// It stages 16 particles at a time in its own part of shared memory (weights,
+// offsets and the factors of momentum and force), then every lane accumulates
+// its stencil column over them, cell by cell.  A column is the 4 nodes along
+// the innermost axis; its sums stay in registers as a window that slides with
+// the cells, so a node is added to the shared patch once per row of cells (7
+// nodes for 4 cells) instead of once per cell or per few particles.  All
+// control flow is the same for the whole warp: the cells' ranges come from the
+// sort.  Where a particle's columns leave lanes over (2D, or without the
+// force), the warp's groups of lanes take the cell's particles in turn and their
+// sums are exchanged when a node leaves the window.  There is no block barrier
+// between the start and the flush of the patch (one global atomic per node and
+// channel).
 //
 // The lanes of a group come in two roles with the same code: role 0 sums mass
 // and momentum, role 1 the force (and friction).  With per-axis factors w and
@@ -781,8 +792,10 @@ __device__ __forceinline__ bool patch_node(const StepHeader* H, const int (&n0)[
 // Bound: FP64 issue and shared-memory loads of the factors.
 // In the sum phase the shared-memory pipe is 73% busy in FP64 (32 wavefronts a
 // particle, most of them 16-byte loads of the factors; ncu).  ms per launch:
-// 1,024,000 particles, cubic, FP64 0.403 -> 0.291, mixed 0.242 -> 0.191; 2M
-// quadratic mixed 0.465 -> 0.351; 51,200 in 2D FP64 0.062 -> 0.024.
+// 1,024,000 particles, cubic, FP64 0.403 -> 0.280, mixed 0.242 -> 0.183; 2M
+// quadratic mixed 0.465 -> 0.320; 51,200 in 2D FP64 0.062 -> 0.020.  A group of
+// lanes on its own run of 4 cells, with its particles' bases checked one by one,
+// took 0.291, 0.191, 0.351 and 0.024.
 // Tried: holding the next chunk's particles in registers while one is summed
 // (spills, 0.35 -> 0.52), a third register bound (80 registers, 0.45).
 // ---------------------------------------------------------------------------
@@ -835,33 +848,123 @@ constexpr int g2p_min_blocks() {
 // Padded to an odd multiple of 16 bytes, so that the lanes that stage
 // neighbouring slots store to different banks (a 512-byte stride made the
 // FP64 stores 16-way conflicts, 65% of the kernel's shared-memory cycles).
-template <int D, typename R>
+template <int D, typename R, int ROLES>
 struct PStageData {
-  R w[D][4], a[2][D][4];
-  R q[2][D][4];
+  R w[D][4], a[ROLES][D][4];
+  R q[ROLES][D][4];
   R mui;  // factor of role 1's fourth channel, the mu(I) deviation (role 0: 1, the mass)
 };
 constexpr size_t stage_stride(size_t n) {
   n = align16(n);
   return n % 32 ? n : n + 16;
 }
-template <int D, typename R>
-struct __align__(16) PStage : PStageData<D, R> {
-  char pad[stage_stride(sizeof(PStageData<D, R>)) - sizeof(PStageData<D, R>)];
+template <int D, typename R, int ROLES>
+struct __align__(16) PStage : PStageData<D, R, ROLES> {
+  char pad[stage_stride(sizeof(PStageData<D, R, ROLES>)) - sizeof(PStageData<D, R, ROLES>)];
 };
-constexpr int kTinyWeight = 1 << 12;  // some node of the particle may fall under the weight threshold
+constexpr int kStage = 16;  // particles a warp stages at a time
 
-// Lane groups of a scatter warp: each of a particle's stencil columns takes
-// ROLES lanes (P2G: mass and momentum, force; MUSL: one).
-template <int D, int ROLES>
-struct ScatterShape {
-  static constexpr int COLS = D == 3 ? 16 : 4;  // stencil columns
-  static constexpr int LPP = COLS * ROLES;      // lanes of a group
-  static constexpr int GR = 32 / LPP;           // groups of a warp
-  static constexpr int CH = COLS;               // particles a group stages at a time (P2G: two lanes each)
+// local stencil base along an axis, with the patch's first node n0, of the
+// particles of the tile's cell c (the cell's floor, clamped at the grid's first
+// node, p2g.cpp:21-24)
+__device__ __forceinline__ int cell_base(int n0, int c) { return max(n0 + c, 0) - n0; }
+
+// One step of a sum over the two halves of a warp's lanes that differ in the bit
+// off: the half without the bit returns the sum of both halves' a, the other
+// that of their b.  Half the exchanges of summing a and b in every lane.
+template <typename R>
+__device__ __forceinline__ R half_sum(R a, R b, int off) {
+  const bool up = threadIdx.x & off;
+  return (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, off);
+}
+
+// The sliding register window of a scatter: a lane's sums of NC channels on the
+// 4 innermost nodes of one stencil column.  GR = 32 / LPP groups of a warp's
+// lanes hold the same columns for different particles of a cell; their sums are
+// taken together when a node leaves the window.  All lanes call together.
+template <typename R, int NC, int LPP>
+struct Window {
+  static constexpr int GR = 32 / LPP;
+  R acc[4][NC];
+  __device__ __forceinline__ Window() {
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) acc[h][c] = R(0.0);
+  }
+  static __device__ __forceinline__ R group_sum(R v, int from) {
+#pragma unroll
+    for (int off = from; off < 32; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
+  }
+  // adds the first node to dst(channel)[node], and moves by one node
+  template <typename Dst>
+  __device__ __forceinline__ void advance(int grp, int& node, Dst&& dst) {
+    if constexpr (GR == 1) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+        if (acc[0][c] != R(0.0)) atomicAdd(dst(c) + node, acc[0][c]);
+    } else {  // channels in pairs, one for each half of the groups
+#pragma unroll
+      for (int c = 0; c + 1 < NC; c += 2) {
+        const R v = group_sum(half_sum(acc[0][c], acc[0][c + 1], LPP), 2 * LPP);
+        if (grp < 2 && v != R(0.0)) atomicAdd((grp ? dst(c + 1) : dst(c)) + node, v);
+      }
+      if constexpr (NC % 2) {
+        const R v = group_sum(acc[0][NC - 1], LPP);
+        if (grp == 0 && v != R(0.0)) atomicAdd(dst(NC - 1) + node, v);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+#pragma unroll
+      for (int h = 0; h < 3; ++h) acc[h][c] = acc[h + 1][c];
+      acc[3][c] = R(0.0);
+    }
+    ++node;
+  }
+  // adds all 4 nodes, each group its share of them, and clears the window
+  template <typename Dst>
+  __device__ __forceinline__ void flush(int grp, int node, Dst&& dst) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      if constexpr (GR == 1) {
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+          if (acc[h][c] != R(0.0)) atomicAdd(dst(c) + node + h, acc[h][c]);
+      } else {
+        const R lo = half_sum(acc[0][c], acc[1][c], LPP), hi = half_sum(acc[2][c], acc[3][c], LPP);
+        if constexpr (GR == 2) {
+          if (lo != R(0.0)) atomicAdd(dst(c) + node + grp, lo);
+          if (hi != R(0.0)) atomicAdd(dst(c) + node + 2 + grp, hi);
+        } else {
+          const R v = group_sum(half_sum(lo, hi, 2 * LPP), 4 * LPP);
+          if (grp < 4 && v != R(0.0)) atomicAdd(dst(c) + node + grp, v);
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 4; ++h) acc[h][c] = R(0.0);
+    }
+  }
 };
-constexpr int kUnits = 16;      // units of 4 cells of a tile
-constexpr int kGroupPad = 64;   // bytes between the groups' stages (different banks)
+
+// node of a lane's column (ix, iy) that a window at cell c of a tile starts at
+template <int D>
+__device__ __forceinline__ int window_node(const int (&n0)[3], int c, int ix, int iy) {
+  constexpr int PN = Tiling<D>::PN;
+  if constexpr (D == 3)
+    return ((cell_base(n0[0], c >> 4) + ix) * PN + cell_base(n0[1], (c >> 2) & 3) + iy) * PN + cell_base(n0[2], c & 3);
+  else
+    return (cell_base(n0[0], c >> 3) + ix) * PN + cell_base(n0[1], c & 7);
+}
+
+// Nodes the window moves on by from a cell to a later one, 4 where it starts anew.
+template <int D>
+__device__ __forceinline__ int window_steps(const int (&n0)[3], int from, int to) {
+  constexpr int TB = Tiling<D>::TB;
+  if (from / TB != to / TB) return 4;
+  return min(cell_base(n0[D - 1], to % TB) - cell_base(n0[D - 1], from % TB), 4);
+}
 
 // Largest block of the MUSL scatter and the resident blocks of that size its
 // register bound asks for (FP64 and FP32 storage): what leaves the gather
@@ -885,43 +988,38 @@ constexpr size_t p2g_crd_bytes() {
 // The patch's last channel (MIBF friction) is allocated only under MIBF: a
 // block without it needs 2.7 KB (FP64, 3D) less shared memory, which lets
 // five FP64 P2G blocks of 128 threads share an SM instead of four.
-template <int D, typename R>
+template <int D, typename R, bool FORCE = true>
 __host__ __device__ constexpr size_t p2g_patch_bytes(bool mibf) {
-  return align16(sizeof(R) * (Tiling<D>::NCH - (mibf ? 0 : 1)) * Tiling<D>::NODES);
+  return align16(sizeof(R) * (FORCE ? Tiling<D>::NCH - (mibf ? 0 : 1) : 1 + D) * Tiling<D>::NODES);
 }
-template <int D, typename R>
-__host__ __device__ constexpr size_t p2g_group_bytes() {
-  return ScatterShape<D, 2>::CH * sizeof(PStage<D, R>) + kGroupPad;
-}
-template <int D, typename R>
+template <int D, typename R, bool FORCE = true>
 constexpr size_t p2g_smem_bytes(int threads, bool mibf = true) {
-  return p2g_crd_bytes<D, R>() + p2g_patch_bytes<D, R>(mibf) +
-         ScatterShape<D, 2>::GR * p2g_group_bytes<D, R>() * (size_t)(threads / 32);
+  return p2g_crd_bytes<D, R>() + p2g_patch_bytes<D, R, FORCE>(mibf) +
+         kStage * sizeof(PStage<D, R, FORCE ? 2 : 1>) * (size_t)(threads / 32);
 }
 
-// local stencil base along axis a of the particles of cell c of a tile at n0
-// (the cell's floor, clamped at the grid's first node, p2g.cpp:21-24)
-__device__ __forceinline__ int cell_base(int n0, int c) { return max(n0 + c, 0) - n0; }
-
-template <int D, int DEG, typename R>
-__device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid, const uint32_t nblk) {
+// FORCE: false for mass and momentum alone (no stress, no friction, no ids)
+template <int D, int DEG, typename R, bool FORCE = true>
+__device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid,
+                                                const uint32_t part, const uint32_t parts) {
   using TL = Tiling<D>;
-  using SS = ScatterShape<D, 2>;
-  constexpr int PN = TL::PN, NODES = TL::NODES, NCH = TL::NCH, TB = TL::TB, Z = D - 1;
-  constexpr int LPP = SS::LPP, GR = SS::GR, CH = SS::CH, NC = D + 1;
+  constexpr int PN = TL::PN, NODES = TL::NODES, NCH = FORCE ? TL::NCH : 1 + D, TB = TL::TB, Z = D - 1;
+  // A lane sums NV vector components of a role and its scalar channel on one
+  // stencil column (in 2D each component takes a lane, the first the scalar
+  // too); GR groups of LPP lanes.
+  constexpr int ROLES = FORCE ? 2 : 1, COLS = D == 3 ? 16 : 4, NV = D == 3 ? 3 : 1, NC = NV + 1;
+  constexpr int LPP = COLS * ROLES * D / NV, GR = 32 / LPP;
   const StepHeader* H = A.H;
   if (step_inactive(H)) return;
   const uint32_t t = bid;
   if (t >= H->ntiles) return;
-  uint32_t pb, pe;
-  tile_range(A, t, pb, pe);
-  if (pb >= pe) return;
+  if (A.cell_start[t * 64u + 64u * part / parts] == A.cell_start[t * 64u + 64u * (part + 1) / parts]) return;
   const DevParams& P = *A.P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double(*crd)[PN] = reinterpret_cast<double(*)[PN]>(smem_raw);
   R(*patch)[NODES] = reinterpret_cast<R(*)[NODES]>(smem_raw + p2g_crd_bytes<D, R>());
-  const bool mibf = P.use_mibf;
-  const int nch = mibf ? NCH : NCH - 1;  // channels the patch holds
+  const bool mibf = FORCE && P.use_mibf;
+  const int nch = !FORCE || mibf ? NCH : NCH - 1;  // channels the patch holds
   int tc[3];
   tile_coords<D>(H, t, tc);
   const int n0[3] = {tc[0] * TB - 1, tc[1] * TB - 1, D == 3 ? tc[2] * TB - 1 : 0};
@@ -937,39 +1035,24 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
   __syncthreads();
   const uint32_t Np = A.Np;
   const double ioh = P.one_over_dx;
-  const R iohR = (R)ioh, dxR = (R)P.dx, apicD = (R)P.apicDinverse;
+  const R iohR = (R)ioh, apicD = (R)P.apicDinverse;
   const bool apic = P.flip_ratio < 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int grp = lane / LPP, q = lane % LPP;
-  const int role = q / (LPP / 2), ci = q % (LPP / 2);
-  const int ix = D == 3 ? ci >> 2 : ci, iy = D == 3 ? ci & 3 : 0;  // this lane's column
-  PStage<D, R>* st = reinterpret_cast<PStage<D, R>*>(smem_raw + p2g_crd_bytes<D, R>() + p2g_patch_bytes<D, R>(mibf) +
-                                                     (size_t)(warp * GR + grp) * p2g_group_bytes<D, R>());
+  const int grp = lane / LPP, role = lane / COLS % ROLES, col = lane % COLS;
+  const int c0 = lane / (COLS * ROLES) % (D / NV);  // first component
+  const int ix = D == 3 ? col >> 2 : col, iy = D == 3 ? col & 3 : 0;  // this lane's column
+  using Stage = PStage<D, R, ROLES>;
+  Stage* st = reinterpret_cast<Stage*>(smem_raw + p2g_crd_bytes<D, R>() + p2g_patch_bytes<D, R, FORCE>(mibf)) + warp * kStage;
   // patch channels of this role: c < D vector component, c == D mass or friction
   R* const vec = patch[role ? 1 + D : 1];
   R* const one = patch[role ? 1 + 2 * D : 0];
-  R acc[4][NC];
-#pragma unroll
-  for (int h = 0; h < 4; ++h)
-#pragma unroll
-    for (int c = 0; c < NC; ++c) acc[h][c] = R(0.0);
+  auto dst = [&](int c) { return c < NV ? vec + (c0 + c) * NODES : one; };
+  Window<R, NC, LPP> win;
   int node0 = 0;  // node of the window's first entry
-  // adds the first node of the window to the patch and moves the window by one
-  auto advance = [&]() {
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const R v = acc[0][c];
-      if (v != R(0.0)) atomicAdd(c < D ? &vec[c * NODES + node0] : &one[node0], v);
-#pragma unroll
-      for (int h = 0; h < 3; ++h) acc[h][c] = acc[h + 1][c];
-      acc[3][c] = R(0.0);
-    }
-    ++node0;
-  };
   // adds a staged particle to the window; TINY: some node may fall under the
   // weight threshold of p2g.cpp:35 (mass and momentum of weights <= 1e-25 are
   // skipped, which is checked node by node for such a particle)
-  auto add = [&](const PStage<D, R>& S, auto tiny) {
+  auto add = [&](const Stage& S, auto tiny) {
     R f1[4], f2[4];
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
@@ -990,76 +1073,78 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
         if (role == 0 && !(f1[h] * u0 > R(1e-25))) f1[h] = f2[h] = R(0.0);
     }
 #pragma unroll
-    for (int c = 0; c < D; ++c) {
-      R a1 = u0 * S.q[role][c][0] + u1 * S.q[role][c][1];
-      if constexpr (D == 3) a1 += u2 * S.q[role][c][2];
-      const R b1 = u0 * S.q[role][c][D];
+    for (int c = 0; c < NV; ++c) {
+      const R* f = S.q[role][c0 + c];
+      R a1 = u0 * f[0] + u1 * f[1];
+      if constexpr (D == 3) a1 += u2 * f[2];
+      const R b1 = u0 * f[D];
 #pragma unroll
-      for (int h = 0; h < 4; ++h) acc[h][c] = f2[h] * b1 + (f1[h] * a1 + acc[h][c]);
+      for (int h = 0; h < 4; ++h) win.acc[h][c] = f2[h] * b1 + (f1[h] * a1 + win.acc[h][c]);
     }
-    const R a1 = u0 * (role ? S.mui : R(1.0));
+    const R a1 = c0 ? R(0.0) : u0 * (role ? S.mui : R(1.0));
 #pragma unroll
-    for (int h = 0; h < 4; ++h) acc[h][D] += f1[h] * a1;
+    for (int h = 0; h < 4; ++h) win.acc[h][NV] += f1[h] * a1;
   };
-  for (int u0 = warp * GR; u0 < kUnits; u0 += nwarps * GR) {
-    const int c1 = 4 * (u0 + grp);  // first cell of the unit
-    const uint32_t ub = cstart[c1], count = cstart[c1 + 4] - ub;
-    const uint32_t most = GR == 1 ? count : __reduce_max_sync(0xffffffffu, count);
-    if (most == 0) continue;
-    // stencil base of the unit's cells; along the innermost axis that of its first cell
-    const int bx = cell_base(n0[0], D == 3 ? c1 >> 4 : c1 >> 3), by = D == 3 ? cell_base(n0[1], (c1 >> 2) & 3) : 0;
-    const int z1 = D == 3 ? 0 : c1 & 7;
-    node0 = D == 3 ? ((bx + ix) * PN + by + iy) * PN + cell_base(n0[Z], 0) : (bx + ix) * PN + cell_base(n0[Z], z1);
-    int cz = 0;  // cell of the unit the window is at
-    for (uint32_t k0 = 0; k0 < most; k0 += CH) {
-      __syncwarp();  // the last chunk has been read
-      // Two lanes per staged particle: role 0 stores the weights, the weights
-      // times offsets, velocity and B, role 1 the weight derivatives, the
-      // stress and mu(I).  Both evaluate both second factors and keep theirs:
-      // a branch on the role would run the two halves one after the other.
-      bool tiny = false;
-      for (int slot = ci; slot < CH; slot += LPP / 2) {
-        if (k0 + slot >= count) break;
-        PStage<D, R>& S = st[slot];
-        const uint32_t s = ub + k0 + slot, j = perm[s];
-        double xp[3] = {0.0, 0.0, 0.0};
+  // this warp's cells: a run of particles
+  const int run = part * nwarps + warp, runs = parts * nwarps;
+  int cell = 64 * run / runs;
+  const uint32_t wend = cstart[64 * (run + 1) / runs];
+  uint32_t k0 = cstart[cell];
+  if (k0 < wend) {
+    while (cstart[cell + 1] <= k0) ++cell;
+    node0 = window_node<D>(n0, cell, ix, iy);
+  }
+  for (; k0 < wend; k0 += kStage) {
+    __syncwarp();  // the last chunk has been read
+    // Role 0 stores the weights, the weights times offsets, velocity and B,
+    // role 1, in another lane, the weight derivatives, the stress and mu(I).
+    // Both evaluate both second factors and keep theirs: a branch on the role
+    // would run the two halves one after the other.
+    bool tiny = false;
+    const uint32_t s = k0 + lane % kStage;
+    const int part = lane / kStage;  // the role this lane stages
+    if (part < ROLES && s < wend) {
+      Stage& S = st[lane % kStage];
+      const uint32_t j = perm[s];
+      double xp[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-        for (int a = 0; a < D; ++a) xp[a] = A.in.x[(size_t)a * Np + j];
-        R qv[D][1 + D], mui = R(0.0);
-        if (role == 0) {
-#pragma unroll
-          for (int a = 0; a < D; ++a) {
-            qv[a][0] = A.in.v[(size_t)a * Np + j];
-#pragma unroll
-            for (int b = 0; b < D; ++b)
-              qv[a][1 + b] = apic ? apicD * A.in.B[(size_t)(a * D + b) * Np + j] : R(0.0);
-          }
-        } else {
-          R tau[Sym<D>::n];
-#pragma unroll
-          for (int i = 0; i < Sym<D>::n; ++i) tau[i] = iohR * A.in.tau[(size_t)i * Np + j];
-#pragma unroll
-          for (int a = 0; a < D; ++a) {
-            qv[a][0] = R(0.0);
-#pragma unroll
-            for (int b = 0; b < D; ++b) qv[a][1 + b] = sym_at<D>(tau, a, b);
-          }
-          if (mibf) mui = (R)((double)A.in.sc[(size_t)MTR_SCALAR_MUI * Np + j] - P.mui0);
-        }
-        // the particle's base must be its cell's (it is, unless its position is
-        // not finite or left of the grid) and its stencil inside the grid
-        const int zc = z1 + (s >= cstart[c1 + 1]) + (s >= cstart[c1 + 2]) + (s >= cstart[c1 + 3]);
-        const int lb[3] = {bx, D == 3 ? by : cell_base(n0[Z], zc), D == 3 ? cell_base(n0[Z], zc) : 0};
-        bool ok = true;
-        int least = 0;
+      for (int a = 0; a < D; ++a) xp[a] = A.in.x[(size_t)a * Np + j];
+      R qv[D][1 + D], mui = R(0.0);
+      if (!FORCE || part == 0) {
 #pragma unroll
         for (int a = 0; a < D; ++a) {
-          const int b = (int)floor((xp[a] - H->org[a]) * ioh) - 1;
-          ok = ok && max(b, 0) == lb[a] + n0[a] && lb[a] + n0[a] + 3 < (int)H->N[a];
-          const double td = (xp[a] - crd[a][lb[a] + 1]) * ioh;
-          R w[4], d[4], o[4];
+          qv[a][0] = A.in.v[(size_t)a * Np + j];
+#pragma unroll
+          for (int b = 0; b < D; ++b)
+            qv[a][1 + b] = apic ? apicD * A.in.B[(size_t)(a * D + b) * Np + j] : R(0.0);
+        }
+      } else {
+        R tau[Sym<D>::n];
+#pragma unroll
+        for (int i = 0; i < Sym<D>::n; ++i) tau[i] = iohR * A.in.tau[(size_t)i * Np + j];
+#pragma unroll
+        for (int a = 0; a < D; ++a) {
+          qv[a][0] = R(0.0);
+#pragma unroll
+          for (int b = 0; b < D; ++b) qv[a][1 + b] = sym_at<D>(tau, a, b);
+        }
+        if (mibf) mui = (R)((double)A.in.sc[(size_t)MTR_SCALAR_MUI * Np + j] - P.mui0);
+      }
+      // the particle's cell, clamped as for the sort; it must lie in the tile
+      // (it does, unless the position is not finite) and its stencil in the grid
+      bool ok = true;
+      int least = 0;
+#pragma unroll
+      for (int a = 0; a < D; ++a) {
+        const int g = (int)floor((xp[a] - H->org[a]) * ioh), c = max(g, 0) - (n0[a] + 1);
+        const bool in = (unsigned)c < (unsigned)TB;
+        const int lb = cell_base(n0[a], in ? c : 0);
+        ok = ok && in && lb + n0[a] + 3 < (int)H->N[a];
+        R w[4], d[4], o[4];
+        if constexpr (FORCE) {
+          const double td = (xp[a] - crd[a][lb + 1]) * ioh;
           axis_weights<DEG, true, R>(td, w, d);
-          if (b < 0) {  // clamped; through copies: w and d stay in registers otherwise
+          if (g < 1) {  // clamped; through copies: w and d stay in registers otherwise
             R wc[4], dc[4];
             axis_weights_any<DEG, R>(td, wc, dc);
 #pragma unroll
@@ -1068,60 +1153,79 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
               d[h] = dc[h];
             }
           }
-          axis_offsets<R>(td, dxR, o);
-          least += least_exponent<DEG>(w);
+          axis_offsets<R>(td, (R)P.dx, o);
+        } else {  // a caller's axes: every node's own coordinate
 #pragma unroll
           for (int h = 0; h < 4; ++h) {
-            if (role == 0) S.w[a][h] = w[h];
-            S.a[role][a][h] = role ? d[h] : w[h] * o[h];
+            o[h] = crd[a][lb + h] - xp[a];
+            w[h] = bspline_N<DEG>((xp[a] - crd[a][lb + h]) * ioh);
+            d[h] = R(0.0);
           }
         }
+        least += least_exponent<DEG>(w);
 #pragma unroll
-        for (int a = 0; a < D; ++a)
-#pragma unroll
-          for (int b = 0; b < 1 + D; ++b) S.q[role][a][b] = qv[a][b];
-        if (role) S.mui = mui;
-        tiny = tiny || least < -82;  // every product of weights is at least 2^least; 1e-25 < 2^-83
-        if (!ok) {  // adds nothing
-          if (role == 0) {
-            raise_status(A.H, MTR_STATUS_STENCIL_OOB, A.in.id[j]);
-#pragma unroll
-            for (int a = 0; a < D; ++a)
-#pragma unroll
-              for (int h = 0; h < 4; ++h) S.w[a][h] = R(0.0);
-          }
-#pragma unroll
-          for (int a = 0; a < D; ++a) {
-#pragma unroll
-            for (int h = 0; h < 4; ++h) S.a[role][a][h] = R(0.0);
-#pragma unroll
-            for (int b = 0; b < 1 + D; ++b) S.q[role][a][b] = R(0.0);
-          }
-          if (role) S.mui = R(0.0);
+        for (int h = 0; h < 4; ++h) {
+          if (part == 0) S.w[a][h] = w[h];
+          S.a[part][a][h] = part ? d[h] : w[h] * o[h];
         }
       }
-      const bool slow = __any_sync(0xffffffffu, tiny);  // (also orders the stage before its reads)
-      __syncwarp();
-      const int kend = count > k0 ? min((int)(count - k0), CH) : 0;
-      for (int k = 0; k < kend;) {
-        const int cend = (int)(cstart[c1 + cz + 1] - ub - k0);  // the cell's end within the chunk
-        const int e = min(cend, kend);
-        if (slow) {
-#pragma unroll 1
-          for (; k < e; ++k) add(st[k], std::true_type{});
-        } else {
-#pragma unroll 2
-          for (; k < e; ++k) add(st[k], std::false_type{});
+#pragma unroll
+      for (int a = 0; a < D; ++a)
+#pragma unroll
+        for (int b = 0; b < 1 + D; ++b) S.q[part][a][b] = qv[a][b];
+      if (part) S.mui = mui;
+      tiny = least < -82;  // every product of weights is at least 2^least; 1e-25 < 2^-83
+      if (!ok) {  // adds nothing
+        if (part == 0) {
+          if constexpr (FORCE)
+            raise_status(A.H, MTR_STATUS_STENCIL_OOB, A.in.id[j]);
+          else
+            atomicOr(&A.H->status, MTR_STATUS_STENCIL_OOB);
+#pragma unroll
+          for (int a = 0; a < D; ++a)
+#pragma unroll
+            for (int h = 0; h < 4; ++h) S.w[a][h] = R(0.0);
         }
-        if (cend > kend || cz == 3) break;  // the cell goes on in the next chunk, or the unit ends
-        // the next cell; its base is the same where both are clamped
-        if (cell_base(n0[Z], z1 + cz + 1) != cell_base(n0[Z], z1 + cz)) advance();
-        ++cz;
+#pragma unroll
+        for (int a = 0; a < D; ++a) {
+#pragma unroll
+          for (int h = 0; h < 4; ++h) S.a[part][a][h] = R(0.0);
+#pragma unroll
+          for (int b = 0; b < 1 + D; ++b) S.q[part][a][b] = R(0.0);
+        }
+        if (part) S.mui = R(0.0);
       }
     }
+    const bool slow = __any_sync(0xffffffffu, tiny);  // (also orders the stage before its reads)
+    __syncwarp();
+    const uint32_t pend = min(k0 + kStage, wend);
+    for (uint32_t k = k0;;) {
+      const uint32_t e = min(cstart[cell + 1], pend);  // the cell's end within the chunk
+      uint32_t i = k + grp;
+      if (slow) {
 #pragma unroll 1
-    for (int h = 0; h < 4; ++h) advance();
+        for (; i < e; i += GR) add(st[i - k0], std::true_type{});
+      } else {
+#pragma unroll (GR == 1 ? 2 : 1)
+        for (; i < e; i += GR) add(st[i - k0], std::false_type{});
+      }
+      if constexpr (GR > 1) __syncwarp();
+      k = e;
+      if (k == pend) break;
+      // the next cell that is not empty; the window moves there, or starts anew
+      int next = cell + 1;
+      while (cstart[next + 1] <= k) ++next;
+      const int steps = window_steps<D>(n0, cell, next);
+      cell = next;
+      if (steps == 4) {
+        win.flush(grp, node0, dst);
+        node0 = window_node<D>(n0, cell, ix, iy);
+      } else {
+        for (int h = 0; h < steps; ++h) win.advance(grp, node0, dst);
+      }
+    }
   }
+  win.flush(grp, node0, dst);
   __syncthreads();
   const uint32_t cap = A.cap_nodes;
   for (int n = threadIdx.x; n < NODES; n += blockDim.x) {
@@ -1138,7 +1242,7 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
 
 template <int D, int DEG, typename R>
 __global__ void __launch_bounds__(MTR_P2G_BOUNDS) k_p2g_w(StepArgsT<R> A, const uint32_t* __restrict__ perm) {
-  p2g_w_body<D, DEG, R>(A, perm, blockIdx.x, gridDim.x);
+  p2g_w_body<D, DEG, R>(A, perm, blockIdx.x, blockIdx.y, gridDim.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -1721,7 +1825,8 @@ __device__ __forceinline__ void gather_gradv(const R* pv, const double (*crd)[Ti
 // block per tile, node patch in shared memory.
 // ---------------------------------------------------------------------------
 template <int D, int DEG, typename R, int PM>
-__device__ __forceinline__ void g2p_t_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid, const uint32_t nblk) {
+__device__ __forceinline__ void g2p_t_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid,
+                                                const uint32_t part, const uint32_t parts) {
   using TL = Tiling<D>;
   constexpr int PN = TL::PN;
   StepHeader* H = A.H;
@@ -1730,6 +1835,7 @@ __device__ __forceinline__ void g2p_t_body(const StepArgsT<R>& A, const uint32_t
   if (t >= H->ntiles) return;
   uint32_t pb, pe;
   tile_range(A, t, pb, pe);
+  part_range(part, parts, pb, pe);
   if (pb >= pe) return;
   const DevParams& P = *A.P;
   __shared__ __align__(16) R pv[NodePatch<D, true, R>::SIZE];
@@ -1801,19 +1907,22 @@ __device__ __forceinline__ void g2p_t_body(const StepArgsT<R>& A, const uint32_t
 
 template <int D, int DEG, typename R, int PM = -1>
 __global__ void __launch_bounds__(kChunk, (g2p_min_blocks<R, PM>())) k_g2p_t(StepArgsT<R> A, const uint32_t* __restrict__ perm) {
-  g2p_t_body<D, DEG, R, PM>(A, perm, blockIdx.x, gridDim.x);
+  g2p_t_body<D, DEG, R, PM>(A, perm, blockIdx.x, blockIdx.y, gridDim.y);
 }
 
 // ---------------------------------------------------------------------------
-// 7b. MUSL (musl.cpp:6-96), one block per tile, each warp on its own units as
-// in P2G.  Phase 1 (a lane per particle): gather pic/B/flip from the shared
-// node patch, blend v, write x + dt pic, v, B.  Phase 2 (lane groups owning
-// stencil columns): the particles are staged in kMuslParts parts (half of the
-// shared memory, so more blocks per SM) and v_p + B D^-1 (x_i - x_p) is summed
-// in the sliding register windows of P2G, one lane per column.
-// Measured, ms per launch at 1,024,000 particles, cubic: FP64 0.393 -> 0.363,
-// mixed 0.258 -> 0.230.  Timing copies without one part each: the gather takes
-// about 80 us of the FP64 launch, the staging and sums 176, the shared adds 25.
+// 7b. MUSL (musl.cpp:6-96), one block per tile (or part of one), each warp on
+// its own run of cells as in P2G, 32 particles at a time.  Phase 1 (a lane per
+// particle): gather pic/B/flip from the shared node patch, blend v, write
+// x + dt pic, v, B.  Phase 2: the particles are staged in kMuslParts parts (half
+// of the shared memory, so more blocks per SM) and v_p + B D^-1 (x_i - x_p) is
+// summed in P2G's windows by two groups of lanes (2D: four, a lane for each
+// component), whose sums meet by half_sum: half the exchanges, and half the
+// shared adds (compare-and-swap loops in FP64) of every group for itself.
+// Measured, ms per launch at 1,024,000 particles, cubic: FP64 0.393 -> 0.336,
+// mixed 0.258 -> 0.217; 100,000 in 2D FP64 0.033 -> 0.027.  Each group on its
+// own 16 particles took 0.362, 0.230 and 0.037; plain sums over both groups in
+// every lane 0.376 and 0.242; two particles a turn (unrolled) 0.345 and 0.223.
 // ---------------------------------------------------------------------------
 constexpr int kMuslParts = 2;
 
@@ -1838,28 +1947,27 @@ constexpr size_t musl_patch_bytes() {
 }
 // a warp stages 32 / kMuslParts particles at a time
 template <int D, typename R>
-__host__ __device__ constexpr size_t musl_group_bytes() {
-  return ScatterShape<D, 1>::LPP / kMuslParts * sizeof(MStage<D, R>) + kGroupPad;
+__host__ __device__ constexpr size_t musl_stage_bytes() {
+  return 32 / kMuslParts * sizeof(MStage<D, R>);
 }
 template <int D, typename R>
 constexpr size_t musl_smem_bytes(int threads) {
   return musl_crd_bytes<D, R>() + musl_patch_bytes<D, R>() +
-         ScatterShape<D, 1>::GR * musl_group_bytes<D, R>() * (size_t)(threads / 32);
+         musl_stage_bytes<D, R>() * (size_t)(threads / 32);
 }
 
 template <int D, int DEG, typename R>
-__device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid, const uint32_t nblk) {
+__device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid,
+                                                const uint32_t part, const uint32_t parts) {
   using TL = Tiling<D>;
-  using SS = ScatterShape<D, 1>;
-  constexpr int PN = TL::PN, NODES = TL::NODES, Z = D - 1;
-  constexpr int LPP = SS::LPP, GR = SS::GR, CH = LPP / kMuslParts;
+  constexpr int PN = TL::PN, NODES = TL::NODES, TB = TL::TB, Z = D - 1;
+  // a lane sums NC components of one stencil column; GR groups of LPP lanes
+  constexpr int NC = D == 3 ? 3 : 1, COLS = D == 3 ? 16 : 4, LPP = COLS * D / NC, GR = 32 / LPP, CH = 32 / kMuslParts;
   StepHeader* H = A.H;
   if (step_inactive(H)) return;
   const uint32_t t = bid;
   if (t >= H->ntiles) return;
-  uint32_t pb, pe;
-  tile_range(A, t, pb, pe);
-  if (pb >= pe) return;
+  if (A.cell_start[t * 64u + 64u * part / parts] == A.cell_start[t * 64u + 64u * (part + 1) / parts]) return;
   const DevParams& P = *A.P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double(*crd)[PN] = reinterpret_cast<double(*)[PN]>(smem_raw);
@@ -1873,189 +1981,179 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
   const double fr = P.flip_ratio;
   load_patch<D, true, R>(A, H, n0, A.nv, vref, A.nflip, fr >= -1, pv);
   for (int i = threadIdx.x; i < D * NODES; i += blockDim.x) (&vsum[0][0])[i] = R(0.0);
-  __shared__ uint32_t ustart[kUnits + 1];  // first particle of each unit
-  if (threadIdx.x <= kUnits) ustart[threadIdx.x] = A.cell_start[t * 64u + 4u * threadIdx.x];
+  __shared__ uint32_t cstart[65];  // first particle of each cell of the tile
+  for (int i = threadIdx.x; i < 65; i += blockDim.x) cstart[i] = A.cell_start[t * 64u + i];
   __syncthreads();
   const uint32_t Np = A.Np;
   const double dt = H->dt, ioh = P.one_over_dx;
   const R dx = (R)P.dx, apicD = (R)P.apicDinverse;
   const bool apic = fr < 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int grp = lane / LPP, q = lane % LPP;
-  const int ix = D == 3 ? q >> 2 : q, iy = D == 3 ? q & 3 : 0;  // this lane's column
+  const int grp = lane / LPP, col = lane % COLS, c0 = NC == 1 ? lane % LPP / COLS : 0;
+  const int ix = D == 3 ? col >> 2 : col, iy = D == 3 ? col & 3 : 0;  // this lane's column
   MStage<D, R>* st = reinterpret_cast<MStage<D, R>*>(smem_raw + musl_crd_bytes<D, R>() + musl_patch_bytes<D, R>() +
-                                                     (size_t)(warp * GR + grp) * musl_group_bytes<D, R>());
+                                                     (size_t)warp * musl_stage_bytes<D, R>());
   // the gather's x and y factors use the warp's stage, which phase 1 does not
-  R* xfac = reinterpret_cast<R*>(smem_raw + musl_crd_bytes<D, R>() + musl_patch_bytes<D, R>() +
-                                 (size_t)warp * GR * musl_group_bytes<D, R>()) + lane;
-  static_assert(8 * (D - 1) * 32 * sizeof(R) <= GR * musl_group_bytes<D, R>(), "x and y factors must fit the warp's stage");
-  for (int u0 = warp * GR; u0 < kUnits; u0 += nwarps * GR) {
-    const uint32_t ub = ustart[u0 + grp], count = ustart[u0 + grp + 1] - ub;
-    const uint32_t most = GR == 1 ? count : __reduce_max_sync(0xffffffffu, count);
-    for (uint32_t k0 = 0; k0 < most; k0 += LPP) {
-      // phase 1
-      __syncwarp();  // the stage has been read
-      const bool has = k0 + q < count;
-      int packed = -1;
-      R vs[D], Bs[D][D];
-      double td[3] = {0.0, 0.0, 0.0};
-      if (has) {
-        const uint32_t s = ub + k0 + q, j = perm[s];
-        double xp[3] = {0, 0, 0};
+  R* xfac = reinterpret_cast<R*>(st) + lane;
+  static_assert(8 * (D - 1) * 32 * sizeof(R) <= musl_stage_bytes<D, R>(), "x and y factors must fit the warp's stage");
+  // this warp's cells: a run of particles
+  const int run = part * nwarps + warp, runs = parts * nwarps;
+  int cell = 64 * run / runs;
+  const uint32_t wend = cstart[64 * (run + 1) / runs];
+  for (uint32_t k0 = cstart[cell]; k0 < wend; k0 += 32) {
+    // phase 1
+    __syncwarp();  // the stage has been read
+    const uint32_t s = k0 + lane;
+    bool ok = false;
+    R vs[D], Bs[D][D];
+    double td[3] = {0.0, 0.0, 0.0};
+    if (s < wend) {
+      const uint32_t j = perm[s];
+      double xp[3] = {0, 0, 0};
 #pragma unroll
-        for (int a = 0; a < D; ++a) xp[a] = A.in.x[(size_t)a * Np + j];
-        double pic[3];
-        R flp[3], Bp[D][D], gv[D][D];
-        int lb[3];
-        if (local_base<D>(H, xp, ioh, n0, false, lb)) {
-          gather_patch<D, DEG, false, 32, 4, R>(pv, crd, lb, xp, ioh, dx, xfac, vref, pic, Bp, flp, gv, apic, fr >= -1);
-          // the re-scatter's base, clamped at zero like P2G's (musl.cpp:35-40), is
-          // the same one: the gather takes no particle left of the first node
-          packed = lb[0] | (lb[1] << 4) | (lb[2] << 8);
+      for (int a = 0; a < D; ++a) xp[a] = A.in.x[(size_t)a * Np + j];
+      double pic[3];
+      R flp[3], Bp[D][D], gv[D][D];
+      int lb[3];
+      ok = local_base<D>(H, xp, ioh, n0, false, lb);
+      if (ok) {
+        gather_patch<D, DEG, false, 32, 4, R>(pv, crd, lb, xp, ioh, dx, xfac, vref, pic, Bp, flp, gv, apic, fr >= -1);
 #pragma unroll
-          for (int a = 0; a < D; ++a) td[a] = (xp[a] - crd[a][lb[a] + 1]) * ioh;
-        } else {
-          raise_status(H, MTR_STATUS_STENCIL_OOB, A.in.id[j]);
+        for (int a = 0; a < D; ++a) td[a] = (xp[a] - crd[a][lb[a] + 1]) * ioh;
+      } else {
+        raise_status(H, MTR_STATUS_STENCIL_OOB, A.in.id[j]);
 #pragma unroll
-          for (int a = 0; a < 3; ++a) {
-            pic[a] = 0.0;
-            flp[a] = R(0.0);
-          }
-#pragma unroll
-          for (int r = 0; r < D; ++r)
-#pragma unroll
-            for (int c = 0; c < D; ++c) Bp[r][c] = R(0.0);
+        for (int a = 0; a < 3; ++a) {
+          pic[a] = 0.0;
+          flp[a] = R(0.0);
         }
-        double xn[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int a = 0; a < D; ++a) {
-          const double vn = blend_v(fr, (double)A.in.v[(size_t)a * Np + j], (double)flp[a], pic[a]);
-          vs[a] = (R)vn;
-          xn[a] = xp[a] + dt * pic[a];  // positionUpdate: x + dt pic
-          A.out.v[(size_t)a * Np + s] = (R)vn;
-        }
-        wrap_and_teleport(P, xn);
-#pragma unroll
-        for (int a = 0; a < D; ++a) A.out.x[(size_t)a * Np + s] = xn[a];
 #pragma unroll
         for (int r = 0; r < D; ++r)
 #pragma unroll
-          for (int c = 0; c < D; ++c) {
-            const R b = apic ? Bp[r][c] : R(0.0);
-            A.out.B[(size_t)(r * D + c) * Np + s] = b;
-            Bs[r][c] = apicD * b;
-          }
-        A.out.id[s] = A.in.id[j];
-        if (P.store_pic_flip) {
-#pragma unroll
-          for (int a = 0; a < D; ++a) {
-            A.pic[(size_t)a * Np + s] = (R)pic[a];
-            A.flip[(size_t)a * Np + s] = (fr >= -1) ? flp[a] : R(0.0);
-          }
-        }
+          for (int c = 0; c < D; ++c) Bp[r][c] = R(0.0);
       }
-      // phase 2; the window starts and ends with the chunk, so that its registers
-      // are free during the gather
-      R acc[4][D];
+      double xn[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-      for (int h = 0; h < 4; ++h)
+      for (int a = 0; a < D; ++a) {
+        const double vn = blend_v(fr, (double)A.in.v[(size_t)a * Np + j], (double)flp[a], pic[a]);
+        vs[a] = (R)vn;
+        xn[a] = xp[a] + dt * pic[a];  // positionUpdate: x + dt pic
+        A.out.v[(size_t)a * Np + s] = (R)vn;
+      }
+      wrap_and_teleport(P, xn);
 #pragma unroll
-        for (int c = 0; c < D; ++c) acc[h][c] = R(0.0);
-      int curb = 0, curz = -1;
-      auto advance = [&]() {
-        const int bx = curb & 15, by = curb >> 4;
-        const int node = D == 3 ? ((bx + ix) * PN + (by + iy)) * PN + curz : (bx + ix) * PN + curz;
+      for (int a = 0; a < D; ++a) A.out.x[(size_t)a * Np + s] = xn[a];
+#pragma unroll
+      for (int r = 0; r < D; ++r)
 #pragma unroll
         for (int c = 0; c < D; ++c) {
-          if (acc[0][c] != R(0.0)) atomicAdd(&vsum[c][node], acc[0][c]);
-#pragma unroll
-          for (int h = 0; h < 3; ++h) acc[h][c] = acc[h + 1][c];
-          acc[3][c] = R(0.0);
+          const R b = apic ? Bp[r][c] : R(0.0);
+          A.out.B[(size_t)(r * D + c) * Np + s] = b;
+          Bs[r][c] = apicD * b;
         }
-        ++curz;
-      };
-#pragma unroll 1
-      for (int part = 0; part < kMuslParts; ++part) {
-        if (k0 + part * CH >= most) break;
-        __syncwarp();  // the last part has been read
-        if (q / CH == part) {
-          MStage<D, R>& S = st[q % CH];
-          if (packed >= 0) {
-            int least = 0;
+      A.out.id[s] = A.in.id[j];
+      if (P.store_pic_flip) {
 #pragma unroll
-            for (int a = 0; a < D; ++a) {
-              R w[4], d[4], o[4];
-              axis_weights<DEG, false, R>(td[a], w, d);
-              axis_offsets<R>(td[a], dx, o);
-#pragma unroll
-              for (int h = 0; h < 4; ++h) {
-                S.w[a][h] = w[h];
-                S.a[a][h] = w[h] * o[h];
-              }
-              least += least_exponent<DEG>(w);
-            }
-#pragma unroll
-            for (int r = 0; r < D; ++r) {
-              S.q[r][0] = vs[r];
-#pragma unroll
-              for (int c = 0; c < D; ++c) S.q[r][1 + c] = Bs[r][c];
-            }
-            S.lb = packed | (least < -82 ? kTinyWeight : 0);
-          } else {
-            S.lb = -1;
-          }
+        for (int a = 0; a < D; ++a) {
+          A.pic[(size_t)a * Np + s] = (R)pic[a];
+          A.flip[(size_t)a * Np + s] = (fr >= -1) ? flp[a] : R(0.0);
         }
-        __syncwarp();
-        const uint32_t left = most - k0 - part * CH;
-        const int kend = left < (uint32_t)CH ? (int)left : CH;
-#pragma unroll 1
-        for (int k = 0; k < kend; ++k) {
-          const MStage<D, R>& S = st[k];
-          const int lbp = S.lb;
-          if (lbp < 0) continue;
-          const int base = D == 3 ? lbp & 255 : lbp & 15, bz = (D == 3 ? lbp >> 8 : lbp >> 4) & 15;
-          if (base != curb || bz != curz) {
-            if (curz >= 0) {
-              const int to = base == curb && bz > curz && bz < curz + 4 ? bz : curz + 4;
-              while (curz < to) advance();
-            }
-            curb = base;
-            curz = bz;
-          }
-          R f1[4], f2[4];
-#pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            f1[h] = S.w[Z][h];
-            f2[h] = S.a[Z][h];
-          }
-          R u0 = S.w[0][ix], u1 = S.a[0][ix];
-          [[maybe_unused]] R u2 = R(0.0);
-          if constexpr (D == 3) {
-            const R wy = S.w[1][iy], ay = S.a[1][iy];
-            u2 = u0 * ay;
-            u0 *= wy;
-            u1 *= wy;
-          }
-          if (lbp & kTinyWeight) {  // musl.cpp:51 skips weights <= 1e-25
-#pragma unroll
-            for (int h = 0; h < 4; ++h)
-              if (!(f1[h] * u0 > R(1e-25))) f1[h] = f2[h] = R(0.0);
-          }
-#pragma unroll
-          for (int c = 0; c < D; ++c) {
-            R a1 = u0 * S.q[c][0] + u1 * S.q[c][1];
-            if constexpr (D == 3) a1 += u2 * S.q[c][2];
-            const R b1 = u0 * S.q[c][D];
-#pragma unroll
-            for (int h = 0; h < 4; ++h) acc[h][c] = f2[h] * b1 + (f1[h] * a1 + acc[h][c]);
-          }
-        }
-      }
-      if (curz >= 0) {
-        const int to = curz + 4;
-        while (curz < to) advance();
       }
     }
+    // phase 2; the window starts and ends with the chunk, so that its registers
+    // are free during the gather.  The re-scatter's base, clamped at zero like
+    // P2G's (musl.cpp:35-40), is the gather's, which takes no particle left of
+    // the first node, and so the cell's.
+    Window<R, NC, LPP> win;
+    auto dst = [&](int c) { return vsum[c0 + c]; };
+    while (cstart[cell + 1] <= k0) ++cell;
+    int node0 = window_node<D>(n0, cell, ix, iy);  // node of the window's first entry
+#pragma unroll 1
+    for (int part = 0; part < kMuslParts; ++part) {
+      const uint32_t p0 = k0 + part * CH, pend = min(p0 + CH, wend);
+      if (p0 >= wend) break;
+      __syncwarp();  // the last part has been read
+      bool tiny = false;
+      if (lane / CH == part) {
+        MStage<D, R>& S = st[lane % CH];
+        int least = 0;
+#pragma unroll
+        for (int a = 0; a < D; ++a) {
+          R w[4], d[4], o[4];
+          axis_weights<DEG, false, R>(td[a], w, d);
+          axis_offsets<R>(td[a], dx, o);
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            S.w[a][h] = ok ? w[h] : R(0.0);
+            S.a[a][h] = ok ? w[h] * o[h] : R(0.0);
+          }
+          least += least_exponent<DEG>(w);
+        }
+#pragma unroll
+        for (int r = 0; r < D; ++r) {
+          S.q[r][0] = ok ? vs[r] : R(0.0);
+#pragma unroll
+          for (int c = 0; c < D; ++c) S.q[r][1 + c] = ok ? Bs[r][c] : R(0.0);
+        }
+        tiny = least < -82;
+      }
+      const bool slow = __any_sync(0xffffffffu, tiny);
+      __syncwarp();
+      auto add = [&](const MStage<D, R>& S, auto small) {
+        R f1[4], f2[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          f1[h] = S.w[Z][h];
+          f2[h] = S.a[Z][h];
+        }
+        R u0 = S.w[0][ix], u1 = S.a[0][ix];
+        [[maybe_unused]] R u2 = R(0.0);
+        if constexpr (D == 3) {
+          const R wy = S.w[1][iy], ay = S.a[1][iy];
+          u2 = u0 * ay;
+          u0 *= wy;
+          u1 *= wy;
+        }
+        if constexpr (decltype(small)::value) {  // musl.cpp:51 skips weights <= 1e-25
+#pragma unroll
+          for (int h = 0; h < 4; ++h)
+            if (!(f1[h] * u0 > R(1e-25))) f1[h] = f2[h] = R(0.0);
+        }
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          R a1 = u0 * S.q[c0 + c][0] + u1 * S.q[c0 + c][1];
+          if constexpr (D == 3) a1 += u2 * S.q[c0 + c][2];
+          const R b1 = u0 * S.q[c0 + c][D];
+#pragma unroll
+          for (int h = 0; h < 4; ++h) win.acc[h][c] = f2[h] * b1 + (f1[h] * a1 + win.acc[h][c]);
+        }
+      };
+      for (uint32_t k = p0;;) {
+        const uint32_t e = min(cstart[cell + 1], pend);  // the cell's end within the part
+        if (slow) {
+#pragma unroll 1
+          for (k += grp; k < e; k += GR) add(st[k - p0], std::true_type{});
+        } else {
+#pragma unroll 1
+          for (k += grp; k < e; k += GR) add(st[k - p0], std::false_type{});
+        }
+        __syncwarp();
+        k = e;
+        if (k == pend) break;
+        // the next cell that is not empty; the window moves there, or starts anew
+        int next = cell + 1;
+        while (cstart[next + 1] <= k) ++next;
+        const int steps = window_steps<D>(n0, cell, next);
+        cell = next;
+        if (steps == 4) {
+          win.flush(grp, node0, dst);
+          node0 = window_node<D>(n0, cell, ix, iy);
+        } else {
+          for (int h = 0; h < steps; ++h) win.advance(grp, node0, dst);
+        }
+      }
+    }
+    win.flush(grp, node0, dst);
   }
   __syncthreads();
   const uint32_t cap = A.cap_nodes;
@@ -2073,7 +2171,7 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
 template <int D, int DEG, typename R>
 __global__ void __launch_bounds__(MTR_MUSL_BOUNDS)
     k_g2p_musl_w(StepArgsT<R> A, const uint32_t* __restrict__ perm) {
-  g2p_musl_w_body<D, DEG, R>(A, perm, blockIdx.x, gridDim.x);
+  g2p_musl_w_body<D, DEG, R>(A, perm, blockIdx.x, blockIdx.y, gridDim.y);
 }
 
 // MUSL: deformation update from the re-projected velocity v2 and the old
@@ -2082,7 +2180,8 @@ __global__ void __launch_bounds__(MTR_MUSL_BOUNDS)
 // division a patch node, where a kernel of its own over the grid took 6 us at
 // 172,000 nodes and a launch.
 template <int D, int DEG, typename R, int PM>
-__device__ __forceinline__ void defgrad_t_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid, const uint32_t nblk) {
+__device__ __forceinline__ void defgrad_t_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid,
+                                                const uint32_t part, const uint32_t parts) {
   using TL = Tiling<D>;
   constexpr int PN = TL::PN;
   StepHeader* H = A.H;
@@ -2091,6 +2190,7 @@ __device__ __forceinline__ void defgrad_t_body(const StepArgsT<R>& A, const uint
   if (t >= H->ntiles) return;
   uint32_t pb, pe;
   tile_range(A, t, pb, pe);
+  part_range(part, parts, pb, pe);
   if (pb >= pe) return;
   __shared__ __align__(16) R pv[NodePatch<D, false, R>::SIZE];
   __shared__ R xfac[8 * (D - 1) * kMaxTileThreads];  // x and y factors of each thread's gather
@@ -2131,7 +2231,7 @@ __device__ __forceinline__ void defgrad_t_body(const StepArgsT<R>& A, const uint
 
 template <int D, int DEG, typename R, int PM = -1>
 __global__ void __launch_bounds__(MTR_DEFGRAD_BOUNDS) k_defgrad_t(StepArgsT<R> A, const uint32_t* __restrict__ perm) {
-  defgrad_t_body<D, DEG, R, PM>(A, perm, blockIdx.x, gridDim.x);
+  defgrad_t_body<D, DEG, R, PM>(A, perm, blockIdx.x, blockIdx.y, gridDim.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -2276,7 +2376,7 @@ __global__ void __launch_bounds__(kSortThreads) kb_sort_rank(BatchView<R> B) {
 
 template <int D, int DEG, typename R>
 __global__ void __launch_bounds__(MTR_P2G_BOUNDS) kb_p2g_w(BatchView<R> B) {
-  batch_tiles(B, [&](const StepArgsT<R>& A, uint32_t b, uint32_t nb) { p2g_w_body<D, DEG, R>(A, A.perm, b, nb); });
+  batch_tiles(B, [&](const StepArgsT<R>& A, uint32_t b, uint32_t nb) { p2g_w_body<D, DEG, R>(A, A.perm, b, 0u, 1u); });
 }
 
 template <int D, typename R>
@@ -2288,20 +2388,20 @@ __global__ void __launch_bounds__(256) kb_grid(BatchView<R> B) {
 
 template <int D, int DEG, typename R, int PM = -1>
 __global__ void __launch_bounds__(kChunk, (g2p_min_blocks<R, PM>())) kb_g2p_t(BatchView<R> B) {
-  batch_tiles(B, [&](const StepArgsT<R>& A, uint32_t b, uint32_t nb) { g2p_t_body<D, DEG, R, PM>(A, A.perm, b, nb); });
+  batch_tiles(B, [&](const StepArgsT<R>& A, uint32_t b, uint32_t nb) { g2p_t_body<D, DEG, R, PM>(A, A.perm, b, 0u, 1u); });
 }
 
 template <int D, int DEG, typename R>
 __global__ void __launch_bounds__(MTR_MUSL_BOUNDS) kb_g2p_musl_w(BatchView<R> B) {
   batch_tiles(B, [&](const StepArgsT<R>& A, uint32_t b, uint32_t nb) {
-    g2p_musl_w_body<D, DEG, R>(A, A.perm, b, nb);
+    g2p_musl_w_body<D, DEG, R>(A, A.perm, b, 0u, 1u);
   });
 }
 
 template <int D, int DEG, typename R, int PM = -1>
 __global__ void __launch_bounds__(MTR_DEFGRAD_BOUNDS) kb_defgrad_t(BatchView<R> B) {
   batch_tiles(B, [&](const StepArgsT<R>& A, uint32_t b, uint32_t nb) {
-    defgrad_t_body<D, DEG, R, PM>(A, A.perm, b, nb);
+    defgrad_t_body<D, DEG, R, PM>(A, A.perm, b, 0u, 1u);
   });
 }
 

@@ -77,160 +77,18 @@ namespace {
 std::mutex g_setup_mutex;
 void* g_scratch_ptr[kMaxDevices] = {};
 
-template <int D>
-struct NStage {
-  double x[D], v[D], B[D * D], w[D * 4];
-  int lb;
-  int pad;
-};
+// Threads of a scatter block.  Eight warps per tile: a call's tiles are few (64
+// for 4k particles, about 700 at capacity), so the chain of particles that each
+// warp works through sets how long the launch takes.  Whole call, with the
+// step's scatter in place of one that staged a block's particles between
+// barriers: 4k particles 82 -> 49 us, 261k 109 -> 97 us.
+constexpr int kScatterThreads = 256;
 
-// The P2G variant: as k_p2g_w, but mass and momentum only (no stress, no
-// friction channel), accumulating into the scratch grid.
+// The step's scatter, mass and momentum only, accumulating into the scratch
+// grid.
 template <int D, int DEG>
-__global__ void __launch_bounds__(kChunk) k_p2g_noalloc(StepArgs A, const uint32_t* __restrict__ perm) {
-  using TL = Tiling<D>;
-  constexpr int PN = TL::PN, NODES = TL::NODES, TB = TL::TB;
-  constexpr int NCH = 1 + D;
-  const StepHeader* H = A.H;
-  const uint32_t t = blockIdx.x;
-  if (t >= H->ntiles) return;
-  uint32_t pb, pe;
-  tile_range(A, t, pb, pe);
-  if (pb >= pe) return;
-  const DevParams& P = *A.P;
-  extern __shared__ double smem[];
-  double(*patch)[NODES] = reinterpret_cast<double(*)[NODES]>(smem);
-  double(*crd)[PN] = reinterpret_cast<double(*)[PN]>(smem + NCH * NODES);
-  NStage<D>* st = reinterpret_cast<NStage<D>*>(smem + NCH * NODES + 3 * PN);
-  int tc[3];
-  tile_coords<D>(H, t, tc);
-  const int n0[3] = {tc[0] * TB - 1, tc[1] * TB - 1, D == 3 ? tc[2] * TB - 1 : 0};
-  for (int i = threadIdx.x; i < NCH * NODES; i += blockDim.x) (&patch[0][0])[i] = 0.0;
-  for (int i = threadIdx.x; i < D * PN; i += blockDim.x) {
-    const int a = i / PN, o = i % PN;
-    const int g = n0[a] + o;
-    const double* ax = a == 0 ? A.gx : (a == 1 ? A.gy : A.gz);
-    crd[a][o] = (g >= 0 && g < (int)H->N[a]) ? ax[g] : 0.0;
-  }
-  __syncthreads();
-  const uint32_t Np = A.Np;
-  const double ioh = P.one_over_dx, apicD = P.apicDinverse;
-  const bool apic = P.flip_ratio < 0;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int LPP = D == 3 ? 16 : 4;
-  const int q = lane % LPP;
-  const int iy = D == 3 ? (q >> 2) : q;
-  const int iz = D == 3 ? (q & 3) : 0;
-  const int kbeg = warp * 32 + (lane / LPP) * LPP, kend = kbeg + LPP;
-  for (uint32_t c0 = pb; c0 < pe; c0 += kChunk) {
-    {
-      const uint32_t s = c0 + threadIdx.x;
-      NStage<D>& S = st[threadIdx.x];
-      int packed = -1;
-      if (s < pe) {
-        const uint32_t j = perm[s];
-        double xp[3] = {0, 0, 0};
-#pragma unroll
-        for (int a = 0; a < D; ++a) {
-          xp[a] = A.in.x[(size_t)a * Np + j];
-          S.x[a] = xp[a];
-          S.v[a] = A.in.v[(size_t)a * Np + j];
-        }
-#pragma unroll
-        for (int r = 0; r < D * D; ++r) S.B[r] = apic ? A.in.B[(size_t)r * Np + j] : 0.0;
-        int lb[3];
-        if (local_base<D>(H, xp, ioh, n0, true, lb)) {
-#pragma unroll
-          for (int a = 0; a < D; ++a)
-#pragma unroll
-            for (int o = 0; o < 4; ++o) S.w[a * 4 + o] = bspline_N<DEG>((xp[a] - crd[a][lb[a] + o]) * ioh);
-          packed = lb[0] | (lb[1] << 4) | (lb[2] << 8);
-        } else {
-          atomicOr(&A.H->status, MTR_STATUS_STENCIL_OOB);
-        }
-      }
-      S.lb = packed;
-    }
-    __syncthreads();
-    {
-      double acc[4][NCH];
-#pragma unroll
-      for (int h = 0; h < 4; ++h)
-#pragma unroll
-        for (int ch = 0; ch < NCH; ++ch) acc[h][ch] = 0.0;
-      int cur = -1;
-      auto flush = [&]() {
-        const int lbx = cur & 15, lby = (cur >> 4) & 15, lbz = cur >> 8;
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          const int node = D == 3 ? ((lbx + h) * PN + (lby + iy)) * PN + (lbz + iz) : (lbx + h) * PN + (lby + iy);
-#pragma unroll
-          for (int ch = 0; ch < NCH; ++ch) {
-            if (acc[h][ch] != 0.0) atomicAdd(&patch[ch][node], acc[h][ch]);
-            acc[h][ch] = 0.0;
-          }
-        }
-      };
-      for (int k = kbeg; k < kend; ++k) {
-        const NStage<D>& S = st[k];
-        const int lbp = S.lb;
-        if (lbp < 0) continue;
-        if (lbp != cur) {
-          if (cur >= 0) flush();
-          cur = lbp;
-        }
-        const int lbx = lbp & 15, lby = (lbp >> 4) & 15, lbz = lbp >> 8;
-        const double wyz = D == 3 ? S.w[4 + iy] * S.w[8 + iz] : S.w[4 + iy];
-        const double pdy = crd[1][lby + iy] - S.x[1];
-        const double pdz = D == 3 ? crd[2][lbz + iz] - S.x[D - 1] : 0.0;
-        double Tm[D], Sm[D];
-#pragma unroll
-        for (int a = 0; a < D; ++a) {
-          if (apic) {
-            double byz = S.B[a * D + 1] * pdy;
-            if constexpr (D == 3) byz += S.B[a * D + 2] * pdz;
-            Tm[a] = S.v[a] + apicD * byz;
-            Sm[a] = apicD * S.B[a * D];
-          } else {
-            Tm[a] = S.v[a];
-            Sm[a] = 0.0;
-          }
-        }
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          const double weight = S.w[h] * wyz;
-          if (!(weight > 1e-25)) continue;
-          const double pdx = crd[0][lbx + h] - S.x[0];
-          acc[h][0] += weight;
-#pragma unroll
-          for (int a = 0; a < D; ++a) acc[h][1 + a] += weight * (Tm[a] + Sm[a] * pdx);
-        }
-      }
-      if (cur >= 0) flush();
-    }
-    __syncthreads();
-  }
-  const uint32_t cap = A.cap_nodes;
-  for (int n = threadIdx.x; n < NODES; n += blockDim.x) {
-    int li, lj, lk;
-    if constexpr (D == 3) {
-      lk = n % PN;
-      lj = (n / PN) % PN;
-      li = n / (PN * PN);
-    } else {
-      lk = 0;
-      lj = n % PN;
-      li = n / PN;
-    }
-    const int gi = n0[0] + li, gj = n0[1] + lj, gk = n0[2] + lk;
-    if (gi < 0 || gj < 0 || gk < 0 || gi >= (int)H->N[0] || gj >= (int)H->N[1] || gk >= (int)H->N[2]) continue;
-    const uint32_t l = node_index(H, gi, gj, gk);
-#pragma unroll
-    for (int ch = 0; ch < NCH; ++ch) {
-      const double val = patch[ch][n];
-      if (val != 0.0) atomicAdd(&A.acc[(size_t)ch * cap + l], val);
-    }
-  }
+__global__ void __launch_bounds__(kScatterThreads, 2) k_p2g_noalloc(StepArgs A, const uint32_t* __restrict__ perm) {
+  p2g_w_body<D, DEG, double, false>(A, perm, blockIdx.x, 0u, 1u);
 }
 
 // Cell keys.  A particle whose cell lies outside the caller's grid (or whose
@@ -268,7 +126,7 @@ __global__ void __launch_bounds__(kSortThreads) k_noalloc_keys(StepCommon A) {
 
 template <int D>
 constexpr size_t noalloc_smem_bytes() {
-  return sizeof(double) * ((1 + D) * Tiling<D>::NODES + 3 * Tiling<D>::PN) + sizeof(NStage<D>) * kChunk;
+  return p2g_smem_bytes<D, double, false>(kScatterThreads);
 }
 
 // Writes the grid description and the few constants the kernels read into
@@ -404,7 +262,7 @@ int run_noalloc(unsigned char* base, const mtr_params& p, const double* x, const
   k_sort_scan<<<supers, kSortThreads, 0, st>>>(A);
   k_sort_place<<<pblocks, kSortThreads, 0, st>>>(A);
   k_sort_rank<<<pblocks, kSortThreads, 0, st>>>(A);
-  k_p2g_noalloc<D, DEG><<<(uint32_t)ntiles, kChunk, noalloc_smem_bytes<D>(), st>>>(A, A.perm);
+  k_p2g_noalloc<D, DEG><<<(uint32_t)ntiles, kScatterThreads, noalloc_smem_bytes<D>(), st>>>(A, A.perm);
   k_noalloc_finalize<D><<<(uint32_t)std::min<uint64_t>((G + 255) / 256, 148 * 8), 256, 0, st>>>(
       A.acc, (uint32_t)G, (uint32_t)G, p.particle_mass, grid_mass, grid_v, H, status);
   return cudaGetLastError() == cudaSuccess ? MTR_OK : MTR_ERR_CUDA;
