@@ -106,6 +106,7 @@ struct EventMarks {
 enum { kSlotP2G = 0, kSlotMUSL = 1, kSlotG2P = 2, kSlotDefgrad = 3, kTileSlots = 4 };
 // mark names that end each slot's kernel in a step
 const char* const kSlotMark[kTileSlots] = {"k_p2g", "k_g2p_musl", "k_g2p", "k_defgrad"};
+constexpr uint32_t kResidentTiles = 4 * 148;  // tile blocks taken to be on the chip at once
 // largest block of each slot (k_g2p_t is register-bounded per 128 threads)
 const int kSlotMax[kTileSlots] = {kMaxTileThreads, MTR_MUSL_MAX_THREADS, kChunk, kMaxTileThreads};
 const int kTileCandidates[3] = {64, 128, 256};
@@ -497,7 +498,7 @@ int rm_specialization(int dim, bool musl, int pm) {
 }
 
 template <int D, int DEG, typename R>
-void launch_defgrad(int spm, uint32_t blocks, int threads, cudaStream_t st, const StepArgsT<R>& A,
+void launch_defgrad(int spm, dim3 blocks, int threads, cudaStream_t st, const StepArgsT<R>& A,
                     const uint32_t* perm) {
   if constexpr (D == 3) {
     if (spm == MTR_PM_DPMUI) {
@@ -509,7 +510,7 @@ void launch_defgrad(int spm, uint32_t blocks, int threads, cudaStream_t st, cons
 }
 
 template <int D, int DEG, typename R>
-void launch_g2p(int spm, uint32_t blocks, int threads, cudaStream_t st, const StepArgsT<R>& A,
+void launch_g2p(int spm, dim3 blocks, int threads, cudaStream_t st, const StepArgsT<R>& A,
                 const uint32_t* perm) {
   if constexpr (D == 3) {
     if (spm == MTR_PM_DP) {
@@ -522,6 +523,17 @@ void launch_g2p(int spm, uint32_t blocks, int threads, cudaStream_t st, const St
     }
   }
   k_g2p_t<D, DEG, R><<<blocks, threads, 0, st>>>(A, perm);
+}
+
+// Blocks of a tile's particles.  A scene of few tiles leaves SMs idle and its
+// tile kernels last as long as one block's chain of passes over its tile, so
+// each tile is cut in 2 or 4 while the blocks still fit the chip at once (four
+// an SM); occupied tiles are counted at 8 (3D) or 4 (2D) particles a cell.  us
+// per step in 1, 2 and 4 parts: 2D 5k particles 63, 53, 47; 2D 51k 67, 58, 63;
+// 2D 212k mixed 84, 92, 112; 3D 150k 145, 144, 148; 3D 1M 831, 894, 1078.
+uint32_t tile_parts(const mtr_ctx* c) {
+  const uint32_t tiles = std::min<uint32_t>(c->cap_tiles, c->Np / (c->dim == 3 ? 512 : 256) + 1);
+  return tiles * 4 <= kResidentTiles ? 4 : (tiles * 2 <= kResidentTiles ? 2 : 1);
 }
 
 // `follows`: the step enqueued just before left its commit to this one;
@@ -554,9 +566,10 @@ int enqueue_step_t(mtr_ctx* c, int parity, bool follows, bool commit) {
   n += 4;
   const uint32_t* perm = c->perm_rank;
   const int* tt = c->tile_threads;
+  const dim3 tiles(c->cap_tiles, tile_parts(c));
   {
     const size_t sm = p2g_smem_bytes<D, R>(tt[kSlotP2G], c->prm.use_mibf != 0);
-    k_p2g_w<D, DEG, R><<<c->cap_tiles, tt[kSlotP2G], sm, st>>>(A, perm);
+    k_p2g_w<D, DEG, R><<<tiles, tt[kSlotP2G], sm, st>>>(A, perm);
   }
   ++n;
   mark(c, "k_p2g");
@@ -571,14 +584,14 @@ int enqueue_step_t(mtr_ctx* c, int parity, bool follows, bool commit) {
   mark(c, "k_grid");
   if (c->prm.use_musl) {
     const size_t sm = musl_smem_bytes<D, R>(tt[kSlotMUSL]);
-    k_g2p_musl_w<D, DEG, R><<<c->cap_tiles, tt[kSlotMUSL], sm, st>>>(A, perm);
+    k_g2p_musl_w<D, DEG, R><<<tiles, tt[kSlotMUSL], sm, st>>>(A, perm);
     mark(c, "k_g2p_musl");
-    launch_defgrad<D, DEG, R>(rm_specialization(D, true, c->prm.plastic_model), c->cap_tiles, tt[kSlotDefgrad], st,
+    launch_defgrad<D, DEG, R>(rm_specialization(D, true, c->prm.plastic_model), tiles, tt[kSlotDefgrad], st,
                               A, perm);
     mark(c, "k_defgrad");
     n += 2;
   } else {
-    launch_g2p<D, DEG, R>(rm_specialization(D, false, c->prm.plastic_model), c->cap_tiles, tt[kSlotG2P], st, A,
+    launch_g2p<D, DEG, R>(rm_specialization(D, false, c->prm.plastic_model), tiles, tt[kSlotG2P], st, A,
                           perm);
     ++n;
     mark(c, "k_g2p");
