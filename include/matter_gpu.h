@@ -320,7 +320,8 @@ int mtr_get_grid_friction(mtr_ctx* ctx, double* friction);
 
 /* Block shapes of the tile kernels — no counterpart in the reference, whose
  * loops are OpenMP-scheduled over particles.  Each step phase that walks the
- * particles of a grid tile runs one thread block per tile; its size is chosen
+ * particles of a grid tile runs one thread block per tile (two or four for a
+ * context whose tiles are few); its size is chosen
  * per context (or per batch group) among 64, 128 and 256 threads, by slot:
  *   threads[MTR_TILE_P2G]     P2G with the stress force (default 128)
  *   threads[MTR_TILE_MUSL]    MUSL G2P and re-scatter (default 128)

@@ -2,7 +2,8 @@
 // step loop of Simulation::simulate (simulation.cpp:73-213) driving the
 // kernels of mtr_kernels.cuh on one CUDA stream.
 //
-// A step is ~16 kernel launches with no host synchronisation: dt, the grid
+// A step is 9 or 10 kernel launches with no host synchronisation (and one more
+// where it commits itself instead of in the next step's header): dt, the grid
 // extents and the clock live in a device-side StepHeader.  Steps are captured
 // into CUDA graphs of kGraphSteps steps (two variants, one per starting
 // particle buffer) and replayed; the host reads the header back once per

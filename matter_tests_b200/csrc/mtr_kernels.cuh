@@ -6,7 +6,7 @@
 //   k_header      dt, gravity ramp, remesh + arange axes      update_dt.cpp:5-66, remesh.cpp:38-311
 //   k_sort_*      stable counting sort by blocked cell key    (new: locality for P2G); the cell
 //                 starts it leaves are the particle ranges of every cell and 4^3 (2D: 8^2) tile
-//   k_p2g_w       tile block -> shared grid patch -> one global atomic per node and channel
+//   k_p2g_w       tile block(s) -> shared grid patch -> one global atomic per node and channel
 //                 (mass, momentum with APIC, force tau.grad w, MIBF friction)
 //                                                              p2g.cpp:6-100, explicit_euler_update.cpp:15-77
 //   k_grid        normalise, v += -dt V0 f/m + dt g, boundary collision, flip, FP64 balances
@@ -24,8 +24,9 @@
 // every later read of the same data is nearly coalesced.
 //
 // Precision.  Every kernel that touches particle or grid state is templated
-// on the storage type R.  R = double is the reference's FP64 arithmetic,
-// operation for operation.  R = float is the mixed-precision form: particle
+// on the storage type R.  R = double is FP64 throughout, the reference's
+// formulas with sums over a stencil factorised and the SVD of a deformation near
+// the identity replaced by a series.  R = float is the mixed-precision form: particle
 // v, F, B, stress and plastic scalars, the grid mass, momentum, force,
 // friction and flip channels, the spline weights, the P2G and MUSL sums and
 // the G2P gathers are FP32.  FP64 stays on the positions, the clock, the grid
