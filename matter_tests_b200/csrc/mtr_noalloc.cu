@@ -77,18 +77,21 @@ namespace {
 std::mutex g_setup_mutex;
 void* g_scratch_ptr[kMaxDevices] = {};
 
-// Threads of a scatter block.  Eight warps per tile: a call's tiles are few (64
-// for 4k particles, about 700 at capacity), so the chain of particles that each
-// warp works through sets how long the launch takes.  Whole call, with the
-// step's scatter in place of one that staged a block's particles between
-// barriers: 4k particles 82 -> 49 us, 261k 109 -> 97 us.
+// Scatter blocks: a call's tiles are few (64 for 4k particles, about 700 at
+// capacity), so the chain of particles that each warp works through sets how
+// long the launch takes.  While four blocks of a tile each fit the chip at once,
+// a tile takes four of 256 threads, else two of 128 (whose shared memory lets
+// more of them share an SM).  us per call, tiles as 1, 2, 4 blocks of 256, and 2,
+// 4 of 128: 4k particles 49, 41, 38, 47, 41; 261k 94, 96, 111, 90, 94.  The
+// scatter that staged a block's particles between barriers took 82 and 109.
 constexpr int kScatterThreads = 256;
+constexpr uint64_t kFewTiles = 148;
 
 // The step's scatter, mass and momentum only, accumulating into the scratch
 // grid.
 template <int D, int DEG>
 __global__ void __launch_bounds__(kScatterThreads, 2) k_p2g_noalloc(StepArgs A, const uint32_t* __restrict__ perm) {
-  p2g_w_body<D, DEG, double, false>(A, perm, blockIdx.x, 0u, 1u);
+  p2g_w_body<D, DEG, double, false>(A, perm, blockIdx.x, blockIdx.y, gridDim.y);
 }
 
 // Cell keys.  A particle whose cell lies outside the caller's grid (or whose
@@ -125,8 +128,8 @@ __global__ void __launch_bounds__(kSortThreads) k_noalloc_keys(StepCommon A) {
 }
 
 template <int D>
-constexpr size_t noalloc_smem_bytes() {
-  return p2g_smem_bytes<D, double, false>(kScatterThreads);
+constexpr size_t noalloc_smem_bytes(int threads = kScatterThreads) {
+  return p2g_smem_bytes<D, double, false>(threads);
 }
 
 // Writes the grid description and the few constants the kernels read into
@@ -262,7 +265,8 @@ int run_noalloc(unsigned char* base, const mtr_params& p, const double* x, const
   k_sort_scan<<<supers, kSortThreads, 0, st>>>(A);
   k_sort_place<<<pblocks, kSortThreads, 0, st>>>(A);
   k_sort_rank<<<pblocks, kSortThreads, 0, st>>>(A);
-  k_p2g_noalloc<D, DEG><<<(uint32_t)ntiles, kScatterThreads, noalloc_smem_bytes<D>(), st>>>(A, A.perm);
+  const int parts = ntiles <= kFewTiles ? 4 : 2, threads = ntiles <= kFewTiles ? kScatterThreads : kScatterThreads / 2;
+  k_p2g_noalloc<D, DEG><<<dim3((uint32_t)ntiles, parts), threads, noalloc_smem_bytes<D>(threads), st>>>(A, A.perm);
   k_noalloc_finalize<D><<<(uint32_t)std::min<uint64_t>((G + 255) / 256, 148 * 8), 256, 0, st>>>(
       A.acc, (uint32_t)G, (uint32_t)G, p.particle_mass, grid_mass, grid_v, H, status);
   return cudaGetLastError() == cudaSuccess ? MTR_OK : MTR_ERR_CUDA;

@@ -16,17 +16,14 @@ from test_zz_no_alloc import _Call, _scene, _uniform_grid
 pytestmark = [pytest.mark.gpu, needs_gpu]
 
 
-@pytest.mark.parametrize("dim,deg", [(2, 2), (2, 3), (3, 2), (3, 3)])
-@pytest.mark.parametrize("n", [1, 15, 16, 17, 33, 255, 257, 3000])
-@pytest.mark.parametrize("crowded", [False, True])
-def test_counts_and_crowding(dim, deg, n, crowded):
+def _check(dim, deg, n, crowded, dims):
     p = _scene(dim, deg, n=4, seed=1).params
     rng = np.random.default_rng(n)
-    dims = np.array([13, 17, 11 if dim == 3 else 1])
+    dims = np.array(dims[:dim] + (1,) * (3 - dim))
     axes = _uniform_grid(dims, p.dx, (-0.3, 0.7, 0.1))
-    cells = rng.integers(1, dims[:dim] - 3, size=(n, dim))
+    cells = rng.integers(1, np.maximum(dims[:dim] - 3, 2), size=(n, dim))
     if crowded:
-        cells = np.where(rng.uniform(size=(n, 1)) < 0.8, 5, 1 + (cells - 1) // 3 * 3)
+        cells = np.where(rng.uniform(size=(n, 1)) < 0.8, np.minimum(5, dims[:dim] - 3), 1 + (cells - 1) // 3 * 3)
     x = np.array([a[0] for a in axes[:dim]]) + (cells + rng.uniform(0.0, 1.0, size=(n, dim))) * p.dx
     v, B = rng.normal(size=(n, dim)), rng.normal(size=(n, dim * dim)) * p.dx
     om, ov, left = p2g_grid(p, x, v, B, *axes, dims)
@@ -36,3 +33,20 @@ def test_counts_and_crowding(dim, deg, n, crowded):
     assert np.abs(m - om).max() <= 1e-12 * om.max()
     mom = om[:, None] * ov
     assert np.abs(m[:, None] * vv - mom).max() <= 1e-12 * np.abs(mom).max()
+
+
+@pytest.mark.parametrize("dim,deg", [(2, 2), (2, 3), (3, 2), (3, 3)])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 33, 255, 257, 3000])
+@pytest.mark.parametrize("crowded", [False, True])
+def test_counts_and_crowding(dim, deg, n, crowded):
+    _check(dim, deg, n, crowded, (13, 17, 11))
+
+
+@pytest.mark.parametrize("dim,deg", [(2, 2), (3, 3)])
+@pytest.mark.parametrize("over", [0, 1])
+@pytest.mark.parametrize("crowded", [False, True])
+def test_both_sides_of_the_tile_count_where_the_blocks_change(dim, deg, over, crowded):
+    """148 and 149 tiles: a tile has four blocks of 256 threads, then two of 128."""
+    tile = 4 if dim == 3 else 8
+    dims = (149 * tile, tile, tile) if over else (74 * tile, 2 * tile, tile)
+    _check(dim, deg, 5000, crowded, dims)
