@@ -1131,14 +1131,17 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
         }
         if (mibf) mui = (R)((double)A.in.sc[(size_t)MTR_SCALAR_MUI * Np + j] - P.mui0);
       }
-      // the particle's cell, clamped as for the sort; it must lie in the tile
-      // (it does, unless the position is not finite) and its stencil in the grid
+      // The particle's cell, clamped at the first one; it must lie in the tile
+      // and its stencil in the grid.  The sort sends a coordinate that is not
+      // finite to the first cells, so the test is on the floor itself, which no
+      // NaN passes; left of cell -2 every weight is zero.
       bool ok = true;
       int least = 0;
 #pragma unroll
       for (int a = 0; a < D; ++a) {
-        const int g = (int)floor((xp[a] - H->org[a]) * ioh), c = max(g, 0) - (n0[a] + 1);
-        const bool in = (unsigned)c < (unsigned)TB;
+        const double fl = floor((xp[a] - H->org[a]) * ioh);
+        const int g = (int)fl, c = max(g, 0) - (n0[a] + 1);
+        const bool in = fl >= -2.0 && (unsigned)c < (unsigned)TB;
         const int lb = cell_base(n0[a], in ? c : 0);
         ok = ok && in && lb + n0[a] + 3 < (int)H->N[a];
         R w[4], d[4], o[4];
@@ -1287,10 +1290,10 @@ __global__ void __launch_bounds__(256) k_p2g_periodic(StepArgsT<R> A) {
     bool oob = false;
 #pragma unroll
     for (int a = 0; a < D; ++a) {
-      int b = (int)floor((xp[a] - H->org[a]) * ioh) - 1;
-      b = b < 0 ? 0 : b;  // p2g.cpp:21-24 clamps at zero
-      base[a] = b;
-      if (b + 3 >= (int)H->N[a]) oob = true;
+      const double fl = floor((xp[a] - H->org[a]) * ioh);
+      const bool in = fl >= -2.0 && fl + 2.0 < (double)H->N[a];  // false for NaN; left of cell -2 no weight is left
+      base[a] = in ? max((int)fl - 1, 0) : 0;                    // p2g.cpp:21-24 clamps at zero
+      if (!in || base[a] + 3 >= (int)H->N[a]) oob = true;
     }
     if (oob) {
       raise_status(A.H, MTR_STATUS_STENCIL_OOB, A.in.id[i]);
