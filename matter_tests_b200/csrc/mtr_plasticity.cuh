@@ -819,7 +819,7 @@ __device__ __noinline__ bool return_map_svd(const DevParams& P, int pm, double d
     return false;
   }
 #pragma unroll
-  for (int i = 0; i < D; ++i) hencky[i] = S[i] > 1e-4 ? h[i] : ool_log(1e-4);  // plasticity.cpp:21
+  for (int i = 0; i < D; ++i) hencky[i] = S[i] < 1e-4 ? ool_log(1e-4) : h[i];  // plasticity.cpp:21; a NaN stays one, as in std::max
   RmTrial T;
   T.trace = hencky[0];
 #pragma unroll
