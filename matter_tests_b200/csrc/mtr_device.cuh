@@ -291,24 +291,21 @@ __device__ __noinline__ void axis_weights_any(double td, R (&w)[4], R (&d)[4]) {
   }
 }
 
-// binary exponent of a positive weight; zero (which adds nothing) counts as one
-__device__ __forceinline__ int weight_exponent(double w) {
-  const int e = __double2hiint(w) >> 20;
-  return e ? e - 1023 : 0;
-}
-__device__ __forceinline__ int weight_exponent(float w) {
-  const int e = __float_as_int(w) >> 23;
-  return e ? e - 127 : 0;
-}
+// A weight's leading word, ordered as the weight; zero, which adds nothing,
+// counts as the largest.
+__device__ __forceinline__ int weight_word(double w) { return w == 0.0 ? 0x7fffffff : __double2hiint(w); }
+__device__ __forceinline__ int weight_word(float w) { return w == 0.0f ? 0x7fffffff : __float_as_int(w); }
 
-// a lower bound of the exponents of one axis's weights: the outer ones of the
-// cubic spline, the outer two of the three quadratic ones (the fourth is zero)
-template <int DEG, typename R>
+// A lower bound of the binary exponents of one axis's weights (a subnormal
+// weight's and a negative one's, which rounding leaves outside [0, 1], are below
+// the threshold of the products in any case).  ANY: of a stencil that is clamped
+// or on a caller's axes; otherwise the second and third cubic weights are 1/6 or
+// more and need no look.
+template <int DEG, bool ANY, typename R>
 __device__ __forceinline__ int least_exponent(const R (&w)[4]) {
-  if constexpr (DEG == 3)
-    return min(weight_exponent(w[0]), weight_exponent(w[3]));
-  else
-    return min(min(weight_exponent(w[0]), weight_exponent(w[1])), min(weight_exponent(w[2]), weight_exponent(w[3])));
+  int m = min(weight_word(w[0]), weight_word(w[3]));
+  if constexpr (ANY || DEG == 2) m = min(m, min(weight_word(w[1]), weight_word(w[2])));
+  return sizeof(R) == 8 ? (m >> 20) - 1023 : (m >> 23) - 127;
 }
 
 // ---------------------------------------------------------------------------

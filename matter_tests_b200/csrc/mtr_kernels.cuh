@@ -1166,7 +1166,7 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
             d[h] = R(0.0);
           }
         }
-        least += least_exponent<DEG>(w);
+        least += FORCE && g >= 1 ? least_exponent<DEG, false>(w) : least_exponent<DEG, true>(w);
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
           if (part == 0) S.w[a][h] = w[h];
@@ -2091,7 +2091,7 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
             S.w[a][h] = ok ? w[h] : R(0.0);
             S.a[a][h] = ok ? w[h] * o[h] : R(0.0);
           }
-          least += least_exponent<DEG>(w);
+          least += least_exponent<DEG, false>(w);
         }
 #pragma unroll
         for (int r = 0; r < D; ++r) {
