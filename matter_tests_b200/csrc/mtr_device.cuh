@@ -269,14 +269,24 @@ __device__ __forceinline__ void axis_weights(double td, R (&w)[4], R (&d)[4]) {
   if constexpr (!DW) d[0] = d[1] = d[2] = d[3] = R(0.0);
 }
 
-// node offsets x_i - x_p of the same 4 nodes
+// Node offsets x_i - x_p of the same 4 nodes, formed in FP64 and rounded once:
+// in FP32 arithmetic, from the rounded position and the rounded dx, they had an
+// rms error of 4.7e-8 dx instead of 2.9e-8, and dx's own rounding in all of them.
 template <typename R>
-__device__ __forceinline__ void axis_offsets(double td, R dx, R (&o)[4]) {
-  const R t = (R)td, s = (R)(1.0 - td);
-  o[0] = -(R(1.0) + t) * dx;
-  o[1] = -t * dx;
-  o[2] = s * dx;
-  o[3] = (R(1.0) + s) * dx;
+__device__ __forceinline__ void axis_offsets(double td, double dx, R (&o)[4]) {
+  if constexpr (sizeof(R) == 8) {
+    const double s = 1.0 - td;
+    o[0] = -(1.0 + td) * dx;
+    o[1] = -td * dx;
+    o[2] = s * dx;
+    o[3] = (1.0 + s) * dx;
+  } else {
+    const double a = -td * dx;
+    o[0] = (R)(a - dx);
+    o[1] = (R)a;
+    o[2] = (R)(a + dx);
+    o[3] = (R)(a + (dx + dx));
+  }
 }
 
 // A stencil that P2G clamped at the grid's first node: t may lie outside

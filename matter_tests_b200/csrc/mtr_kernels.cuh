@@ -1157,7 +1157,7 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
               d[h] = dc[h];
             }
           }
-          axis_offsets<R>(td, (R)P.dx, o);
+          axis_offsets<R>(td, P.dx, o);
         } else {  // a caller's axes: every node's own coordinate
 #pragma unroll
           for (int h = 0; h < 4; ++h) {
@@ -1691,7 +1691,7 @@ __device__ __forceinline__ void load_patch(const StepCommon& A, const StepHeader
 // incline, FP64 0.524 -> 0.488).
 template <int D, int DEG, bool FLIP, bool WP, bool WB, bool WF, bool GV, int STRIDE, int ROWS, typename R>
 __device__ __forceinline__ void gather_sums(const R* pv, const double (*crd)[Tiling<D>::PN], const int (&lb)[3],
-                                            const double (&xp)[3], double ioh, R dx, R* xf, R (&ps)[3],
+                                            const double (&xp)[3], double ioh, double dx, R* xf, R (&ps)[3],
                                             R (&Bp)[D][D], R (&flp)[3], R (&gv)[D][D]) {
   constexpr int PN = Tiling<D>::PN, STR = NodePatch<D, FLIP, R>::STRIDE;
   constexpr int Z = D - 1;                  // innermost axis
@@ -1784,7 +1784,7 @@ __device__ __forceinline__ void gather_sums(const R* pv, const double (*crd)[Til
 // grad v scaled by 1/dx.
 template <int D, int DEG, bool GV, int STRIDE, int ROWS, typename R>
 __device__ __forceinline__ void gather_patch(const R* pv, const double (*crd)[Tiling<D>::PN], const int (&lb)[3],
-                                             const double (&xp)[3], double ioh, R dx, R* xf,
+                                             const double (&xp)[3], double ioh, double dx, R* xf,
                                              const double (&vref)[3],
                                              double (&pic)[3], R (&Bp)[D][D], R (&flp)[3], R (&gv)[D][D], bool want_b,
                                              bool want_flip) {
@@ -1814,7 +1814,7 @@ __device__ __forceinline__ void gather_patch(const R* pv, const double (*crd)[Ti
 // grad v alone (MUSL deformation update), from a patch without flips
 template <int D, int DEG, int STRIDE, int ROWS, typename R>
 __device__ __forceinline__ void gather_gradv(const R* pv, const double (*crd)[Tiling<D>::PN], const int (&lb)[3],
-                                             const double (&xp)[3], double ioh, R dx, R* xf, R (&gv)[D][D]) {
+                                             const double (&xp)[3], double ioh, double dx, R* xf, R (&gv)[D][D]) {
   R ps[3], Bp[D][D], flp[3];
   gather_sums<D, DEG, false, false, false, false, true, STRIDE, ROWS, R>(pv, crd, lb, xp, ioh, dx, xf, ps, Bp, flp, gv);
   const R iohR = (R)ioh;
@@ -1863,7 +1863,7 @@ __device__ __forceinline__ void g2p_t_body(const StepArgsT<R>& A, const uint32_t
     R flp[3], Bp[D][D], gv[D][D];
     int lb[3];
     if (local_base<D>(H, p.x, ioh, n0, false, lb)) {
-      gather_patch<D, DEG, true, kChunk, 1, R>(pv, crd, lb, p.x, ioh, (R)P.dx, xfac + threadIdx.x, vref, pic, Bp, flp, gv, fr < 0, fr >= -1);
+      gather_patch<D, DEG, true, kChunk, 1, R>(pv, crd, lb, p.x, ioh, P.dx, xfac + threadIdx.x, vref, pic, Bp, flp, gv, fr < 0, fr >= -1);
     } else {
       raise_status(H, MTR_STATUS_STENCIL_OOB, p.id);
 #pragma unroll
@@ -1990,7 +1990,8 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
   __syncthreads();
   const uint32_t Np = A.Np;
   const double dt = H->dt, ioh = P.one_over_dx;
-  const R dx = (R)P.dx, apicD = (R)P.apicDinverse;
+  const double dx = P.dx;
+  const R apicD = (R)P.apicDinverse;
   const bool apic = fr < 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int grp = lane / LPP, col = lane % COLS, c0 = NC == 1 ? lane % LPP / COLS : 0;
@@ -2216,7 +2217,7 @@ __device__ __forceinline__ void defgrad_t_body(const StepArgsT<R>& A, const uint
     R gv[D][D];
     int lb[3];
     if (local_base<D>(H, p.x, ioh, n0, false, lb)) {
-      gather_gradv<D, DEG, kMaxTileThreads, 4, R>(pv, crd, lb, p.x, ioh, (R)A.P->dx, xfac + threadIdx.x, gv);
+      gather_gradv<D, DEG, kMaxTileThreads, 4, R>(pv, crd, lb, p.x, ioh, A.P->dx, xfac + threadIdx.x, gv);
     } else {
       raise_status(H, MTR_STATUS_STENCIL_OOB, p.id);
 #pragma unroll
