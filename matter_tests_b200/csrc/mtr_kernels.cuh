@@ -737,6 +737,39 @@ __device__ __forceinline__ void part_range(uint32_t part, uint32_t parts, uint32
   if (part + 1 < parts) pe = b + (n * (part + 1) / parts & ~31u);
 }
 
+// One warp's run [b, e) of a tile's sorted particles: run `run` of `runs` (at most
+// 32, one lane each below).  The tile's 64 cells are shared out evenly, so that a
+// run starts with a row of cells, unless a run then holds over a quarter more than
+// its share of the particles: such tiles (crowded cells, layers, the faces of a
+// body) are cut by particles, at whole chunks of CH where every run has one.
+// us per step, equal cells and this rule: 960k particles in a layer one cell thick
+// in x, FP64 1764, 972, mixed 1131, 749; 1M and one cell of 3000 more, FP64 1968, 881;
+// 1M in a lattice 769, 761.  All tiles cut by particles: 764 for the lattice, 971.
+// False if the block's runs (nwarps of them from `first`) are all empty.
+// All lanes call together; `cs` = the tile's 65 cell starts.
+template <uint32_t CH>
+__device__ __forceinline__ bool warp_run(const uint32_t* __restrict__ cs, int first, int nwarps, int run, int runs,
+                                         uint32_t& b, uint32_t& e) {
+  const int lane = threadIdx.x & 31;
+  uint32_t lo = cs[64 * min(lane, runs) / runs], hi = cs[64 * min(lane + 1, runs) / runs];
+  const uint32_t p0 = __shfl_sync(0xffffffffu, lo, 0), n = __shfl_sync(0xffffffffu, hi, runs - 1) - p0;
+  const uint32_t worst = __reduce_max_sync(0xffffffffu, hi - lo);
+  if (worst - worst / 5 > (n + runs - 1) / runs) {
+    const uint32_t r = min(lane, runs), unit = n >= CH * runs ? CH : 1, m = (n + unit - 1) / unit;
+    lo = p0 + min(n, m * r / runs * unit);
+    hi = p0 + min(n, m * min(r + 1, (uint32_t)runs) / runs * unit);
+  }
+  b = __shfl_sync(0xffffffffu, lo, run);
+  e = __shfl_sync(0xffffffffu, hi, run);
+  return __shfl_sync(0xffffffffu, lo, first) != __shfl_sync(0xffffffffu, hi, first + nwarps - 1);
+}
+
+// the cell of a tile that holds its sorted particle k (all lanes call together)
+__device__ __forceinline__ int cell_of(const uint32_t (&cstart)[65], uint32_t k) {
+  const int lane = threadIdx.x & 31;
+  return __popc(__ballot_sync(0xffffffffu, cstart[lane + 1] <= k)) + __popc(__ballot_sync(0xffffffffu, cstart[lane + 33] <= k));
+}
+
 template <int D>
 __device__ __forceinline__ void tile_coords(const StepHeader* H, uint32_t t, int (&tc)[3]) {
   if constexpr (D == 3) {
@@ -1061,7 +1094,9 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
   if (step_inactive(H)) return;
   const uint32_t t = bid;
   if (t >= H->ntiles) return;
-  if (A.cell_start[t * 64u + 64u * part / parts] == A.cell_start[t * 64u + 64u * (part + 1) / parts]) return;
+  const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  uint32_t k0, wend;  // this warp's particles
+  if (!warp_run<kStage>(A.cell_start + t * 64u, part * nwarps, nwarps, part * nwarps + warp, parts * nwarps, k0, wend)) return;
   const DevParams& P = *A.P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double(*crd)[PN] = reinterpret_cast<double(*)[PN]>(smem_raw);
@@ -1085,7 +1120,7 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
   const double ioh = P.one_over_dx;
   const R iohR = (R)ioh, apicD = (R)P.apicDinverse;
   const bool apic = P.flip_ratio < 0;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
   const int grp = lane / LPP, role = lane / COLS % ROLES, col = lane % COLS;
   const int c0 = lane / (COLS * ROLES) % (D / NV);  // first component
   const int ix = D == 3 ? col >> 2 : col, iy = D == 3 ? col & 3 : 0;  // this lane's column
@@ -1133,13 +1168,9 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
 #pragma unroll
     for (int h = 0; h < 4; ++h) win.acc[h][NV] += f1[h] * a1;
   };
-  // this warp's cells: a run of particles
-  const int run = part * nwarps + warp, runs = parts * nwarps;
-  int cell = 64 * run / runs;
-  const uint32_t wend = cstart[64 * (run + 1) / runs];
-  uint32_t k0 = cstart[cell];
+  int cell = 0;
   if (k0 < wend) {
-    while (cstart[cell + 1] <= k0) ++cell;
+    cell = cell_of(cstart, k0);
     node0 = window_node<D>(n0, cell, ix, iy);
   }
   for (; k0 < wend; k0 += kStage) {
@@ -2018,7 +2049,9 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
   if (step_inactive(H)) return;
   const uint32_t t = bid;
   if (t >= H->ntiles) return;
-  if (A.cell_start[t * 64u + 64u * part / parts] == A.cell_start[t * 64u + 64u * (part + 1) / parts]) return;
+  const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  uint32_t k0, wend;  // this warp's particles
+  if (!warp_run<32>(A.cell_start + t * 64u, part * nwarps, nwarps, part * nwarps + warp, parts * nwarps, k0, wend)) return;
   const DevParams& P = *A.P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double(*crd)[PN] = reinterpret_cast<double(*)[PN]>(smem_raw);
@@ -2040,7 +2073,7 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
   const double dx = P.dx;
   const R apicD = (R)P.apicDinverse;
   const bool apic = fr < 0;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
   const int grp = lane / LPP, col = lane % COLS, c0 = NC == 1 ? lane % LPP / COLS : 0;
   const int ix = D == 3 ? col >> 2 : col, iy = D == 3 ? col & 3 : 0;  // this lane's column
   MStage<D, R>* st = reinterpret_cast<MStage<D, R>*>(smem_raw + musl_crd_bytes<D, R>() + musl_patch_bytes<D, R>() +
@@ -2048,11 +2081,8 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
   // the gather's x and y factors use the warp's stage, which phase 1 does not
   R* xfac = reinterpret_cast<R*>(st) + lane;
   static_assert(8 * (D - 1) * 32 * sizeof(R) <= musl_stage_bytes<D, R>(), "x and y factors must fit the warp's stage");
-  // this warp's cells: a run of particles
-  const int run = part * nwarps + warp, runs = parts * nwarps;
-  int cell = 64 * run / runs;
-  const uint32_t wend = cstart[64 * (run + 1) / runs];
-  for (uint32_t k0 = cstart[cell]; k0 < wend; k0 += 32) {
+  int cell = k0 < wend ? cell_of(cstart, k0) : 0;
+  for (; k0 < wend; k0 += 32) {
     // phase 1
     __syncwarp();  // the stage has been read
     const uint32_t s = k0 + lane;
