@@ -108,6 +108,7 @@ enum { kSlotP2G = 0, kSlotMUSL = 1, kSlotG2P = 2, kSlotDefgrad = 3, kTileSlots =
 // mark names that end each slot's kernel in a step
 const char* const kSlotMark[kTileSlots] = {"k_p2g", "k_g2p_musl", "k_g2p", "k_defgrad"};
 constexpr uint32_t kResidentTiles = 4 * 148;  // tile blocks taken to be on the chip at once
+constexpr uint32_t kMostTileBlocks = 16384;   // launched to cut tiles, empty ones included
 // largest block of each slot (k_g2p_t is register-bounded per 128 threads)
 const int kSlotMax[kTileSlots] = {kMaxTileThreads, MTR_MUSL_MAX_THREADS, kChunk, kMaxTileThreads};
 const int kTileCandidates[3] = {64, 128, 256};
@@ -526,15 +527,20 @@ void launch_g2p(int spm, dim3 blocks, int threads, cudaStream_t st, const StepAr
   k_g2p_t<D, DEG, R><<<blocks, threads, 0, st>>>(A, perm);
 }
 
-// Blocks of a tile's particles.  A scene of few tiles leaves SMs idle and its
+// Blocks launched for a tile.  A scene of few tiles leaves SMs idle and its
 // tile kernels last as long as one block's chain of passes over its tile, so
 // each tile is cut in 2 or 4 while the blocks still fit the chip at once (four
 // an SM); occupied tiles are counted at 8 (3D) or 4 (2D) particles a cell.  us
 // per step in 1, 2 and 4 parts: 2D 5k particles 63, 53, 47; 2D 51k 67, 58, 63;
 // 2D 212k mixed 84, 92, 112; 3D 150k 145, 144, 148; 3D 1M 831, 894, 1078.
+// A sparse tile takes fewer of them (tile_blocks), and where the grid is large
+// against its particles even the blocks that leave at once cost too much: 20k
+// particles over 106^3 cells (46,656 tiles of capacity) 1214 us a step in 4
+// parts, 885 in 1; 150k over the same, 1569 in 2, 1455 in 1.
 uint32_t tile_parts(const mtr_ctx* c) {
   const uint32_t tiles = std::min<uint32_t>(c->cap_tiles, c->Np / (c->dim == 3 ? 512 : 256) + 1);
-  return tiles * 4 <= kResidentTiles ? 4 : (tiles * 2 <= kResidentTiles ? 2 : 1);
+  auto ok = [&](uint32_t p) { return tiles <= kResidentTiles / p && c->cap_tiles <= kMostTileBlocks / p; };
+  return ok(4) ? 4 : (ok(2) ? 2 : 1);
 }
 
 // `follows`: the step enqueued just before left its commit to this one;

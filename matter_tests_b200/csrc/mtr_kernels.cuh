@@ -730,6 +730,18 @@ __device__ __forceinline__ void tile_range(const StepCommon& A, uint32_t t, uint
   pe = A.cell_start[t * 64u + 64u];
 }
 
+// Blocks that a tile of n particles takes of the `launched` ones: each loads,
+// clears and adds a patch of its own, so a block gets a quarter of a full tile
+// (at 8 particles a cell in 3D, 4 in 2D) before the next one takes part.  us per
+// step with all launched blocks and with this rule, FP64 and mixed: 20k particles
+// at one a cell 158, 107 and 127, 97; 150k 490, 367 and 356, 269; 60k in a layer one
+// cell thick in x 198, 131 and 161, 110; full tiles (60k, 125k) 135, 122 and 166, 166.
+template <int D>
+__device__ __forceinline__ uint32_t tile_blocks(uint32_t n, uint32_t launched) {
+  constexpr uint32_t unit = D == 3 ? 128 : 64;
+  return min(launched, (n + unit - 1) / unit);
+}
+
 // Share `part` of `parts` of a tile's particles [pb, pe): even, cut at whole warps.
 __device__ __forceinline__ void part_range(uint32_t part, uint32_t parts, uint32_t& pb, uint32_t& pe) {
   const uint32_t n = pe - pb, b = pb;
@@ -737,30 +749,38 @@ __device__ __forceinline__ void part_range(uint32_t part, uint32_t parts, uint32
   if (part + 1 < parts) pe = b + (n * (part + 1) / parts & ~31u);
 }
 
-// One warp's run [b, e) of a tile's sorted particles: run `run` of `runs` (at most
-// 32, one lane each below).  The tile's 64 cells are shared out evenly, so that a
+// This warp's run [b, e) of a tile's sorted particles, one of at most 32 (4 blocks
+// of 8 warps), each a lane's below.  The tile's 64 cells are shared out evenly, so that a
 // run starts with a row of cells, unless a run then holds over a quarter more than
 // its share of the particles: such tiles (crowded cells, layers, the faces of a
 // body) are cut by particles, at whole chunks of CH where every run has one.
 // us per step, equal cells and this rule: 960k particles in a layer one cell thick
 // in x, FP64 1764, 972, mixed 1131, 749; 1M and one cell of 3000 more, FP64 1968, 881;
 // 1M in a lattice 769, 761.  All tiles cut by particles: 764 for the lattice, 971.
-// False if the block's runs (nwarps of them from `first`) are all empty.
-// All lanes call together; `cs` = the tile's 65 cell starts.
-template <uint32_t CH>
-__device__ __forceinline__ bool warp_run(const uint32_t* __restrict__ cs, int first, int nwarps, int run, int runs,
-                                         uint32_t& b, uint32_t& e) {
-  const int lane = threadIdx.x & 31;
+// TRIM: the tile takes fewer blocks than launched where it is sparse.  False if
+// the block has none.  All lanes call together; `cs` = the tile's 65 cell starts.
+template <int D, uint32_t CH, bool TRIM = true>
+__device__ __forceinline__ bool warp_run(const uint32_t* __restrict__ cs, int part, int launched, uint32_t& b, uint32_t& e) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  int runs = launched * nwarps;
   uint32_t lo = cs[64 * min(lane, runs) / runs], hi = cs[64 * min(lane + 1, runs) / runs];
   const uint32_t p0 = __shfl_sync(0xffffffffu, lo, 0), n = __shfl_sync(0xffffffffu, hi, runs - 1) - p0;
+  const int parts = TRIM ? (int)tile_blocks<D>(n, launched) : launched;
+  if (part >= parts) return false;
+  if (TRIM && parts < launched) {
+    runs = parts * nwarps;
+    lo = cs[64 * min(lane, runs) / runs];
+    hi = cs[64 * min(lane + 1, runs) / runs];
+  }
   const uint32_t worst = __reduce_max_sync(0xffffffffu, hi - lo);
   if (worst - worst / 5 > (n + runs - 1) / runs) {
     const uint32_t r = min(lane, runs), unit = n >= CH * runs ? CH : 1, m = (n + unit - 1) / unit;
     lo = p0 + min(n, m * r / runs * unit);
     hi = p0 + min(n, m * min(r + 1, (uint32_t)runs) / runs * unit);
   }
-  b = __shfl_sync(0xffffffffu, lo, run);
-  e = __shfl_sync(0xffffffffu, hi, run);
+  const int first = part * nwarps;
+  b = __shfl_sync(0xffffffffu, lo, first + warp);
+  e = __shfl_sync(0xffffffffu, hi, first + warp);
   return __shfl_sync(0xffffffffu, lo, first) != __shfl_sync(0xffffffffu, hi, first + nwarps - 1);
 }
 
@@ -1082,7 +1102,7 @@ constexpr size_t p2g_smem_bytes(int threads, bool mibf = true) {
 // FORCE: false for mass and momentum alone (no stress, no friction, no ids)
 template <int D, int DEG, typename R, bool FORCE = true>
 __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid,
-                                                const uint32_t part, const uint32_t parts) {
+                                                const uint32_t part, const uint32_t launched) {
   using TL = Tiling<D>;
   constexpr int PN = TL::PN, NODES = TL::NODES, NCH = FORCE ? TL::NCH : 1 + D, TB = TL::TB, Z = D - 1;
   // A lane sums NV vector components of a role and its scalar channel on one
@@ -1094,9 +1114,9 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
   if (step_inactive(H)) return;
   const uint32_t t = bid;
   if (t >= H->ntiles) return;
-  const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int warp = threadIdx.x >> 5;
   uint32_t k0, wend;  // this warp's particles
-  if (!warp_run<kStage>(A.cell_start + t * 64u, part * nwarps, nwarps, part * nwarps + warp, parts * nwarps, k0, wend)) return;
+  if (!warp_run<D, kStage, FORCE>(A.cell_start + t * 64u, part, launched, k0, wend)) return;
   const DevParams& P = *A.P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double(*crd)[PN] = reinterpret_cast<double(*)[PN]>(smem_raw);
@@ -1908,7 +1928,7 @@ __device__ __forceinline__ void gather_gradv(const R* pv, const double (*crd)[Ti
 // ---------------------------------------------------------------------------
 template <int D, int DEG, typename R, int PM>
 __device__ __forceinline__ void g2p_t_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid,
-                                                const uint32_t part, const uint32_t parts) {
+                                                const uint32_t part, const uint32_t launched) {
   using TL = Tiling<D>;
   constexpr int PN = TL::PN;
   StepHeader* H = A.H;
@@ -1917,6 +1937,8 @@ __device__ __forceinline__ void g2p_t_body(const StepArgsT<R>& A, const uint32_t
   if (t >= H->ntiles) return;
   uint32_t pb, pe;
   tile_range(A, t, pb, pe);
+  const uint32_t parts = tile_blocks<D>(pe - pb, launched);
+  if (part >= parts) return;
   part_range(part, parts, pb, pe);
   if (pb >= pe) return;
   const DevParams& P = *A.P;
@@ -2040,7 +2062,7 @@ constexpr size_t musl_smem_bytes(int threads) {
 
 template <int D, int DEG, typename R>
 __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid,
-                                                const uint32_t part, const uint32_t parts) {
+                                                const uint32_t part, const uint32_t launched) {
   using TL = Tiling<D>;
   constexpr int PN = TL::PN, NODES = TL::NODES, TB = TL::TB, Z = D - 1;
   // a lane sums NC components of one stencil column; GR groups of LPP lanes
@@ -2049,9 +2071,9 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
   if (step_inactive(H)) return;
   const uint32_t t = bid;
   if (t >= H->ntiles) return;
-  const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int warp = threadIdx.x >> 5;
   uint32_t k0, wend;  // this warp's particles
-  if (!warp_run<32>(A.cell_start + t * 64u, part * nwarps, nwarps, part * nwarps + warp, parts * nwarps, k0, wend)) return;
+  if (!warp_run<D, 32>(A.cell_start + t * 64u, part, launched, k0, wend)) return;
   const DevParams& P = *A.P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double(*crd)[PN] = reinterpret_cast<double(*)[PN]>(smem_raw);
@@ -2263,7 +2285,7 @@ __global__ void __launch_bounds__(MTR_MUSL_BOUNDS)
 // 172,000 nodes and a launch.
 template <int D, int DEG, typename R, int PM>
 __device__ __forceinline__ void defgrad_t_body(const StepArgsT<R>& A, const uint32_t* __restrict__ perm, const uint32_t bid,
-                                                const uint32_t part, const uint32_t parts) {
+                                                const uint32_t part, const uint32_t launched) {
   using TL = Tiling<D>;
   constexpr int PN = TL::PN;
   StepHeader* H = A.H;
@@ -2272,6 +2294,8 @@ __device__ __forceinline__ void defgrad_t_body(const StepArgsT<R>& A, const uint
   if (t >= H->ntiles) return;
   uint32_t pb, pe;
   tile_range(A, t, pb, pe);
+  const uint32_t parts = tile_blocks<D>(pe - pb, launched);
+  if (part >= parts) return;
   part_range(part, parts, pb, pe);
   if (pb >= pe) return;
   __shared__ __align__(16) R pv[NodePatch<D, false, R>::SIZE];
