@@ -750,13 +750,15 @@ __device__ __forceinline__ void part_range(uint32_t part, uint32_t parts, uint32
 }
 
 // This warp's run [b, e) of a tile's sorted particles, one of at most 32 (4 blocks
-// of 8 warps), each a lane's below.  The tile's 64 cells are shared out evenly, so that a
-// run starts with a row of cells, unless a run then holds over a quarter more than
-// its share of the particles: such tiles (crowded cells, layers, the faces of a
-// body) are cut by particles, at whole chunks of CH where every run has one.
-// us per step, equal cells and this rule: 960k particles in a layer one cell thick
-// in x, FP64 1764, 972, mixed 1131, 749; 1M and one cell of 3000 more, FP64 1968, 881;
-// 1M in a lattice 769, 761.  All tiles cut by particles: 764 for the lattice, 971.
+// of 8 warps), each a lane's below.  The tile's 64 cells are shared out evenly, so
+// that a run starts with a row of cells, unless a run then holds over a quarter more
+// than its share of the particles and takes more chunks of CH: such tiles (crowded
+// cells, layers, the faces of a body) are cut by particles, at whole chunks where
+// every run has one.  us, equal cells and this rule: 960k particles in a layer one
+// cell thick in x 1762, 974 a step (mixed 1128, 746); 1M and one cell of 3000 more
+// 1968, 886 (mixed 1667, 772); 1M in a lattice 766, 763; no-allocation transfer of
+// 262k random particles 167, 169 a call.  Without the test on chunks that takes 177,
+// from twice the share on the 1M column's passes lose their 3%.
 // TRIM: the tile takes fewer blocks than launched where it is sparse.  False if
 // the block has none.  All lanes call together; `cs` = the tile's 65 cell starts.
 template <int D, uint32_t CH, bool TRIM = true>
@@ -773,7 +775,8 @@ __device__ __forceinline__ bool warp_run(const uint32_t* __restrict__ cs, int pa
     hi = cs[64 * min(lane + 1, runs) / runs];
   }
   const uint32_t worst = __reduce_max_sync(0xffffffffu, hi - lo);
-  if (worst - worst / 5 > (n + runs - 1) / runs) {
+  const uint32_t share = (n + runs - 1) / runs;
+  if (worst - worst / 5 > share && (worst + CH - 1) / CH > (share + CH - 1) / CH) {
     const uint32_t r = min(lane, runs), unit = n >= CH * runs ? CH : 1, m = (n + unit - 1) / unit;
     lo = p0 + min(n, m * r / runs * unit);
     hi = p0 + min(n, m * min(r + 1, (uint32_t)runs) / runs * unit);
