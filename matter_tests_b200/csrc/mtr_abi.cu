@@ -1926,9 +1926,7 @@ int mtr_set_tile_lanes(mtr_ctx* c, const int* lanes) {
   return guarded([&]() -> int {
     if (!c || !lanes) throw MtrError{MTR_ERR_INVALID, "null argument"};
     if (!valid_tile_lanes(c->dim, lanes)) throw MtrError{MTR_ERR_INVALID, "lanes per particle: 16 or 32 (3D), 4 or 8 (2D)"};
-    CK(cudaSetDevice(c->device));
     for (int i = 0; i < kScatterSlots; ++i) c->tile_split[i] = lanes[i] / scatter_columns(c->dim);
-    free_graphs(c);
     return MTR_OK;
   });
 }
@@ -2276,7 +2274,6 @@ int mtr_batch_set_tile_lanes(mtr_batch* b, int group, const int* lanes) {
     mtr_batch_group& g = b->groups[group];
     if (!valid_tile_lanes(g.dim, lanes)) throw MtrError{MTR_ERR_INVALID, "lanes per particle: 16 or 32 (3D), 4 or 8 (2D)"};
     for (int i = 0; i < kScatterSlots; ++i) g.tile_split[i] = lanes[i] / scatter_columns(g.dim);
-    b->dirty = true;
     return MTR_OK;
   });
 }

@@ -2046,7 +2046,6 @@ template <int D, typename R>
 struct MStageData {
   R w[D][4], a[D][4];  // weights and weights times offsets
   R q[D][4];           // V, X, Y, Z (2D: V, X, Z) of each component
-  int lb;
 };
 template <int D, typename R>
 struct __align__(16) MStage : MStageData<D, R> {
