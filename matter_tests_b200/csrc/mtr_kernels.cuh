@@ -665,7 +665,7 @@ static __device__ void order_cell(const StepCommon& A, uint32_t b, uint32_t e) {
   uint32_t lo = 0xffffffffu;
   for (uint32_t q = b + threadIdx.x; q < e; q += kSortThreads) lo = min(lo, A.perm_tmp[q]);
   lo = block_min(lo);
-  for (uint32_t at = b; at < e;) {
+  for (uint32_t at = b; at < e && lo != 0xffffffffu;) {  // (lo is an index while members are left)
     for (uint32_t w = threadIdx.x; w < kMarkWords; w += kSortThreads) marks[w] = 0u;
     __syncthreads();
     uint32_t next = 0xffffffffu;

@@ -65,3 +65,26 @@ def test_one_crowded_cell_in_a_large_scene(prec):
     x = _lattice([50, 50, 50])
     crowd = 0.07 + np.random.default_rng(2).uniform(0.0002, 0.0098, size=(3000, 3))
     assert _step_ms(np.concatenate([x, crowd]), prec) <= 1.6 * _step_ms(x, prec)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("deg", [2, 3])
+@pytest.mark.parametrize("n", [63, 65, 129, 257, 513, 700])
+def test_transfer_sums_in_the_mixed_form(dim, deg, n):
+    """Node mass and momentum of an uneven tile against the oracle.  A node sums at
+    most n products of about 8 roundings of 6e-8 each, of any sign: 1e-5 of the
+    largest is over 6 standard errors at n = 700."""
+    sc = cases.apply(cases.block(dim, deg, n=10 if dim == 3 else 20), precision=PREC_MIXED, gravity=(0.0, 0.0, 0.0),
+                     plastic_model=cases.PM.NoPlasticity)
+    rng = np.random.default_rng(n)
+    cells = np.full((n, dim), 5.0)
+    cells[::9] = rng.integers(3, 9, size=cells[::9].shape)
+    sc.x = np.ascontiguousarray((cells + rng.uniform(0.05, 0.95, size=cells.shape)) * sc.params.dx)
+    for k in ("v", "B", "scalars"):
+        setattr(sc, k, np.ascontiguousarray(getattr(sc, k)[:n]))
+    sc.F = None  # no stress: the grid velocity is the transferred one
+    sc.plates, sc.objects = [], []
+    g, o = run_gpu(sc, 1)["g"], run_oracle(sc, 1)["g"]
+    assert np.abs(g["mass"] - o["mass"]).max() <= 1e-5 * o["mass"].max()
+    p, q = g["mass"][:, None] * g["v"], o["mass"][:, None] * o["v"]
+    assert np.abs(p - q).max() <= 1e-5 * np.abs(q).max()
