@@ -731,14 +731,16 @@ __device__ __forceinline__ void tile_range(const StepCommon& A, uint32_t t, uint
 }
 
 // Blocks that a tile of n particles takes of the `launched` ones: each loads,
-// clears and adds a patch of its own, so a block gets a quarter of a full tile
-// (at 8 particles a cell in 3D, 4 in 2D) before the next one takes part.  us per
-// step with all launched blocks and with this rule, FP64 and mixed: 20k particles
-// at one a cell 158, 107 and 127, 97; 150k 490, 367 and 356, 269; 60k in a layer one
-// cell thick in x 198, 131 and 161, 110; full tiles (60k, 125k) 135, 122 and 166, 166.
+// clears and adds a patch of its own, so a block gets an eighth of a full tile
+// (at 8 particles a cell in 3D, 4 in 2D), a chunk a warp, before the next one takes
+// part.  us per step with all launched blocks and with this rule, FP64 and mixed:
+// 20k particles at one a cell 144 -> 118 and 120 -> 100, 150k 456 -> 361 and 330 ->
+// 265, 60k in a layer one cell thick in x 151 -> 134 and 133 -> 114; full tiles (60k,
+// 125k) 130, 131 and 167, 167.  A quarter of a tile a block: 106 and 95 for the first,
+// but 8553 particles, whose tiles are half full, 82 -> 87 (mixed), here 83.
 template <int D>
 __device__ __forceinline__ uint32_t tile_blocks(uint32_t n, uint32_t launched) {
-  constexpr uint32_t unit = D == 3 ? 128 : 64;
+  constexpr uint32_t unit = D == 3 ? 64 : 32;
   return min(launched, (n + unit - 1) / unit);
 }
 
