@@ -753,14 +753,19 @@ __device__ __forceinline__ void part_range(uint32_t part, uint32_t parts, uint32
 
 // This warp's run [b, e) of a tile's sorted particles, one of at most 32 (4 blocks
 // of 8 warps), each a lane's below.  The tile's 64 cells are shared out evenly, so
-// that a run starts with a row of cells, unless a run then holds over a quarter more
-// than its share of the particles and takes more chunks of CH: such tiles (crowded
-// cells, layers, the faces of a body) are cut by particles, at whole chunks where
-// every run has one.  us, equal cells and this rule: 960k particles in a layer one
-// cell thick in x 1762, 974 a step (mixed 1128, 746); 1M and one cell of 3000 more
-// 1968, 886 (mixed 1667, 772); 1M in a lattice 766, 763; no-allocation transfer of
-// 262k random particles 167, 169 a call.  Without the test on chunks that takes 177,
-// from twice the share on the 1M column's passes lose their 3%.
+// that a run starts with a row of cells, unless a run then holds far more than its
+// share of the particles and takes more chunks of CH: such tiles (crowded cells,
+// layers) are cut by particles, at whole chunks where every run has one.  us per
+// step, equal cells and this rule: 960k particles in a layer one cell thick in x
+// 1762, 981 (mixed 1128, 748); 1M and one cell of 3000 more 1968, 846 (mixed 1667,
+// 718).  FAR: 2.5 times the share.  In FP64 with one block a tile a quarter over it
+// is enough (EVEN), which the faces of a body gain from: 96 steps of the 1M column
+// 89.6 -> 86.6 ms, 500k two cells thick in x 598 -> 440 us a step.  More blocks have
+// runs of one or two chunks, and a run that starts inside a row of cells adds a
+// window: 42k particles 102 -> 104 us a step with the lower line.  In FP32 four warps
+// instead of two on the same nodes of a face order their sums in more ways: 1M column
+// 63.5 -> 62.4 ms, but 15-18 in 100 runs then leave the FP64 run's side of a stick-slip
+// threshold at the floor within 80 steps, 1 in 100 with FAR.
 // TRIM: the tile takes fewer blocks than launched where it is sparse.  False if
 // the block has none.  All lanes call together; `cs` = the tile's 65 cell starts,
 // lo and hi = even_run of all launched warps, which a kernel loads before it looks
@@ -771,7 +776,7 @@ __device__ __forceinline__ void even_run(const uint32_t* __restrict__ cs, int ru
   lo = cs[64 * min(lane, runs) / runs];
   hi = cs[64 * min(lane + 1, runs) / runs];
 }
-template <int D, uint32_t CH, bool TRIM = true>
+template <int D, uint32_t CH, bool EVEN, bool TRIM = true>
 __device__ __forceinline__ bool warp_run(const uint32_t* __restrict__ cs, int part, int launched, uint32_t lo, uint32_t hi,
                                          uint32_t& b, uint32_t& e) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -785,7 +790,8 @@ __device__ __forceinline__ bool warp_run(const uint32_t* __restrict__ cs, int pa
   }
   const uint32_t worst = __reduce_max_sync(0xffffffffu, hi - lo);
   const uint32_t share = (n + runs - 1) / runs;
-  if (worst - worst / 5 > share && (worst + CH - 1) / CH > (share + CH - 1) / CH) {
+  const bool far = EVEN && launched == 1 ? worst - worst / 5 > share : worst / 5 * 2 > share;
+  if (far && (worst + CH - 1) / CH > (share + CH - 1) / CH) {
     const uint32_t r = min(lane, runs), unit = n >= CH * runs ? CH : 1, m = (n + unit - 1) / unit;
     lo = p0 + min(n, m * r / runs * unit);
     hi = p0 + min(n, m * min(r + 1, (uint32_t)runs) / runs * unit);
@@ -1130,7 +1136,7 @@ __device__ __forceinline__ void p2g_w_body(const StepArgsT<R>& A, const uint32_t
   if (t >= H->ntiles) return;
   const int warp = threadIdx.x >> 5;
   uint32_t k0, wend;  // this warp's particles
-  if (!warp_run<D, kStage, FORCE>(A.cell_start + t * 64u, part, launched, lo, hi, k0, wend)) return;
+  if (!warp_run<D, kStage, kFP64<R>, FORCE>(A.cell_start + t * 64u, part, launched, lo, hi, k0, wend)) return;
   const DevParams& P = *A.P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double(*crd)[PN] = reinterpret_cast<double(*)[PN]>(smem_raw);
@@ -2088,7 +2094,7 @@ __device__ __forceinline__ void g2p_musl_w_body(const StepArgsT<R>& A, const uin
   if (t >= H->ntiles) return;
   const int warp = threadIdx.x >> 5;
   uint32_t k0, wend;  // this warp's particles
-  if (!warp_run<D, 32>(A.cell_start + t * 64u, part, launched, lo, hi, k0, wend)) return;
+  if (!warp_run<D, 32, kFP64<R>>(A.cell_start + t * 64u, part, launched, lo, hi, k0, wend)) return;
   const DevParams& P = *A.P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double(*crd)[PN] = reinterpret_cast<double(*)[PN]>(smem_raw);
